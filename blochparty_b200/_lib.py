@@ -72,6 +72,7 @@ BP_NUF_MAX_TERMS = 6
 BP_SEG_DT, BP_SEG_WX, BP_SEG_WY, BP_SEG_KX, BP_SEG_KY, BP_SEG_KZ, BP_SEG_BETA = (1 << k for k in range(7))
 BP_SEG_ALL = 0x7F
 BP_SPIN_NO_OFFSETS = 0x80  # with seg_mask: the position and dB0 rows of the spin gradients are not wanted
+BP_CLIP_BEGIN, BP_CLIP_END = 1, 2  # bp_propagate, bp_readout: the windows' samples alone of a run cut by them
 BP_SPIN_NONE = 0x100  # with seg_mask: no row of the spin gradients is wanted
 ERRORS = {BP_E_ARG: "invalid argument", BP_E_ALIGN: "misaligned buffer", BP_E_LAUNCH: "CUDA launch failed",
           BP_E_SIZE: "size above the documented maximum"}
@@ -87,6 +88,11 @@ SIGNATURES = {
     "bp_forward_grid": (c_int, [c_int, c_int]),
     "bp_forward_mma_grid": (c_int, [c_int]),
     "bp_forward": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, _P, _P]),
+    "bp_sample_runs": (c_int, [_P, c_int64, c_int, _P, c_int64, _P, _P, c_int64, _P]),
+    "bp_propagate": (c_int, [_P, c_int, _P, _P, _P, c_int, c_int, _P, _P, c_int, _P, _P, c_int, _P, c_int, c_int, c_int,
+                             _P, _P]),
+    "bp_readout": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, _P, c_int, _P, c_int, _P, c_int, c_int, _P,
+                           _P]),
     "bp_forward_spans": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, _P, c_int, _P, _P, _P, c_int, _P, _P]),
     "bp_signal_finish": (c_int, [_P, _P, c_int, c_int, _P, _P]),
     "bp_ffma_peak": (c_int, [_P, c_int, _P, _P]),

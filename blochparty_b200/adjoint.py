@@ -280,11 +280,8 @@ class Checkpointed:
         """The forward over intervals [ka, kb), saving the states after the RF runs in them into their slots."""
         pk, plan = self.pk, self.plan
         fa, fb = plan.franges[ka][0], plan.franges[kb - 1][1]
-        code = _lib.lib().bp_forward_saving(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs),
-                                            ptr(pk.seg64), ptr(plan.fwin_dev), fa, fb, ptr(state), ptr(raw),
-                                            ptr(self.fslot_dev), ptr(self.slots), 0, ptr(self.status),
-                                            _lib.stream_ptr())
-        _lib.check(code, "bp_forward_saving")
+        engine.run_forward(pk, state, plan.fwin_dev, fa, fb, raw, self.status, wstates=self.slots,
+                           wslot=self.fslot_dev, whole_runs=True)
 
     def forward(self, state: torch.Tensor) -> None:
         """All intervals from ``state`` ([6][n], advanced in place), the raw coil sums into ``raw`` (zeroed first),
@@ -311,7 +308,8 @@ class Checkpointed:
         """The forward kernel over windows [wa, wb) (the physics variant with the field model)."""
         pk = self.pk
         if self.phys is None:
-            engine.run_forward(pk, state, wdev, wa, wb, raw, self.status, wstates=wstates, wstate_stride=1)
+            engine.run_forward(pk, state, wdev, wa, wb, raw, self.status, wstates=wstates, wstate_stride=1,
+                               whole_runs=True)
             return
         import ctypes
 

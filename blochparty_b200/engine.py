@@ -33,6 +33,44 @@ F32, F64 = torch.float32, torch.float64
 RF, ADC, SPOIL, SAME_FREE, SAME_RFDT, SAME_OFF, SMALL = 1, 2, 4, 8, 16, 32, 64
 
 
+Z_BYTES = 1 << 30  # the forward's workspace at most: the first samples of the runs of one launch
+RUN_MAX = 256  # samples per run
+
+
+def sample_runs(flags: np.ndarray):
+    """(runs (R, 4), subs (B, 2)) int32: the runs of samples (``bp_propagate`` in the header: first segment, the segment
+    after it or -1, samples, ADC row of the first) and their 32-sample blocks. A sample joins the run before it when it
+    follows it on a free segment, unspoiled, with the factors of the run's samples (a run of one sample takes any: a
+    readout's first sample half a dwell in, then the dwells). A run that would pass ``RUN_MAX`` samples ends at a
+    multiple of 32 segments."""
+    fl = np.ascontiguousarray(flags, dtype=np.int32)
+    n_adc = int(np.count_nonzero(fl & ADC))
+    runs, subs = np.empty((n_adc, 4), dtype=np.int32), np.empty((n_adc, 2), dtype=np.int32)
+    n = np.zeros(2, dtype=np.int64)
+    code = _lib.lib().bp_sample_runs(fl.ctypes.data, fl.shape[0], RUN_MAX, runs.ctypes.data, n_adc, n[:1].ctypes.data,
+                                     subs.ctypes.data, n_adc, n[1:].ctypes.data)
+    _lib.check(code, "bp_sample_runs")
+    return runs[: n[0]], subs[: n[1]]
+
+
+class SampleRuns:
+    """The runs of samples of a sequence and their blocks of 32, on the device for ``bp_propagate`` and
+    ``bp_readout``."""
+
+    def __init__(self, flags: np.ndarray, device):
+        runs, subs = sample_runs(flags)
+        both = torch.from_numpy(np.concatenate([runs.reshape(-1), subs.reshape(-1)])).to(device)
+        self.n_runs, self.n_subs = runs.shape[0], subs.shape[0]
+        self.runs, self.subs = both[: runs.size], both[runs.size:]
+        self.starts = runs[:, 0]
+
+    def most_in(self, segments: int) -> int:
+        """The most runs that start within any stretch of ``segments`` segments."""
+        if self.n_runs == 0:
+            return 0
+        return int((np.searchsorted(self.starts, self.starts + segments) - np.arange(self.n_runs)).max())
+
+
 @dataclass
 class Packed:
     """A case's device buffers (see module docstring) and sizes."""
@@ -47,6 +85,12 @@ class Packed:
     psi: torch.Tensor  # (A,) float64 receiver phase of every sample
     flags: np.ndarray  # (S,) int32 on the host
     device: torch.device
+    runs: SampleRuns | None = None  # the runs of samples (sample_runs), laid out on the first forward with a readout
+
+    def sample_runs(self) -> SampleRuns:
+        if self.runs is None:
+            self.runs = SampleRuns(self.flags, self.device)
+        return self.runs
 
 
 def _bools(flags, n: int) -> np.ndarray:
@@ -200,11 +244,44 @@ def pack(case, device) -> Packed:
 
 def run_forward(pk: Packed, state: torch.Tensor, windows_dev: torch.Tensor, w_begin: int, w_end: int,
                 raw: torch.Tensor | None, status: torch.Tensor, wstates: torch.Tensor | None = None,
-                wstate_stride: int = 1, max_ctas: int = 0) -> None:
-    code = _lib.lib().bp_forward(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64),
-                                 ptr(windows_dev), w_begin, w_end, ptr(state), ptr(raw), ptr(wstates),
-                                 wstate_stride, max_ctas, ptr(status), _lib.stream_ptr())
-    _lib.check(code, "bp_forward")
+                wstate_stride: int = 1, max_ctas: int = 0, wslot: torch.Tensor | None = None,
+                whole_runs: bool = False) -> None:
+    """The forward over windows [w_begin, w_end) from ``state``, advanced in place: ``bp_propagate``, then with
+    ``raw`` (the coil sums, added to) ``bp_readout``, over as many windows at a time as keep the workspace between
+    them under ``Z_BYTES``. ``wstates``: states at window starts, every ``wstate_stride``-th or by slot (``wslot``).
+    ``whole_runs``: a run of samples is formed whole by the call whose windows it starts in (calls over consecutive
+    windows then give the same bits wherever they are divided); else the windows' samples alone."""
+    lib, stream = _lib.lib(), _lib.stream_ptr()
+    runs = pk.sample_runs() if raw is not None else None
+    step, cap, z = max(w_end - w_begin, 1), 0, None
+    if runs is not None and runs.n_runs:
+        room = max(Z_BYTES // (8 * pk.n), 1)
+        cap = runs.n_runs
+        if cap > room:  # fewer windows at a time
+            step = max(1, step * room // cap)
+            while step > 1 and runs.most_in(step * _lib.BP_SEG_MAX) + 1 > room:
+                step = (step + 1) // 2
+            cap = min(cap, runs.most_in(step * _lib.BP_SEG_MAX) + 1)
+        z = torch.empty(cap, pk.n, 2, dtype=F32, device=pk.device)
+    for wa in range(w_begin, w_end, step):
+        wb = min(wa + step, w_end)
+        clip = 0 if whole_runs else ((_lib.BP_CLIP_BEGIN if wa == w_begin else 0)
+                                     | (_lib.BP_CLIP_END if wb == w_end else 0))
+        slot0 = None if wstates is None or wslot is not None else (wa - w_begin)
+        ws = wstates
+        if slot0:  # (a strided save over several launches: the slots continue)
+            if slot0 % wstate_stride:
+                raise ValueError("window states every few windows need one launch")
+            ws = wstates[slot0 // wstate_stride:]
+        code = lib.bp_propagate(ptr(pk.spins), pk.n, ptr(pk.segs), ptr(pk.seg64), ptr(windows_dev), wa, wb, ptr(state),
+                                ptr(ws), wstate_stride, ptr(wslot), ptr(runs.runs) if z is not None else None,
+                                runs.n_runs if z is not None else 0, ptr(z), cap, clip, max_ctas, ptr(status), stream)
+        _lib.check(code, "bp_propagate")
+        if z is not None:
+            code = lib.bp_readout(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64),
+                                  ptr(windows_dev), wa, wb, ptr(runs.runs), runs.n_runs, ptr(runs.subs), runs.n_subs,
+                                  ptr(z), cap, clip, ptr(raw), stream)
+            _lib.check(code, "bp_readout")
 
 
 def finish_signal(pk: Packed, raw: torch.Tensor) -> torch.Tensor:
@@ -267,6 +344,9 @@ def forward_spans(pk: Packed, state: torch.Tensor, plan, spans, raw: torch.Tenso
     """``forward_replacing`` in one native call: ``spans`` is a ctypes array of ``_lib.BpSpan`` (one per span of
     ``plan``, from ``plan_replacing``), launched in order by ``bp_forward_spans``."""
     _, wdev, ranges = plan
+    if len(ranges) == 1:  # nothing is replaced: the stepped forward
+        run_forward(pk, state, wdev, *ranges[0], raw, status, max_ctas=max_ctas)
+        return
     rng = np.ascontiguousarray(np.asarray(ranges, dtype=np.int32).reshape(-1, 2))
     n_spans = rng.shape[0] - 1
     code = _lib.lib().bp_forward_spans(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64),

@@ -95,6 +95,35 @@ int bp_forward_saving(const float* spins, const float* sens, int n, int n_coils,
                       const int32_t* windows, int w_begin, int w_end, float* state, double* raw, const int32_t* wslot,
                       float* wstates, int max_ctas, int32_t* status, void* stream);
 
+/* The runs of samples of bp_propagate and their 32-sample blocks from the flags (host arrays): runs of at most run_max
+ * (>= 64) samples. */
+int bp_sample_runs(const int32_t* flags, int64_t n, int run_max, int32_t* runs, int64_t max_runs, int64_t* n_runs,
+                   int32_t* subs, int64_t max_subs, int64_t* n_subs);
+
+/* bp_forward in two kernels with a workspace between them, and faster for it: bp_propagate takes the spins through
+ * windows [w_begin, w_end) and writes every spin's first sample of each run of samples into z; bp_readout forms the
+ * runs' samples and adds their coil sums to raw. bp_propagate alone (z NULL) is a forward without a readout.
+ *   wstates, wstate_stride, wslot  as bp_forward's and bp_forward_saving's (wslot may be NULL)
+ *   runs    [n_runs] int32 x 4, the whole sequence's runs in order: the first sample's segment, the segment after it
+ *           (whose factor separates the samples; -1 for a single sample), the samples, the first one's ADC row. A
+ *           run's samples lie on consecutive segments; all but the first are on free segments with one dt, moments
+ *           and b0_offset; no sample but the last spoils; a run starts where those factors, a sample or its absence,
+ *           a spoil or a multiple of 32 segments starts
+ *   subs    [n_subs] int32 x 2: run, block of 32 samples of it, for every run and block in order
+ *   z       [z_cap][n] (float32, float32) workspace (8-byte aligned), run by run from the first run of the windows;
+ *           z_cap at least the runs that start in the windows (and the one they start inside of)
+ *   clip    which of a run that reaches beyond the windows' samples are theirs: 0, the whole run where it starts
+ *           (calls over consecutive windows then form each run once); BP_CLIP_BEGIN | BP_CLIP_END, the samples in the
+ *           windows alone */
+#define BP_CLIP_BEGIN 1
+#define BP_CLIP_END 2
+int bp_propagate(const float* spins, int n, const void* segs, const double* seg64, const int32_t* windows, int w_begin,
+                 int w_end, float* state, float* wstates, int wstate_stride, const int32_t* wslot, const int32_t* runs,
+                 int n_runs, float* z, int z_cap, int clip, int max_ctas, int32_t* status, void* stream);
+int bp_readout(const float* spins, const float* sens, int n, int n_coils, const void* segs, const double* seg64,
+               const int32_t* windows, int w_begin, int w_end, const int32_t* runs, int n_runs, const int32_t* subs,
+               int n_subs, const float* z, int z_cap, int clip, double* raw, void* stream);
+
 /* Readout runs through a nonuniform FFT (simulate(..., readout="nufft"); replaces the NUFFT readouts of
  * engines/gpu/cuda/kernels.cu.in:91-140 with engines/gpu/driver.py:236-266). A run is L consecutive samples with
  * one free segment's factors (dt, moments, offset), so spin j's samples are z1 q^p, p < L, q = e^(-dt r2)

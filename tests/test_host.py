@@ -435,3 +435,57 @@ def test_saved_slots_protocol_in_blocks(budget):
                 e = win + 1
                 if sv.rf[win] and (e == W or not sv.rf[e]):  # the end of an RF run: its state is read
                     assert slots.get(run_of[e] % cap) == run_of[e], (budget, K, cap, win)
+
+
+def _runs_by_hand(flags):
+    """sample_runs, one sample at a time."""
+    out, row, cut = [], 0, False  # cut: the last run is the rest of one that was too long
+    for s in range(len(flags)):
+        f = int(flags[s])
+        if not f & engine.ADC:
+            continue
+        joins = full = False
+        if out and out[-1][0] + out[-1][2] == s and not f & engine.RF and not flags[s - 1] & engine.SPOIL:
+            first, _, n, _ = out[-1]
+            full = s % 32 == 0 and s - first + 32 > engine.RUN_MAX
+            joins = (n == 1 and not cut) or (bool(f & engine.SAME_FREE) and not full)
+        if joins:
+            out[-1][2] += 1
+            out[-1][1] = out[-1][0] + 1
+        else:
+            cut = full and bool(f & engine.SAME_FREE) and out[-1][2] > 1
+            out.append([s, -1, 1, row])
+        row += 1
+    return np.asarray(out, dtype=np.int32).reshape(-1, 4)
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_sample_runs(seed):
+    """The runs of samples of random sequences (readouts of every length, factors that change from sample to sample,
+    RF segments that sample, spoils) are those of a walk over the samples, and their 32-sample blocks cover them."""
+    r = np.random.RandomState(seed)
+    flags = []
+    while len(flags) < 4000:
+        k = int(r.choice([1, 2, 3, 7, 40, 300, 600]))
+        kind = r.rand()
+        if kind < 0.2:  # RF, some sampling
+            flags += [engine.RF | (engine.ADC if r.rand() < 0.3 else 0) for _ in range(min(k, 40))]
+        elif kind < 0.4:  # free, no samples
+            flags += [0] + [engine.SAME_FREE] * (k - 1)
+        elif kind < 0.5:  # samples with changing factors
+            flags += [engine.ADC | (engine.SAME_FREE if r.rand() < 0.4 else 0) for _ in range(k)]
+        else:  # a readout: another first segment, then one set of factors
+            flags += [engine.ADC, engine.ADC] + [engine.ADC | engine.SAME_FREE] * k
+            if r.rand() < 0.3:
+                flags[-int(r.randint(1, k + 1))] |= engine.SPOIL
+    flags = np.asarray(flags, dtype=np.int32)
+    prev_rf = np.concatenate([[True], (flags[:-1] & engine.RF) != 0])
+    flags[prev_rf] &= ~engine.SAME_FREE
+    want = _runs_by_hand(flags)
+    got = engine.SampleRuns(flags, "cpu")
+    assert np.array_equal(engine.sample_runs(flags)[0], want)
+    assert want[:, 2].sum() == ((flags & engine.ADC) != 0).sum() and want[:, 2].max() <= engine.RUN_MAX
+    subs = got.subs.numpy().reshape(-1, 2)
+    assert np.array_equal(np.bincount(subs[:, 0], minlength=len(want)), -(-want[:, 2] // 32))
+    most = max(int(((want[:, 0] >= s) & (want[:, 0] < s + 500)).sum()) for s in want[:, 0])
+    assert got.most_in(500) == most
