@@ -1,7 +1,7 @@
 // Forward propagation with the coil readout on the tensor cores (tcgen05, split bfloat16, float32 accumulation).
 //
-// The propagation (windows, persistent CTAs over 128-spin tiles, TMA-staged segment blocks, compensated float32
-// state) is that of forward.cu. The readout differs: the coil sum of a block of 16 ADC samples over a tile's 128
+// The propagation's steps are those of bp_propagate_kernel (windows, persistent CTAs over 128-spin tiles, TMA-staged
+// segment blocks, compensated float32 state). The readout differs: the coil sum of a block of 16 ADC samples over a tile's 128
 // spins is one small matrix product on the tensor cores,
 //     D[m][t] += sum_k A[m][k] B[t][k],   k = 2 j + {0, 1} (spin j's Mx, My),
 // with A the tile's coil sensitivities (row m = 2c: (s_r, -s_i), row 2c + 1: (s_i, s_r) per spin, coil c) and B
@@ -22,7 +22,7 @@
 
 #include <cstdint>
 
-#include "bloch_common.cuh"
+#include "packed.cuh"
 #include "tcgen05.cuh"
 #include "../../include/blochparty_b200.h"
 
@@ -145,15 +145,16 @@ __global__ void __launch_bounds__(MM_THREADS, 3) bp_forward_mma_kernel(MmaArgs a
             const int j0 = tile * MM_THREADS + tid;
             const bool active = j0 < n;
             const int j = active ? j0 : 0;
-            const Spin p = load_spin(a.spins, n, j, active);
-            float mx = 0.f, my = 0.f, mz = 0.f, lx = 0.f, ly = 0.f, lz = 0.f;
+            const Spin sp = load_spin(a.spins, n, j, active);
+            const PropSpin p{(double)sp.px, (double)sp.py, (double)sp.pz, (double)sp.db0, sp.pd, sp.r1, sp.r2};
+            const Pk<1> b1{sp.b1}, nb1{-sp.b1};
+            State<1> m;
+            m.x.f = m.y.f = m.z.f = m.lx.f = m.ly.f = m.lz.f = 0.0f;
             if (active) {
-                mx = a.state[j], my = a.state[n + j], mz = a.state[2 * n + j];
-                lx = a.state[3 * n + j], ly = a.state[4 * n + j], lz = a.state[5 * n + j];
+                m.x.f = a.state[j], m.y.f = a.state[n + j], m.z.f = a.state[2 * n + j];
+                m.lx.f = a.state[3 * n + j], m.ly.f = a.state[4 * n + j], m.lz.f = a.state[5 * n + j];
             }
-            FreeFactors ff{1.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            RfRelax rr{1.f, 1.f, 0.f, 0.f, 0.f, 0.f};
-            float wz = 0.0f;
+            RfRun<1> rr;
             int slot = 0, grp = 0, row = 0;
             // one sample (x, y) into the B block; a full block (or the window's last sample) goes to the tensor
             // cores. Returns false when a wait failed (the CTA stops).
@@ -204,74 +205,54 @@ __global__ void __launch_bounds__(MM_THREADS, 3) bp_forward_mma_kernel(MmaArgs a
                 }
                 return true;
             };
-            for (int s = 0; s < nseg && !fail; ++s) {
+            // the steps of bp_propagate_kernel with one spin per thread (the same arithmetic, bit for bit)
+            for (int s = 0; s < nseg && !fail;) {
                 const SegRec q = q0[s];
                 const int f = q.flags;
                 if (f & BP_RF) {
-                    if (s == 0 || !(f & BP_SAME_RFDT)) rr = rf_relax(q.dt, p);
-                    if (s == 0 || !(f & BP_SAME_OFF)) wz = rf_wz(q, p);
-                    rf_step_wz(q, p, rr, wz, mx, my, mz, lx, ly, lz);
-                    if (!(f & (BP_ADC | BP_SPOIL))) {  // the rest of the pulse, as in bp_forward
-                        constexpr int kRun = BP_RF | BP_SAME_RFDT | BP_SAME_OFF;
-                        if (f & BP_SMALL) {  // (the run's small steps without the factors' tier tests)
-                            constexpr int kSmall = kRun | BP_SMALL;
-                            while (s + 1 < nseg) {
-                                const SegRec& qn = q0[s + 1];
-                                if ((qn.flags & (kSmall | BP_ADC | BP_SPOIL)) != kSmall) break;
-                                ++s;
-                                rf_step_wz<true>(qn, p, rr, wz, mx, my, mz, lx, ly, lz);
-                            }
-                        }
-                        while (s + 1 < nseg) {
-                            const SegRec& qn = q0[s + 1];
-                            if ((qn.flags & (kRun | BP_ADC | BP_SPOIL)) != kRun) break;
-                            ++s;
-                            rf_step_wz(qn, p, rr, wz, mx, my, mz, lx, ly, lz);
-                        }
-                        continue;
-                    }
-                } else {
-                    if (s == 0 || !(f & BP_SAME_FREE)) ff = free_factors(q, a.seg64[win.x + s], p);
-                    free_step(ff, p, mx, my, mz, lx, ly, lz);
-                    if ((f & (BP_ADC | BP_SPOIL)) == BP_ADC) {
-                        // a readout run, as in bp_forward: the samples by a float32 recurrence within this window
-                        // and block of BP_ADJ_WIN segments, the state after it from the merged factors
-                        const int block_end = min(nseg, (win.x + s) / BP_ADJ_WIN * BP_ADJ_WIN + BP_ADJ_WIN - win.x);
-                        int e = s + 1;
-                        float zr = mx + lx, zi = my + ly;
-                        if (readout && !stage(zr, zi)) fail = true;
-                        while (!fail && e < block_end && (q0[e].flags & ~BP_SPOIL) == (BP_ADC | BP_SAME_FREE)) {
-                            if (readout) {
-                                readout_advance(ff, zr, zi);
-                                if (!stage(zr, zi)) {
-                                    fail = true;
-                                    break;
-                                }
-                            }
-                            if (q0[e++].flags & BP_SPOIL) break;
-                        }
-                        if (fail) break;
-                        if (e > s + 1) {
-                            const FreeFactors fr = free_factors_merged(q, a.seg64[win.x + s], p, e - s - 1);
-                            free_step(fr, p, mx, my, mz, lx, ly, lz);
-                            if (q0[e - 1].flags & BP_SPOIL) mx = my = lx = ly = 0.0f;
-                        }
-                        s = e - 1;
-                        continue;
-                    }
-                }
-                if (f & (BP_ADC | BP_SPOIL)) {
-                    if ((f & BP_ADC) && readout && !stage(mx + lx, my + ly)) {
+                    if (s == 0 || !(f & BP_SAME_RFDT)) rf_run_relax(rr, q.dt, &p);
+                    if (s == 0 || !(f & BP_SAME_OFF)) rf_run_offset(rr, q, &p);
+                    if (f & BP_SMALL)
+                        rf_step_packed<true>(Pk<1>{q.wx0}, Pk<1>{q.wy0}, b1, nb1, rr, m);
+                    else
+                        rf_step_packed<false>(Pk<1>{q.wx0}, Pk<1>{q.wy0}, b1, nb1, rr, m);
+                    if ((f & BP_ADC) && readout && !stage(m.x.f + m.lx.f, m.y.f + m.ly.f)) {
                         fail = true;
                         break;
                     }
-                    if (f & BP_SPOIL) mx = my = lx = ly = 0.0f;
+                    if (f & BP_SPOIL) m.x.f = m.y.f = m.lx.f = m.ly.f = 0.0f;
+                    ++s;
+                    continue;
                 }
+                // a piece: free segments with the factors of s, all samples or none, a spoil at most on the last,
+                // within a block of BP_ADJ_WIN segments
+                const int block_end = min(nseg, (win.x + s) / BP_ADJ_WIN * BP_ADJ_WIN + BP_ADJ_WIN - win.x);
+                int e = s + 1;
+                while (e < block_end && !(q0[e - 1].flags & BP_SPOIL) &&
+                       (q0[e].flags & (BP_RF | BP_ADC | BP_SAME_FREE)) == ((f & BP_ADC) | BP_SAME_FREE))
+                    ++e;
+                const double4 k64 = a.seg64[win.x + s];
+                if ((f & BP_ADC) && readout) {  // the samples by a float32 recurrence
+                    const FreeFactors one = prop_factors(q.dt, k64, p, 1);
+                    float zr = m.x.f + m.lx.f, zi = m.y.f + m.ly.f;
+                    for (int t = s; t < e; ++t) {
+                        readout_advance(one, zr, zi);
+                        if (!stage(zr, zi)) {
+                            fail = true;
+                            break;
+                        }
+                    }
+                    if (fail) break;
+                }
+                const FreeFactors all = prop_factors(q.dt, k64, p, e - s);
+                free_step_packed(&all, &p, m);
+                if (q0[e - 1].flags & BP_SPOIL) m.x.f = m.y.f = m.lx.f = m.ly.f = 0.0f;
+                s = e;
             }
             // (on a failure the tile loop ends below, after the A-tile copy has been waited for)
             if (active) {
-                a.state[j] = mx, a.state[n + j] = my, a.state[2 * n + j] = mz;
-                a.state[3 * n + j] = lx, a.state[4 * n + j] = ly, a.state[5 * n + j] = lz;
+                a.state[j] = m.x.f, a.state[n + j] = m.y.f, a.state[2 * n + j] = m.z.f;
+                a.state[3 * n + j] = m.lx.f, a.state[4 * n + j] = m.ly.f, a.state[5 * n + j] = m.lz.f;
             }
             if (readout && !a_waited && tid == 0) mbar_wait_bounded(&bars[4], a_phase);  // only on a failure path
             if (readout && !a_waited) a_phase ^= 1u;
