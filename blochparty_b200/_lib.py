@@ -44,6 +44,13 @@ class BpPhysics(ctypes.Structure):
                 ("wstate_stride", c_int)]
 
 
+class BpHostSpins(ctypes.Structure):
+    """``BpHostSpins`` of the C ABI: the host arrays ``bp_pack_spins`` reads."""
+
+    _fields_ = [(f, c_void_p) for f in ("pos", "pd", "t1", "t2", "db0", "b1", "coils", "m0")] + [
+        ("wide", ctypes.c_int32 * 8)]
+
+
 class BpForwardWorkspace(ctypes.Structure):
     """``BpForwardWorkspace`` of the C ABI: the forward's device buffer sizes in bytes."""
 
@@ -61,6 +68,7 @@ BP_OK, BP_E_ARG, BP_E_ALIGN, BP_E_LAUNCH, BP_E_SIZE = 0, 1, 2, 3, 4
 BP_MAX_COILS = 32
 BP_SEG_MAX = 160
 BP_ADJ_WIN = 32
+BP_PACK_BLOCK = 32768  # spins per block of bp_pack_spins
 BP_MMA_MAX_COILS = 8
 BP_MLP_PARAMS = 10320
 BP_MLP_INPUTS = 2
@@ -88,7 +96,11 @@ SIGNATURES = {
     "bp_forward_grid": (c_int, [c_int, c_int]),
     "bp_forward_mma_grid": (c_int, [c_int]),
     "bp_forward": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, _P, _P]),
+    "bp_pack_segments": (c_int, [_P, _P, _P, _P, _P, _P, _P, _P, c_int64, _P, _P, _P, _P, _P, _P]),
     "bp_sample_runs": (c_int, [_P, c_int64, c_int, _P, c_int64, _P, _P, c_int64, _P]),
+    "bp_pack_spins_staging": (c_int64, [c_int64, c_int]),
+    "bp_pack_spins": (c_int, [_P, c_int64, c_int, _P, _P, _P, _P, _P, c_int64, _P]),
+    "bp_final_m": (c_int, [_P, c_int, _P, _P]),
     "bp_propagate": (c_int, [_P, c_int, _P, _P, _P, c_int, c_int, _P, _P, c_int, _P, _P, c_int, _P, c_int, c_int, c_int,
                              _P, _P]),
     "bp_readout": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, _P, c_int, _P, c_int, _P, c_int, c_int, _P,

@@ -127,8 +127,8 @@ def simulate(phantom, seq, coils: Tensor | None = None, *, m_init: Tensor | None
     if coils is None:
         coils = torch.ones(n, 1, dtype=torch.complex64)
     inp = Inputs(phantom.pos, phantom.pd, phantom.t1, phantom.t2, phantom.db0, getattr(phantom, "b1", None), coils,
-                 seq.dt, seq.rf, seq.grad, seq.adc_phase, getattr(seq, "b0_offset", None), list(seq.is_rf),
-                 list(seq.adc), list(seq.spoil), m_init)
+                 seq.dt, seq.rf, seq.grad, seq.adc_phase, getattr(seq, "b0_offset", None),
+                 *(f if isinstance(f, list) else list(f) for f in (seq.is_rf, seq.adc, seq.spoil)), m_init)
     if grad:
         from .adjoint import simulate_grad
 

@@ -669,3 +669,19 @@ extern "C" int bp_readout(const float* spins, const float* sens, int n, int n_co
     }
     return cudaGetLastError() == cudaSuccess ? BP_OK : BP_E_LAUNCH;
 }
+
+// ---- the magnetization from the state: [n][3], high and low parts added ----
+__global__ void bp_final_m_kernel(const float* __restrict__ state, int n, float* __restrict__ m) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 3 * (int64_t)n) return;
+    const int64_t j = i / 3, c = i - 3 * j;
+    m[i] = (float)((double)state[c * n + j] + (double)state[(3 + c) * n + j]);
+}
+
+extern "C" int bp_final_m(const float* state, int n, float* m, void* stream) {
+    if (n < 0 || (n > 0 && (!state || !m))) return BP_E_ARG;
+    if (n == 0) return BP_OK;
+    const int64_t blocks = (3 * (int64_t)n + 255) / 256;
+    bp_final_m_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(state, n, m);
+    return cudaGetLastError() == cudaSuccess ? BP_OK : BP_E_LAUNCH;
+}

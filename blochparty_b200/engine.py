@@ -110,10 +110,47 @@ def _np64(t) -> np.ndarray:
     return t.detach().to(F64).cpu().numpy()
 
 
+def _host(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as a contiguous host tensor of float32, float64, complex64 or complex128."""
+    t = t.detach().cpu().resolve_conj().resolve_neg()
+    if t.dtype not in (F32, F64, torch.complex64, torch.complex128):
+        t = t.to(F64)
+    return t.contiguous()
+
+
+def _upload_spins(pos, pd, t1, t2, db0, b1, coils, m_init, device, want_state: bool):
+    """(spins [8][N], sens [16 ceil(C/8)][N], state [6][N] or None, extent): every value rounded once to float32 from
+    its float64 value (the rates 1/T1, 1/T2 formed in float64), by the native packer through page-locked staging;
+    extent: the largest magnitude of every row of ``spins`` (float32 on the host)."""
+    n, n_coils = pd.shape[0], coils.shape[1]
+    rows = [_host(t.expand(n)) for t in (pd, t1, t2, db0)]
+    pos = _host(pos.expand(n, 3))
+    b1 = None if b1 is None else _host(b1.expand(n))
+    coils = _host(coils if coils.dtype in (torch.complex64, torch.complex128) else coils.to(torch.complex128))
+    m0 = None if m_init is None else _host(m_init.expand(n, 3))
+    spins = torch.empty(8, n, dtype=F32, device=device)
+    sens = torch.empty(16 * ((n_coils + 7) // 8), n, dtype=F32, device=device)
+    state = torch.empty(6, n, dtype=F32, device=device) if want_state else None
+    extent = np.zeros(8, dtype=np.float32)
+    arrays = [pos, *rows, b1, coils, m0]
+    src = _lib.BpHostSpins(*(ptr(t) for t in arrays))
+    for i, t in enumerate(arrays):
+        src.wide[i] = int(t is not None and t.dtype in (F64, torch.complex128))
+    lib = _lib.lib()
+    staging = torch.empty(lib.bp_pack_spins_staging(n, n_coils), dtype=torch.uint8, pin_memory=True)
+    with torch.cuda.device(device):
+        code = lib.bp_pack_spins(ctypes.addressof(src), n, n_coils, ptr(spins), ptr(sens), ptr(state),
+                                 extent.ctypes.data, ptr(staging), staging.numel(), _lib.stream_ptr())
+    _lib.check(code, "bp_pack_spins")
+    return spins, sens, state, extent
+
+
 def pack_spins(pos, pd, t1, t2, db0, b1, coils, device):
-    """spins [8][N] and sens [16 ceil(C/8)][N] float32 on ``device``: every value rounded once to float32 from its
-    float64 value (the rates 1/T1, 1/T2 formed in float64), written row by row into the float32 buffers."""
+    """spins [8][N] and sens [16 ceil(C/8)][N] float32 on ``device`` (``_upload_spins``; on the CPU row by row in
+    torch)."""
     n = pd.shape[0]
+    if torch.device(device).type == "cuda" and 0 < n and 0 < coils.shape[1] <= _lib.BP_MAX_COILS:
+        return _upload_spins(pos, pd, t1, t2, db0, b1, coils, None, device, False)[:2]
     d64 = lambda t: t.detach().cpu().to(F64)
     spins = torch.empty(8, n, dtype=F32)
     spins[0:3] = d64(pos).T
@@ -127,52 +164,40 @@ def pack_spins(pos, pd, t1, t2, db0, b1, coils, device):
         spins[7] = d64(b1)
     n_coils = coils.shape[1]
     ncg = (n_coils + 7) // 8
-    # (N, 2C) float32 rounded on the host, moved as it lies, transposed on the device (a host-side transpose of the
-    # spin-major coil array costs more than the copy)
     c = torch.view_as_real(coils.detach().cpu().to(torch.complex128).contiguous()).reshape(n, 2 * n_coils).to(F32)
     sens = torch.zeros(16 * ncg, n, dtype=F32, device=device)
     sens[0:2 * n_coils] = c.to(device).T
     return spins.to(device).contiguous(), sens.contiguous()
 
 
-def pack_segments(dt, rf, grad, b0_offset, adc_phase, is_rf, adc, spoil, device):
-    """Segment records (float64 arithmetic, one rounding to float32), the float64 moments, flags and psi. The
-    fields are filled and compared as contiguous rows of a field-major array, then transposed once into records."""
-    dt, rf, grad = _np64(dt), _np64(rf), _np64(grad)
+def pack_segments(dt, rf, grad, b0_offset, adc_phase, is_rf, adc, spoil, device, extent: np.ndarray | None = None):
+    """Segment records (float64 arithmetic, one rounding to float32), the float64 moments, psi, the flags (host) and
+    the number of samples, by the native packer into one buffer and, on a GPU, one copy from page-locked memory.
+    ``extent``: the spins' extents (``_upload_spins``), to set SMALL as ``mark_small_rf`` does."""
+    arrays = [np.ascontiguousarray(_np64(t)) for t in (dt, rf, grad, adc_phase)]
+    dt, rf, grad, phase = arrays
     S = dt.shape[0]
-    b0 = np.zeros(S) if b0_offset is None else _np64(b0_offset)
-    w = -TWO_PI * dt
-    k = grad.T * dt  # (3, S)
-    beta = b0 * dt
-    cols = np.empty((8, S), dtype=np.float32)  # the record's fields, one row each
-    cols[0] = dt
-    cols[1] = w * rf[:, 0]
-    cols[2] = w * rf[:, 1]
-    cols[3:6] = k
-    cols[6] = beta
-    k64 = np.empty((4, S), dtype=np.float64)
-    k64[0:3] = k
-    k64[3] = beta
-    is_rf, adc_b, spoil_b = (_bools(f, S) for f in (is_rf, adc, spoil))
-    flags = is_rf.astype(np.int32) | (adc_b.astype(np.int32) << 1) | (spoil_b.astype(np.int32) << 2)
-    if S > 1:
-        free = ~is_rf
-        same_dt = cols[0, 1:] == cols[0, :-1]
-        same_k = same_dt.copy()  # the moments and the offset phase
-        for c in range(4):
-            same_k &= k64[c, 1:] == k64[c, :-1]
-        same_free = free[1:] & free[:-1] & same_k
-        same_rf = is_rf[1:] & is_rf[:-1] & same_dt
-        same_off = same_rf.copy()  # the same G.r + dt dB0 + beta per spin
-        for c in range(3, 7):
-            same_off &= cols[c, 1:] == cols[c, :-1]
-        flags[1:] |= ((same_free.astype(np.int32) << 3) | (same_rf.astype(np.int32) << 4)
-                      | (same_off.astype(np.int32) << 5))
-    cols.view(np.int32)[7] = flags
-    rec, seg64 = np.ascontiguousarray(cols.T), np.ascontiguousarray(k64.T)
-    psi = np.remainder(_np64(adc_phase)[adc_b], TWO_PI)
-    return (torch.from_numpy(rec).to(device).contiguous(), torch.from_numpy(seg64).to(device).contiguous(),
-            torch.from_numpy(psi).to(device).contiguous(), flags, int(adc_b.sum()))
+    b0 = None if b0_offset is None else np.ascontiguousarray(_np64(b0_offset))
+    shapes = ((dt, (S,)), (rf, (S, 2)), (grad, (S, 3)), (phase, (S,)), (b0, (S,)))
+    for t, shape in shapes:
+        if t is not None and t.shape != shape:
+            raise ValueError(f"a sequence of {S} segments takes an array {shape}, got {t.shape}")
+    marks = [np.ascontiguousarray(_bools(f, S)).view(np.uint8) for f in (is_rf, adc, spoil)]
+    n_adc = int(np.count_nonzero(marks[1]))
+    flags = np.empty(S, dtype=np.int32)
+    gpu = torch.device(device).type == "cuda"
+    host = torch.empty(64 * S + 8 * n_adc, dtype=torch.uint8, pin_memory=gpu and S > 0)
+    base = host.data_ptr()
+    count = np.zeros(1, dtype=np.int64)
+    code = _lib.lib().bp_pack_segments(dt.ctypes.data, rf.ctypes.data, grad.ctypes.data,
+                                       None if b0 is None else b0.ctypes.data, phase.ctypes.data,
+                                       *(m.ctypes.data for m in marks), S,
+                                       None if extent is None else extent.ctypes.data, base, base + 32 * S,
+                                       flags.ctypes.data, base + 64 * S, count.ctypes.data)
+    _lib.check(code, "bp_pack_segments")
+    dev = host.to(device, non_blocking=True) if gpu else host
+    return (dev[: 32 * S].view(F32).view(S, 8), dev[32 * S: 64 * S].view(F64).view(S, 4), dev[64 * S:].view(F64), flags,
+            n_adc)
 
 
 def plan_windows(flags: np.ndarray, samp_max: int, seg_max: int = _lib.BP_SEG_MAX, breaks: np.ndarray | None = None):
@@ -211,6 +236,10 @@ def initial_state(pd, m_init, device):
 
 
 def final_m(state: torch.Tensor) -> torch.Tensor:
+    if state.is_cuda and state.is_contiguous():
+        m = torch.empty(state.shape[1], 3, dtype=F32, device=state.device)
+        _lib.check(_lib.lib().bp_final_m(ptr(state), state.shape[1], ptr(m), _lib.stream_ptr()), "bp_final_m")
+        return m.cpu()
     s = state.to(F64)
     return (s[0:3] + s[3:6]).to(F32).T.contiguous().cpu()
 
@@ -234,12 +263,25 @@ def mark_small_rf(spins: torch.Tensor, segs: torch.Tensor, flags: np.ndarray) ->
     flags |= small.cpu().numpy().astype(np.int32) * SMALL
 
 
-def pack(case, device) -> Packed:
-    spins, sens = pack_spins(case.pos, case.pd, case.t1, case.t2, case.db0, case.b1, case.coils, device)
+def pack_with_state(case, device):
+    """(``pack(case, device)``, its start state [6][N] on ``device``)."""
+    n, n_coils = case.pd.shape[0], case.coils.shape[1]
+    extent = None
+    if torch.device(device).type == "cuda" and 0 < n and 0 < n_coils <= _lib.BP_MAX_COILS:
+        spins, sens, state, extent = _upload_spins(case.pos, case.pd, case.t1, case.t2, case.db0, case.b1, case.coils,
+                                                   case.m_init, device, True)
+    else:
+        spins, sens = pack_spins(case.pos, case.pd, case.t1, case.t2, case.db0, case.b1, case.coils, device)
+        state = initial_state(case.pd, case.m_init, device)
     segs, seg64, psi, flags, n_adc = pack_segments(case.dt, case.rf, case.grad, case.b0_offset, case.adc_phase,
-                                                   case.is_rf, case.adc, case.spoil, device)
-    mark_small_rf(spins, segs, flags)
-    return Packed(case.pd.shape[0], case.coils.shape[1], n_adc, spins, sens, segs, seg64, psi, flags, device)
+                                                   case.is_rf, case.adc, case.spoil, device, extent)
+    if extent is None:
+        mark_small_rf(spins, segs, flags)
+    return Packed(n, n_coils, n_adc, spins, sens, segs, seg64, psi, flags, device), state
+
+
+def pack(case, device) -> Packed:
+    return pack_with_state(case, device)[0]
 
 
 def run_forward(pk: Packed, state: torch.Tensor, windows_dev: torch.Tensor, w_begin: int, w_end: int,
@@ -255,7 +297,7 @@ def run_forward(pk: Packed, state: torch.Tensor, windows_dev: torch.Tensor, w_be
     runs = pk.sample_runs() if raw is not None else None
     step, cap, z = max(w_end - w_begin, 1), 0, None
     if runs is not None and runs.n_runs:
-        room = max(Z_BYTES // (8 * pk.n), 1)
+        room = max(Z_BYTES // (8 * max(pk.n, 1)), 1)
         cap = runs.n_runs
         if cap > room:  # fewer windows at a time
             step = max(1, step * room // cap)
@@ -357,17 +399,15 @@ def forward_spans(pk: Packed, state: torch.Tensor, plan, spans, raw: torch.Tenso
 
 def forward(case, device, max_ctas: int = 0):
     """Signal (C, A) complex64 and m (N, 3) float32, both on the CPU, of a case (``oracle.bloch.Case``-like)."""
-    pk = pack(case, device)
-    samp = _lib.lib().bp_forward_samp_max(pk.n_coils)
+    samp = _lib.lib().bp_forward_samp_max(case.coils.shape[1])
     if samp <= 0:
-        raise ValueError(f"at most {_lib.BP_MAX_COILS} coils, got {pk.n_coils}")
+        raise ValueError(f"at most {_lib.BP_MAX_COILS} coils, got {case.coils.shape[1]}")
+    pk, state = pack_with_state(case, device)
     windows = plan_windows(pk.flags, samp)
     wdev = torch.from_numpy(windows).to(device).contiguous()
-    state = initial_state(case.pd, case.m_init, device)
     raw = torch.zeros(max(pk.n_adc, 1), 2 * pk.n_coils, dtype=F64, device=device)
     status = torch.zeros(1, dtype=torch.int32, device=device)
     run_forward(pk, state, wdev, 0, windows.shape[0], raw if pk.n_adc else None, status, max_ctas=max_ctas)
     sig = finish_signal(pk, raw)
-    torch.cuda.synchronize(device)
-    _lib.check_status(status, "bp_forward")
+    _lib.check_status(status, "bp_forward")  # (waits for the kernels)
     return sig.cpu(), final_m(state)

@@ -21,6 +21,7 @@ for W = 8, M = 3 and T2 down to 20 ms over a 127-sample run.
 
 from __future__ import annotations
 
+import functools
 import math
 from dataclasses import dataclass
 
@@ -65,10 +66,16 @@ def find_runs(flags: np.ndarray, min_len: int = MIN_RUN, max_len: int = _lib.BP_
     return runs
 
 
+@functools.lru_cache(maxsize=2)
+def _gauss_legendre(n: int):
+    """Nodes and weights of the quadrature (an eigenvalue problem of 13 ms at 400 nodes: solved once)."""
+    return np.polynomial.legendre.leggauss(n)
+
+
 def kernel_ft(kappa: np.ndarray, W: int, beta: float, G: int, n: int = 400) -> np.ndarray:
     """The Fourier transform of psi(u) = exp(beta (sqrt(1 - (2 G u / W)^2) - 1)) (|u| <= W / (2 G)) at the
     integer modes ``kappa`` (Gauss-Legendre quadrature in float64; psi is even)."""
-    t, wt = np.polynomial.legendre.leggauss(n)
+    t, wt = _gauss_legendre(n)
     u = t * W / (2.0 * G)
     val = np.exp(beta * (np.sqrt(1.0 - t * t) - 1.0)) * wt * W / (2.0 * G)
     return (val[None, :] * np.cos(2.0 * np.pi * np.outer(kappa, u))).sum(1)

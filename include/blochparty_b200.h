@@ -95,10 +95,37 @@ int bp_forward_saving(const float* spins, const float* sens, int n, int n_coils,
                       const int32_t* windows, int w_begin, int w_end, float* state, double* raw, const int32_t* wslot,
                       float* wstates, int max_ctas, int32_t* status, void* stream);
 
+/* A sequence's segment records, float64 moments, flags and receiver phases from its float64 values (host arrays, no
+ * GPU): rf [n][2] (Hz), grad [n][3] (Hz/m), b0 [n] (Hz, or NULL), phase [n] (rad); records [n] (32 bytes), seg64 [n][4],
+ * flags [n], psi (room for n, *n_adc used). extent: NULL, or the spins' largest |x| |y| |z| pd r1 r2 |dB0| |b1|
+ * (float32 x 8): then RF segments whose rotation stays below |w|^2 = 0.0624 for every spin carry flag 64.
+ * Replaces the packing of engines/gpu/driver.py:291-440. */
+int bp_pack_segments(const double* dt, const double* rf, const double* grad, const double* b0, const double* phase,
+                     const uint8_t* is_rf, const uint8_t* adc, const uint8_t* spoil, int64_t n, const float* extent,
+                     void* records, double* seg64, int32_t* flags, double* psi, int64_t* n_adc);
+
 /* The runs of samples of bp_propagate and their 32-sample blocks from the flags (host arrays): runs of at most run_max
  * (>= 64) samples. */
 int bp_sample_runs(const int32_t* flags, int64_t n, int run_max, int32_t* runs, int64_t max_runs, int64_t* n_runs,
                    int32_t* subs, int64_t max_subs, int64_t* n_subs);
+
+/* Spins, coil sensitivities and start state from host arrays to the device buffers of bp_forward, through a
+ * page-locked staging area of the caller's (bp_pack_spins_staging bytes, or any room for one block: one thread per
+ * block of it), by several threads; every value rounded once to float32 from its float64 value. The copies are issued
+ * on `stream` and have ended when the call returns. state may be NULL; extent: NULL, or float32 x 8 (host), as
+ * bp_pack_segments takes it. */
+#define BP_PACK_BLOCK 32768
+typedef struct {
+    const void *pos, *pd, *t1, *t2, *db0, *b1, *coils, *m0; /* [n][3], [n] each, b1 NULL: 1, [n][C] complex, [n][3] or
+                                                               NULL: (0, 0, pd) */
+    int32_t wide[8]; /* per array: 1 float64, 0 float32 */
+} BpHostSpins;
+int64_t bp_pack_spins_staging(int64_t n, int n_coils);
+int bp_pack_spins(const BpHostSpins* in, int64_t n, int n_coils, float* spins, float* sens, float* state,
+                  float* extent, void* staging, int64_t staging_bytes, void* stream);
+
+/* m [n][3] float32 = the state's high and low parts added. */
+int bp_final_m(const float* state, int n, float* m, void* stream);
 
 /* bp_forward in two kernels with a workspace between them, and faster for it: bp_propagate takes the spins through
  * windows [w_begin, w_end) and writes every spin's first sample of each run of samples into z; bp_readout forms the

@@ -489,3 +489,38 @@ def test_sample_runs(seed):
     assert np.array_equal(np.bincount(subs[:, 0], minlength=len(want)), -(-want[:, 2] // 32))
     most = max(int(((want[:, 0] >= s) & (want[:, 0] < s + 500)).sum()) for s in want[:, 0])
     assert got.most_in(500) == most
+
+
+@pytest.mark.parametrize("S,b0", [(1, False), (5, True), (9000, True), (40000, False)])
+def test_native_segment_records(S, b0):
+    """The records, moments, flags and receiver phases of the native packer against their definition in numpy, and
+    SMALL from the spins' extents against ``mark_small_rf``: bit for bit."""
+    r = np.random.RandomState(S)
+    pick = lambda *shape: np.where(r.rand(*shape) < 0.7, 1.0, r.rand(*shape))  # neighbours often share a value
+    dt, rf, grad = 1e-5 * pick(S), 4000 * (pick(S, 2) - 0.5), 1e4 * (pick(S, 3) - 0.5)
+    phase, off = 50 * (r.rand(S) - 0.5), 30 * (pick(S) - 0.5) if b0 else None
+    is_rf, adc, spoil = ([bool(x) for x in r.rand(S) < p] for p in (0.5, 0.4, 0.05))
+    t = torch.from_numpy
+    extent = np.array([0.1, 0.1, 0.05, 1, 2, 30, 100, 1.2], dtype=np.float32)
+    args = (t(dt), t(rf), t(grad), None if off is None else t(off), t(phase), is_rf, adc, spoil, "cpu")
+    segs, seg64, psi, flags, n_adc = engine.pack_segments(*args, extent)
+    bare = engine.pack_segments(*args)
+    w, k, beta = -2 * np.pi * dt, grad * dt[:, None], (0.0 if off is None else off) * dt
+    cols = np.stack([dt, w * rf[:, 0], w * rf[:, 1], *k.T, np.broadcast_to(beta, (S,))]).astype(np.float32)
+    assert np.array_equal(segs.numpy()[:, :7], cols.T)
+    assert np.array_equal(seg64.numpy(), np.concatenate([k, np.broadcast_to(beta, (S,))[:, None]], 1))
+    a, s, f = (np.array(v) for v in (adc, spoil, is_rf))
+    assert n_adc == a.sum() and np.array_equal(psi.numpy(), np.remainder(phase[a], 2 * np.pi))
+    want = f * 1 + a * 2 + s * 4
+    m64 = seg64.numpy()
+    for i in range(1, S):
+        same_dt = cols[0, i] == cols[0, i - 1]
+        if not f[i] and not f[i - 1] and same_dt and (m64[i] == m64[i - 1]).all():
+            want[i] |= 8
+        if f[i] and f[i - 1] and same_dt:
+            want[i] |= 16 | (32 if (cols[3:7, i] == cols[3:7, i - 1]).all() else 0)
+    assert np.array_equal(bare[3], want) and np.array_equal(bare[0].numpy().view(np.int32)[:, 7], want)
+    spins = t(extent)[:, None].clone()
+    marked = bare[3].copy()
+    engine.mark_small_rf(spins, bare[0], marked)
+    assert np.array_equal(flags, marked) and np.array_equal(segs.numpy().view(np.int32)[:, 7], marked)
