@@ -68,6 +68,7 @@ BP_OK, BP_E_ARG, BP_E_ALIGN, BP_E_LAUNCH, BP_E_SIZE = 0, 1, 2, 3, 4
 BP_MAX_COILS = 32
 BP_SEG_MAX = 160
 BP_ADJ_WIN = 32
+BP_SWEEP_MAX = 2048  # segments of an interval whose RF gradient bp_sweep forms
 BP_PACK_BLOCK = 32768  # spins per block of bp_pack_spins
 BP_MMA_MAX_COILS = 8
 BP_MLP_PARAMS = 10320
@@ -120,6 +121,11 @@ SIGNATURES = {
     "bp_forward_saving": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, _P, _P, _P, _P, c_int, _P, _P]),
     "bp_adjoint_physics": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, c_int, _P,
                                    _P, _P, _P, c_int, c_int, _P, _P, _P, _P]),
+    "bp_cotangent_split": (c_int, [_P, c_int, c_int, _P, _P, _P]),
+    "bp_cotangent": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, _P, c_int, _P, _P, _P, _P, _P, _P, _P]),
+    "bp_sweep_grid": (c_int, [c_int, c_int, c_int]),
+    "bp_sweep": (c_int, [_P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P, c_int, _P, c_int, _P, _P, _P, _P,
+                         _P, _P, _P, _P]),
     "bp_seg_reduce": (c_int, [_P, c_int, c_int, c_int, _P, _P]),
     "bp_pulse_targets": (c_int, [_P, c_int, c_double, c_double, c_double, c_double, _P, c_int, _P, _P, _P]),
     "bp_mlp_grad_ctas": (c_int, [c_int]),

@@ -232,7 +232,8 @@ class Checkpointed:
         # ``budget_bytes``), the forward stores the state at every start of a block of intervals instead, and the
         # backward rebuilds each block's saved states by one forward of the block (no readout) before its sweep.
         # Its intervals are at most 2048 segments (the sweep sums an interval's RF gradient in shared memory).
-        want = saved and phys is None and rf_relaxation_invertible(pk)
+        invertible = phys is None and rf_relaxation_invertible(pk)
+        want = saved and invertible
         plan = Plan(pk, min(every, 2048), device, saved=True) if want else None
         self.layout = None  # saved: (intervals per block, slots)
         if plan is not None and plan.saved is not None:
@@ -243,6 +244,9 @@ class Checkpointed:
             plan = Plan(pk, every, device)
         self.plan = plan
         self.saved = plan.saved
+        # whether every adjoint window is one run of RF or of free segments: then the gradients that need no
+        # per-segment sums but the RF waveform's take a window in one step (bp_cotangent, bp_sweep)
+        self.uniform = invertible and (plan.saved is not None or SavedStates.of(pk.flags, plan.awin) is not None)
         k = len(plan.starts)
         self.outer = outer if outer > 1 and k > outer and self.saved is None else 0
         fws = _lib.forward_workspace(pk.n, pk.n_adc, pk.n_coils)
@@ -255,6 +259,12 @@ class Checkpointed:
             # interval starts (two levels), or block starts followed by one block's interval starts (three)
             n_states = k if not self.outer else (k + self.outer - 1) // self.outer + self.outer
             self.ckpts = sized(self.ws.checkpoints, (n_states, 6, pk.n), F32, device)
+            if phys is None:  # the checkpoint that takes each forward window's start state, -1: none
+                ck = np.full(plan.fwin.shape[0], -1, dtype=np.int32)
+                every_k = self.outer or 1
+                for i, (fa, _) in enumerate(plan.franges[::every_k]):
+                    ck[fa] = i
+                self.ckslot_dev = torch.from_numpy(ck).to(device)
         else:
             # the block starts (none with one block), then the saved states by slot: the state after run r of RF
             # windows in slot r mod `cap` (not in the workspace query: their count is the sequence's)
@@ -297,6 +307,10 @@ class Checkpointed:
             if self.saved.final:
                 self.slots[self.final_slot].copy_(state)
             return
+        if self.phys is None:  # one call, the checkpoints saved on the way
+            engine.run_forward(pk, state, plan.fwin_dev, 0, plan.fwin.shape[0], self.raw if pk.n_adc else None,
+                               self.status, wstates=self.ckpts, wslot=self.ckslot_dev, whole_runs=True)
+            return
         for k, (fa, fb) in enumerate(plan.franges):
             if not self.outer:
                 self.ckpts[k].copy_(state)
@@ -321,7 +335,55 @@ class Checkpointed:
         ph.wstates, ph.wstate_stride = None, 0
         _lib.check(code, "bp_forward_physics")
 
-    def buffers(self, need_seg: bool, want_gc: bool):
+    def sweeps(self, seg_mask: int, need_seg: bool) -> bool:
+        """Whether the backward runs ``bp_cotangent`` and ``bp_sweep`` (else ``bp_adjoint``)."""
+        offsets = need_seg and seg_mask & _lib.BP_SEG_ALL & ~(_lib.BP_SEG_WX | _lib.BP_SEG_WY)
+        return self.uniform and not offsets and (not need_seg or self.plan.max_len <= _lib.BP_SWEEP_MAX)
+
+    def sweep_buffers(self, h, spin_gradients: bool, want_gc: bool, need_seg: bool):
+        """The sweep's workspace: the cotangents split for the tensor cores, the runs' sums of one interval, the first
+        samples of its runs (with coil gradients) and the per-CTA RF gradient."""
+        pk, plan, b = self.pk, self.plan, {}
+        runs = pk.sample_runs()
+        if h is not None and runs.n_runs:
+            at = np.searchsorted(runs.starts, np.asarray(plan.seg_ranges, dtype=np.int64))
+            cap = max(int((at[:, 1] - at[:, 0]).max()), 1)
+            pair = lambda: torch.empty(cap, pk.n, 2, dtype=F32, device=self.dev)
+            b["hs"] = torch.empty(pk.n_adc, 8 * ((pk.n_coils + 7) // 8), dtype=torch.int64, device=self.dev)
+            b["most"] = torch.empty(1, dtype=torch.int32, device=self.dev)
+            b["g0"], b["cap"] = pair(), cap
+            b["g1"] = pair() if spin_gradients else None
+            b["z"] = pair() if want_gc else None
+            code = _lib.lib().bp_cotangent_split(ptr(h), pk.n_adc, pk.n_coils, ptr(b["hs"]), ptr(b["most"]),
+                                                 _lib.stream_ptr())
+            _lib.check(code, "bp_cotangent_split")
+        b["gseg"] = None
+        if need_seg:
+            rows = max(_lib.lib().bp_sweep_grid(pk.n, b1 - b0, int(spin_gradients))
+                       for b0, b1 in {(0, e - s) for s, e in plan.seg_ranges})
+            if rows < 1:
+                raise RuntimeError("bp_sweep_grid failed")
+            b["gseg"] = torch.empty(rows, plan.max_len, 2, dtype=F32, device=self.dev)
+        return b
+
+    def _sweep(self, k, b, states, wslot, chain, chain_in, lam, gs, gc, seg):
+        """Interval k's samples and its sweep from ``states``."""
+        pk, plan, lib, stream = self.pk, self.plan, _lib.lib(), _lib.stream_ptr()
+        aa, ab = plan.aranges[k]
+        s0, s1 = plan.seg_ranges[k]
+        runs = pk.sample_runs()
+        g0 = b.get("g0")
+        if g0 is not None:
+            code = lib.bp_cotangent(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64),
+                                    ptr(plan.awin_dev), aa, ab, ptr(runs.runs), runs.n_runs, ptr(b["hs"]),
+                                    ptr(b["most"]), ptr(g0), ptr(b["g1"]), ptr(b["z"]), ptr(gc), stream)
+            _lib.check(code, "bp_cotangent")
+        code = lib.bp_sweep(ptr(pk.spins), pk.n, ptr(pk.segs), ptr(pk.seg64), ptr(plan.awin_dev), aa, ab, s0, s1 - s0,
+                            ptr(states), ptr(wslot), ptr(chain), chain_in, ptr(runs.runs), runs.n_runs, ptr(g0),
+                            ptr(b.get("g1")), ptr(lam), ptr(gs), ptr(b["gseg"]), ptr(seg), ptr(self.status), stream)
+        _lib.check(code, "bp_sweep")
+
+    def buffers(self, need_seg: bool, want_gc: bool, sweeps: bool = False):
         pk, plan, ws, dev = self.pk, self.plan, self.ws, self.dev
         if self._bufs is None:
             self._bufs = {"gs": sized(ws.gs, (8, pk.n), F32, dev), "seg": sized(ws.seg, (pk.flags.shape[0], 8), F64, dev)}
@@ -333,7 +395,7 @@ class Checkpointed:
                 if self.n_block_states:
                     self._bufs["state"] = sized(ws.replay_state, (6, pk.n), F32, dev)
         b = self._bufs
-        if need_seg and "gseg" not in b:
+        if need_seg and not sweeps and "gseg" not in b:
             b["gseg"] = sized(ws.gseg, (self.grid, plan.max_len, 8), F32, dev)
         if want_gc and "gc" not in b:
             b["gc"] = sized(ws.gc, (2 * pk.n_coils, pk.n), F32, dev)
@@ -345,17 +407,19 @@ class Checkpointed:
         ``lam`` = dL/dm at the end ([3][n], turned into dL/dm at the start in place). Asynchronous: the status word
         is checked by ``check``."""
         pk, plan = self.pk, self.plan
-        b = self.buffers(need_seg, want_gc)
+        sweeps = self.sweeps(seg_mask, need_seg)
+        b = self.buffers(need_seg, want_gc, sweeps)
         gs, seg, wstates, state = b["gs"], b["seg"], b.get("wstates"), b.get("state")
-        gc, gseg = (b["gc"] if want_gc else None), (b["gseg"] if need_seg else None)
+        gc, gseg = (b["gc"] if want_gc else None), (b["gseg"] if need_seg and not sweeps else None)
         gs.zero_()
         seg.zero_()
         if gc is not None:
             gc.zero_()
         if self.phys is not None and self.phys.gconc is not None:
             self.phys.gconc.zero_()
+        swept = self.sweep_buffers(h, self.saved is None, want_gc, need_seg) if sweeps else None
         if self.saved is not None:
-            self._saved_backward(h, lam, gseg if need_seg else None, seg, seg_mask, want_gc, b["chain"], state)
+            self._saved_backward(h, lam, gseg, seg, seg_mask, want_gc, b["chain"], state, swept)
             return gs, gc, seg
         n_blocks = len(self.blocks())
         for bi, (ka, kb) in reversed(list(enumerate(self.blocks()))):
@@ -368,18 +432,29 @@ class Checkpointed:
                         self._fwd(state, plan.fwin_dev, fa, fb, None)
             for k in reversed(range(ka, kb)):
                 self._interval(k, n_blocks + k - ka if self.outer else k, h, lam, gs, gc, gseg, seg, seg_mask,
-                               need_seg, wstates, state)
+                               need_seg, wstates, state, swept)
         return gs, gc, seg
 
-    def _interval(self, k, ck, h, lam, gs, gc, gseg, seg, seg_mask, need_seg, wstates, state):
+    def _interval(self, k, ck, h, lam, gs, gc, gseg, seg, seg_mask, need_seg, wstates, state, swept=None):
         """Interval k from checkpoint ``ck``: replay with window states, the reverse sweep, the segment reduction."""
         pk, plan = self.pk, self.plan
         lib, stream, n, C, A = _lib.lib(), _lib.stream_ptr(), pk.n, pk.n_coils, pk.n_adc
         aa, ab = plan.aranges[k]
         s0, s1 = plan.seg_ranges[k]
         state.copy_(self.ckpts[ck])
-        self._fwd(state, plan.awin_dev, aa, ab, None, wstates=wstates)
+        z = None if swept is None else swept.get("z")
+        if z is None:
+            self._fwd(state, plan.awin_dev, aa, ab, None, wstates=wstates)
+        else:  # with the first samples of the interval's runs
+            runs = pk.sample_runs()
+            code = lib.bp_propagate(ptr(pk.spins), n, ptr(pk.segs), ptr(pk.seg64), ptr(plan.awin_dev), aa, ab, ptr(state),
+                                    ptr(wstates), 1, None, ptr(runs.runs), runs.n_runs, ptr(z), swept["cap"], 0, 0,
+                                    ptr(self.status), stream)
+            _lib.check(code, "bp_propagate")
         wstates[ab - aa].copy_(state)  # the state after the interval's last window
+        if swept is not None:
+            self._sweep(k, swept, wstates, None, None, 0, lam, gs, gc, seg)
+            return
         if self.phys is None:
             code = lib.bp_adjoint(ptr(pk.spins), ptr(pk.sens), n, C, ptr(pk.segs), ptr(pk.seg64), ptr(plan.awin_dev),
                                   aa, ab, s0, s1 - s0, ptr(wstates), ptr(h), A, ptr(lam), ptr(gs), ptr(gc), ptr(gseg),
@@ -395,7 +470,7 @@ class Checkpointed:
         if need_seg:
             _lib.check(lib.bp_seg_reduce(ptr(gseg), self.grid, s1 - s0, s0, ptr(seg), stream), "bp_seg_reduce")
 
-    def _saved_backward(self, h, lam, gseg, seg, seg_mask, want_gc, chain, state):
+    def _saved_backward(self, h, lam, gseg, seg, seg_mask, want_gc, chain, state, swept=None):
         """The backward without a replay: per block in reverse, its saved states (rebuilt by one forward of the
         block from its start, except the last block's, which the forward left), then per interval in reverse the
         sweep from the saved states, carrying the chain of RF windows integrated backward across the intervals,
@@ -413,6 +488,9 @@ class Checkpointed:
                 aa, ab = plan.aranges[k]
                 s0, s1 = plan.seg_ranges[k]
                 chain_in = int(ab < W and bool(sv.rf[ab]))
+                if swept is not None:
+                    self._sweep(k, swept, self.slots, self.aslot_dev, chain, chain_in, lam, None, None, seg)
+                    continue
                 code = lib.bp_adjoint_saved(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs),
                                             ptr(pk.seg64), ptr(plan.awin_dev), aa, ab, s0, s1 - s0, ptr(self.slots),
                                             ptr(self.aslot_dev), ptr(chain), chain_in, ptr(h), pk.n_adc, ptr(lam),
@@ -425,11 +503,14 @@ class Checkpointed:
     def launches(self, need_seg: bool) -> tuple[int, int]:
         """(forward, backward) kernel launches of one call each."""
         k = len(self.plan.starts)
+        readout = int(self.pk.n_adc > 0)
+        swept = 2 * readout + k * (1 + readout + int(need_seg))  # the split, then per interval samples, sweep, sums
         if self.saved is not None:
             nb = len(self.blocks())
-            return nb, nb - 1 + k * (2 if need_seg else 1)
+            return nb * (1 + readout), nb - 1 + (swept if self.uniform else k * (2 if need_seg else 1))
         rebuild = sum(kb - ka - 1 for ka, kb in self.blocks()) if self.outer else 0
-        return k, k * (3 if need_seg else 2) + rebuild
+        forward = k if self.phys is not None else 1 + readout
+        return forward, rebuild + (k + swept if self.uniform else k * (3 if need_seg else 2))
 
     def check(self, what: str = "bp_forward / bp_adjoint") -> None:
         torch.cuda.synchronize(self.dev)

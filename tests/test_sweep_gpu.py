@@ -1,0 +1,124 @@
+"""The sweep over runs of like segments (``bp_cotangent``, ``bp_sweep``): gradients against the float64 oracle's
+autograd, and against the segment-by-segment sweep (``bp_adjoint``) where the oracle would take long. The bar is the
+gradient tests' 2e-4 of a gradient's largest value (float32 states in a reverse sweep; 1e-5 to 5e-5 here)."""
+
+from dataclasses import replace
+
+import numpy as np
+import pytest
+import torch
+
+import blochparty_b200 as bpb
+from blochparty_b200 import adjoint, sequences
+from oracle import bloch
+
+pytestmark = pytest.mark.gpu
+F64 = torch.float64
+
+
+def _phantom(n, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    rnd = lambda *s: torch.rand(*s, generator=g, dtype=F64)
+    f32 = lambda t: t.float().double()
+    return bpb.Phantom(f32((rnd(n, 3) - 0.5) * 0.2), f32(0.5 + rnd(n)), f32(0.2 + rnd(n)), f32(0.03 + 0.1 * rnd(n)),
+                       f32((rnd(n) - 0.5) * 200), f32(0.8 + 0.4 * rnd(n)))
+
+
+def _sequence(lengths, rf_steps=37, seed=1):
+    """Pulses of one offset, readouts of the given lengths (a first half dwell, or none), a spoil on a sample, a
+    readout that follows another at once, and samples that stop and go within one set of factors."""
+    g = np.random.RandomState(seed)
+    b = sequences.SequenceBuilder()
+    for i, k in enumerate(lengths):
+        b.rf_waveform((g.rand(rf_steps, 2) - 0.4) * 2500 * (10 if i % 2 else 1), 10e-6, grad=(300.0, 0.0, 1000.0))
+        b.delay(0.3e-3, grad=(2000.0, float(g.rand() - 0.5) * 3000, 0.0))
+        b.readout(k, 10e-6, grad=(-2500.0, 300.0, 400.0), phase=0.3 * i)
+        if i % 3 == 0 and k > 4:
+            b._adc[-4] = False  # a gap in the samples of one set of factors
+        if i % 3 == 1:
+            b._adc[-1] = True
+            b.readout(3, 20e-6, grad=(100.0, 0.0, 0.0))
+        if i % 3 == 2:
+            b._spoil[-2] = True  # the last sample spoils
+            b._append(np.full(5, 20e-6), (0.0, 0.0), (500.0, 0.0, 0.0), 0.1, False, True)  # samples from the first on
+        b.delay(1e-3, grad=(g.rand(3) - 0.5) * 8000)
+        b.spoil()
+    return b.build()
+
+
+def _coils(n, c, seed=2):
+    g = torch.Generator().manual_seed(seed)
+    rnd = lambda: torch.rand(n, c, generator=g, dtype=F64).float().double() - 0.5
+    return torch.complex(rnd(), rnd())
+
+
+def _gradients(ph, seq, coils, names, every=None):
+    ph = replace(ph, **{k: getattr(ph, k).clone().requires_grad_() for k in names if k not in ("rf", "coils")})
+    if "rf" in names:
+        seq = replace(seq, rf=seq.rf.clone().requires_grad_())
+    if "coils" in names:
+        coils = coils.clone().requires_grad_()
+    r = bpb.simulate(ph, seq, coils, checkpoint_every=every)
+    leaves = [seq.rf if k == "rf" else coils if k == "coils" else getattr(ph, k) for k in names]
+    return dict(zip(names, torch.autograd.grad(_loss(r.signal, r.m), leaves)))
+
+
+def _loss(sig, m):
+    g = torch.Generator().manual_seed(5)
+    w = torch.randn(sig.shape, generator=g, dtype=F64) * (1.0 + 100.0 * (torch.arange(sig.shape[1]) % 17 == 3))
+    return (sig.real.double() * w).sum() + 0.5 * (sig.imag.double() * w.flip(1)).sum() + 3.0 * (m.double() ** 2).sum()
+
+
+def _spy(monkeypatch, force=None):
+    seen = []
+    sweeps = adjoint.Checkpointed.sweeps
+
+    def spy(self, *a):
+        v = sweeps(self, *a) if force is None else force
+        seen.append(v)
+        return v
+
+    monkeypatch.setattr(adjoint.Checkpointed, "sweeps", spy)
+    return seen
+
+
+def _close(a, b, names, bar=2e-4):
+    for k in names:
+        u, v = (torch.view_as_real(t) if t.is_complex() else t for t in (a[k], b[k]))
+        err = float((u - v).abs().max() / v.abs().max())
+        assert err < bar, (k, err)
+
+
+@pytest.mark.parametrize("n,coils,lengths,names", [
+    (33, 8, (8, 9, 33), ("pd", "t1", "t2", "db0", "b1", "coils", "pos")),
+    (100, 1, (1, 2, 5, 31), ("t1", "rf")),
+    (129, 9, (95, 64, 130), ("rf", "coils")),
+    (61, 17, (40, 32, 16), ("pd", "t1", "t2", "db0", "b1", "rf")),
+    (64, 8, (300, 20, 7), ("rf",)),
+    (40, 3, (260, 12, 45), ("t2", "db0", "coils")),
+])
+def test_against_the_oracle(n, coils, lengths, names, monkeypatch):
+    seen = _spy(monkeypatch)
+    ph, seq, c = _phantom(n), _sequence(lengths), _coils(n, coils)
+    got = _gradients(ph, seq, c, names, every=64)
+    assert seen and all(seen)
+    again = _gradients(ph, seq, c, names, every=32 * 100)
+    for k in names:  # the same bits wherever the checkpoints lie
+        assert torch.equal(got[k], again[k]), k
+    _, want = bloch.gradients(bloch.case_from(ph, seq, c), _loss, names)
+    _close(got, want, names)
+
+
+@pytest.mark.parametrize("n", [37888, 37889, 40001])
+@pytest.mark.parametrize("names", [("rf",), ("t1", "t2", "db0", "coils"), ("pd", "b1", "rf")])
+def test_against_the_segment_sweep(n, names, monkeypatch):
+    """Both spin layouts of the kernels, at and past the line between them."""
+    ph, seq, c = _phantom(n, 3), _sequence((17, 64), rf_steps=70), _coils(n, 8)
+    with monkeypatch.context() as m:
+        seen = _spy(m)
+        got = _gradients(ph, seq, c, names)
+        assert seen and all(seen)
+    with monkeypatch.context() as m:
+        _spy(m, force=False)
+        want = _gradients(ph, seq, c, names)
+    _close(got, want, names)
