@@ -223,7 +223,7 @@ class Checkpointed:
     buffers are allocated on its first call and reused."""
 
     def __init__(self, pk: engine.Packed, every: int, device, outer: int = 0, phys=None, saved: bool = False,
-                 budget_bytes: int | None = None):
+                 budget_bytes: int | None = None, keep: bool = False):
         self.pk, self.dev = pk, device
         self.phys = phys  # the field model (``PhysGrad``): the forward, replay and sweep take its variants
         # saved: the caller wants the RF waveform's gradient alone; then, where the sequence's windows allow it, the
@@ -240,22 +240,37 @@ class Checkpointed:
             if budget_bytes is None:
                 budget_bytes = torch.cuda.mem_get_info(device)[0] // 2 if torch.cuda.is_available() else 1 << 62
             self.layout = saved_layout(plan, 24 * pk.n, budget_bytes)
-        if self.layout is None:
+        # keep: the caller leaves the stored states to this class; then, where the sweep takes a window in one step and
+        # the states fit a quarter of the free memory, the forward saves the state at every adjoint window's start and
+        # the backward replays nothing (its intervals are as long as the sweep takes)
+        self.kept = None
+        if self.layout is None and keep and invertible:
+            plan = Plan(pk, _lib.BP_SWEEP_MAX, device)
+            room = torch.cuda.mem_get_info(device)[0] // 4 if torch.cuda.is_available() else 0
+            uniform = SavedStates.of(pk.flags, plan.awin) is not None
+            if (uniform and 24 * pk.n * (plan.awin.shape[0] + 1) <= room
+                    and 8 * pk.n * pk.sample_runs().n_runs <= min(engine.Z_BYTES, room)):
+                self.kept = torch.empty(plan.awin.shape[0] + 1, 6, pk.n, dtype=F32, device=device)
+        if self.layout is None and self.kept is None:
             plan = Plan(pk, every, device)
         self.plan = plan
         self.saved = plan.saved
         # whether every adjoint window is one run of RF or of free segments: then the gradients that need no
         # per-segment sums but the RF waveform's take a window in one step (bp_cotangent, bp_sweep)
-        self.uniform = invertible and (plan.saved is not None or SavedStates.of(pk.flags, plan.awin) is not None)
+        self.uniform = invertible and (plan.saved is not None or self.kept is not None
+                                       or SavedStates.of(pk.flags, plan.awin) is not None)
         k = len(plan.starts)
-        self.outer = outer if outer > 1 and k > outer and self.saved is None else 0
+        self.outer = outer if outer > 1 and k > outer and self.saved is None and self.kept is None else 0
         fws = _lib.forward_workspace(pk.n, pk.n_adc, pk.n_coils)
         self.grid = _lib.lib().bp_adjoint_grid(pk.n, pk.n_coils)
         if self.grid < 1:
             raise RuntimeError("bp_adjoint_grid failed")
         self.ws = _lib.adjoint_workspace(pk.n, pk.flags.shape[0], pk.n_adc, pk.n_coils, plan.every, plan.max_aw,
                                          self.grid, self.outer)
-        if self.saved is None:
+        self.z = None  # kept: the first samples of the forward's runs
+        if self.kept is not None:
+            pass
+        elif self.saved is None:
             # interval starts (two levels), or block starts followed by one block's interval starts (three)
             n_states = k if not self.outer else (k + self.outer - 1) // self.outer + self.outer
             self.ckpts = sized(self.ws.checkpoints, (n_states, 6, pk.n), F32, device)
@@ -307,6 +322,12 @@ class Checkpointed:
             if self.saved.final:
                 self.slots[self.final_slot].copy_(state)
             return
+        if self.kept is not None:
+            W = plan.awin.shape[0]
+            self.z = engine.run_forward(pk, state, plan.awin_dev, 0, W, self.raw if pk.n_adc else None, self.status,
+                                        wstates=self.kept, whole_runs=True)
+            self.kept[W].copy_(state)
+            return
         if self.phys is None:  # one call, the checkpoints saved on the way
             engine.run_forward(pk, state, plan.fwin_dev, 0, plan.fwin.shape[0], self.raw if pk.n_adc else None,
                                self.status, wstates=self.ckpts, wslot=self.ckslot_dev, whole_runs=True)
@@ -353,7 +374,7 @@ class Checkpointed:
             b["most"] = torch.empty(1, dtype=torch.int32, device=self.dev)
             b["g0"], b["cap"] = pair(), cap
             b["g1"] = pair() if spin_gradients else None
-            b["z"] = pair() if want_gc else None
+            b["z"] = pair() if want_gc and self.kept is None else None
             code = _lib.lib().bp_cotangent_split(ptr(h), pk.n_adc, pk.n_coils, ptr(b["hs"]), ptr(b["most"]),
                                                  _lib.stream_ptr())
             _lib.check(code, "bp_cotangent_split")
@@ -366,8 +387,8 @@ class Checkpointed:
             b["gseg"] = torch.empty(rows, plan.max_len, 2, dtype=F32, device=self.dev)
         return b
 
-    def _sweep(self, k, b, states, wslot, chain, chain_in, lam, gs, gc, seg):
-        """Interval k's samples and its sweep from ``states``."""
+    def _sweep(self, k, b, states, wslot, chain, chain_in, lam, gs, gc, seg, z=None):
+        """Interval k's samples (``z``: its runs' first samples, with coil gradients) and its sweep from ``states``."""
         pk, plan, lib, stream = self.pk, self.plan, _lib.lib(), _lib.stream_ptr()
         aa, ab = plan.aranges[k]
         s0, s1 = plan.seg_ranges[k]
@@ -376,7 +397,7 @@ class Checkpointed:
         if g0 is not None:
             code = lib.bp_cotangent(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64),
                                     ptr(plan.awin_dev), aa, ab, ptr(runs.runs), runs.n_runs, ptr(b["hs"]),
-                                    ptr(b["most"]), ptr(g0), ptr(b["g1"]), ptr(b["z"]), ptr(gc), stream)
+                                    ptr(b["most"]), ptr(g0), ptr(b["g1"]), ptr(z), ptr(gc), stream)
             _lib.check(code, "bp_cotangent")
         code = lib.bp_sweep(ptr(pk.spins), pk.n, ptr(pk.segs), ptr(pk.seg64), ptr(plan.awin_dev), aa, ab, s0, s1 - s0,
                             ptr(states), ptr(wslot), ptr(chain), chain_in, ptr(runs.runs), runs.n_runs, ptr(g0),
@@ -387,7 +408,9 @@ class Checkpointed:
         pk, plan, ws, dev = self.pk, self.plan, self.ws, self.dev
         if self._bufs is None:
             self._bufs = {"gs": sized(ws.gs, (8, pk.n), F32, dev), "seg": sized(ws.seg, (pk.flags.shape[0], 8), F64, dev)}
-            if self.saved is None:
+            if self.kept is not None and sweeps:
+                pass
+            elif self.saved is None:
                 self._bufs["wstates"] = sized(ws.wstates, (plan.max_aw + 1, 6, pk.n), F32, dev)
                 self._bufs["state"] = sized(ws.replay_state, (6, pk.n), F32, dev)
             else:  # the chain's state between intervals, the rebuild's state
@@ -395,6 +418,8 @@ class Checkpointed:
                 if self.n_block_states:
                     self._bufs["state"] = sized(ws.replay_state, (6, pk.n), F32, dev)
         b = self._bufs
+        if self.kept is not None and not sweeps and "wstates" not in b:
+            raise RuntimeError("the states of every window are kept for the sweep over runs alone")
         if need_seg and not sweeps and "gseg" not in b:
             b["gseg"] = sized(ws.gseg, (self.grid, plan.max_len, 8), F32, dev)
         if want_gc and "gc" not in b:
@@ -441,6 +466,10 @@ class Checkpointed:
         lib, stream, n, C, A = _lib.lib(), _lib.stream_ptr(), pk.n, pk.n_coils, pk.n_adc
         aa, ab = plan.aranges[k]
         s0, s1 = plan.seg_ranges[k]
+        if self.kept is not None:  # every state is there
+            z = None if self.z is None else self.z[int(np.searchsorted(pk.sample_runs().starts, s0)):]
+            self._sweep(k, swept, self.kept[aa:], None, None, 0, lam, gs, gc, seg, z)
+            return
         state.copy_(self.ckpts[ck])
         z = None if swept is None else swept.get("z")
         if z is None:
@@ -453,7 +482,7 @@ class Checkpointed:
             _lib.check(code, "bp_propagate")
         wstates[ab - aa].copy_(state)  # the state after the interval's last window
         if swept is not None:
-            self._sweep(k, swept, wstates, None, None, 0, lam, gs, gc, seg)
+            self._sweep(k, swept, wstates, None, None, 0, lam, gs, gc, seg, z)
             return
         if self.phys is None:
             code = lib.bp_adjoint(ptr(pk.spins), ptr(pk.sens), n, C, ptr(pk.segs), ptr(pk.seg64), ptr(plan.awin_dev),
@@ -508,6 +537,8 @@ class Checkpointed:
         if self.saved is not None:
             nb = len(self.blocks())
             return nb * (1 + readout), nb - 1 + (swept if self.uniform else k * (2 if need_seg else 1))
+        if self.kept is not None:
+            return 1 + readout, swept
         rebuild = sum(kb - ka - 1 for ka, kb in self.blocks()) if self.outer else 0
         forward = k if self.phys is not None else 1 + readout
         return forward, rebuild + (k + swept if self.uniform else k * (3 if need_seg else 2))
@@ -576,14 +607,16 @@ class _Simulate(torch.autograd.Function):
         d = lambda t: None if t is None else t.detach()
         inp = Inputs(d(pos), d(pd), d(t1), d(t2), d(db0), d(b1), coils, d(dt), d(rf), d(grad), d(adc_phase),
                      d(b0_offset), *flags_in, d(m0))
-        pk = engine.pack(inp, dev)
+        pk, state = engine.pack_with_state(inp, dev)
         phys = None
         if conc is not None:  # the field model's concomitant coefficients (positions: the encoding ones)
             phys = PhysGrad(conc, opts["conc_mode"], inp.dt, inp.grad, dev, ctx.needs_input_grad[14])
-        # the RF waveform's gradient alone: the backward from saved states where the sequence allows it
+        # the RF waveform's gradient alone: the backward from saved states where the sequence allows it; without
+        # per-segment gradients but the RF's and an interval of the caller's, every state kept where they fit
+        need = ctx.needs_input_grad
         run = Checkpointed(pk, every, dev, opts.get("outer", 0), phys,
-                           saved=opts.get("saved", True) and rf_only(seg_mask_for(ctx.needs_input_grad)))
-        state = engine.initial_state(inp.pd, inp.m_init, dev)
+                           saved=opts.get("saved", True) and rf_only(seg_mask_for(need)),
+                           keep=opts.get("keep", False) and not (need[8] or need[10] or need[12]))
         run.forward(state)
         sig = engine.finish_signal(pk, run.raw)
         run.check("bp_forward")
@@ -698,7 +731,7 @@ def _apply(inp, dev, checkpoint_every, raw: bool, scanner=None):
         m0 = torch.stack([z, z, inp.pd], -1)
     coils_ri = torch.view_as_real(inp.coils if inp.coils.is_complex() else inp.coils.to(torch.complex64))
     opts = {"device": dev, "every": every, "outer": outer, "flags": (inp.is_rf, inp.adc, inp.spoil), "raw": raw,
-            "conc_mode": mode}
+            "conc_mode": mode, "keep": not checkpoint_every}
     return _Simulate.apply(opts, inp.pos, inp.pd, inp.t1, inp.t2, inp.db0, inp.b1, coils_ri, inp.dt, inp.rf, inp.grad,
                            inp.adc_phase, inp.b0_offset, m0, conc)
 

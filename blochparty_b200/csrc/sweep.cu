@@ -348,6 +348,9 @@ template <int K, int NT, bool SG>
 __global__ void __launch_bounds__(NT, NT == 32 ? 8 : 4) bp_sweep_kernel(SweepArgs a) {
     extern __shared__ __align__(16) float iacc[];  // [seg_len][2]: the RF gradient, summed over the CTA's tiles
     __shared__ float segacc[NT / 32][SW_WIN][2];
+    __shared__ int4 win_s[32];     // of up to 32 windows: begin, end (begin: none to sweep), the last segment's flags
+    __shared__ SegRec rec_s[32];   // and their first segments' records
+    __shared__ double4 k64_s[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = a.n;
     constexpr int TILE = NT * K;
@@ -394,21 +397,69 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : 4) bp_sweep_kernel(SweepArg
                     v[i][k] = active[k] ? st[(size_t)i * n + jk[k]] + st[(size_t)(3 + i) * n + jk[k]] : 0.0f;
             x = pmake<K>(v[0]), y = pmake<K>(v[1]), z = pmake<K>(v[2]);
         };
-        int run = hi - 1;
-        int next = run >= lo ? a.runs[run].x : -1;  // the last run not yet met, and its first segment
+        // the last run not yet met: its first segment and what its samples add, read as soon as the one after it is done
+        int run, next;
+        float2 add0[K], add1;
+        SegRec rq{};
+        auto meet = [&](int r) {
+            run = r, next = -1;
+            if (r < lo) return;
+            const int4 rr = a.runs[r];
+            next = rr.x;
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                add0[k] = active[k] ? a.g0[(size_t)(r - lo) * n + jk[k]] : make_float2(0.0f, 0.0f);
+            if constexpr (SG) {
+                add1 = active[0] ? a.g1[(size_t)(r - lo) * n + jk[0]] : make_float2(0.0f, 0.0f);
+                rq = a.segs[rr.y >= 0 ? rr.y : rr.x];  // (a single sample's add1 is 0)
+            }
+        };
+        meet(hi - 1);
+        // windows [blk, ...) are staged in `win_s` and the rest; the state at a window's start is read one window ahead
+        float ahead[6];
+        auto read_ahead = [&](int w) {
+#pragma unroll
+            for (int i = 0; i < 6; ++i) ahead[i] = 0.0f;
+            if (SG && w >= a.wa && active[0]) {
+                const float* st = a.wstates + (size_t)(w - a.wa) * 6 * n + jk[0];
+#pragma unroll
+                for (int i = 0; i < 6; ++i) ahead[i] = st[(size_t)i * n];
+            }
+        };
+        Pk<K> x0 = pset<K>(0.0f), y0 = x0, z0 = x0;  // SG: the state at the start of the window after this one
+        if (SG) load_state(a.wstates + (size_t)(a.wb - a.wa) * 6 * n, x0, y0, z0);
+        read_ahead(a.wb - 1);
+        int blk = a.wb;
         for (int w = a.wb - 1; w >= a.wa; --w) {
-            const int4 win = a.windows[w];
+            if (w < blk) {  // the records of up to 32 windows at once: their loads' latency once
+                blk = max(a.wa, w - 31);
+                __syncthreads();
+                if (tid < w - blk + 1) {
+                    const int4 v = a.windows[blk + tid];
+                    const bool fine = v.y > v.x && v.y - v.x <= SW_WIN && v.x >= a.seg0 && v.y <= a.seg0 + a.seg_len;
+                    win_s[tid] = make_int4(v.x, fine ? v.y : v.x, fine ? a.segs[v.y - 1].flags : 0, 0);
+                    if (fine) rec_s[tid] = a.segs[v.x], k64_s[tid] = a.seg64[v.x];
+                }
+                __syncthreads();
+            }
+            const int4 win = win_s[w - blk];
             const int nseg = win.y - win.x;
-            if (nseg <= 0 || nseg > SW_WIN || win.x < a.seg0 || win.y > a.seg0 + a.seg_len) {  // (uniform)
+            // SG: this window's start state (read ahead), and the next one's on its way
+            const Pk<K> ex = x0, ey = y0, ez = z0;  // the state after the window
+            if constexpr (SG) {
+                x0 = Pk<K>{ahead[0] + ahead[3]}, y0 = Pk<K>{ahead[1] + ahead[4]}, z0 = Pk<K>{ahead[2] + ahead[5]};
+                read_ahead(w - 1);
+            }
+            if (nseg <= 0) {  // (uniform) not a window of this interval
                 if (tid == 0) atomicOr(a.status, BP_ERR_BAD_WINDOW);
                 continue;
             }
-            const SegRec q = a.segs[win.x];
-            const int last = a.segs[win.y - 1].flags;
+            const SegRec q = rec_s[w - blk];
+            const int last = win.z;
             if (q.flags & BP_RF) {
                 Pk<K> ox = cx, oy = cy, oz = cz;  // the state after the window
                 if (SG) {
-                    load_state(a.wstates + (size_t)(w - a.wa + 1) * 6 * n, ox, oy, oz);
+                    ox = ex, oy = ey, oz = ez;
                 } else if (!chained) {
                     const int sl = a.wslot[w + 1];
                     if (sl < 0)
@@ -431,10 +482,15 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : 4) bp_sweep_kernel(SweepArg
                 rb.a1 = pmake<K>(a1), rb.a2 = pmake<K>(a2), rb.ia1 = pmake<K>(i1), rb.ia2 = pmake<K>(i2);
                 rb.pe = pmake<K>(pe), rb.npe = pmake<K>(npe);
                 rb.wz = pmake<K>(wz), rb.nwz = pmake<K>(nwz), rb.wz2 = pmake<K>(wz2);
-                // every rotation small for every spin of the warp: |w|^2 <= b1^2 max(wx0^2 + wy0^2) + wz^2
+                // the window's RF, a segment per lane (its other values are the first segment's); every rotation small for
+                // every spin of the warp: |w|^2 <= b1^2 max(wx0^2 + wy0^2) + wz^2
+                float rfx = q.wx0, rfy = q.wy0;
+                if (nseg > 1) {
+                    const SegRec* qs = a.segs + min(win.x + lane, win.y - 1);
+                    rfx = qs->wx0, rfy = qs->wy0;
+                }
                 {
-                    const SegRec qs = a.segs[min(win.x + lane, win.y - 1)];
-                    const float v = fmaf(qs.wx0, qs.wx0, qs.wy0 * qs.wy0);
+                    const float v = fmaf(rfx, rfx, rfy * rfy);
                     const float top = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
 #pragma unroll
                     for (int k = 0; k < K; ++k) small = small && fmaf(bp[k] * bp[k], top, wz2[k]) < 0.0624f;
@@ -442,10 +498,10 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : 4) bp_sweep_kernel(SweepArg
                 }
                 auto back = [&](auto tag) {
                     for (int s = nseg - 1; s >= 0; --s) {
-                        const SegRec qs = a.segs[win.x + s];
                         Pk<K> gx, gy;
-                        rf_back_packed<decltype(tag)::value, SG>(pset<K>(qs.wx0), pset<K>(qs.wy0), b1, nb1, rb, p, qs, ox,
-                                                                 oy, oz, lx, ly, lz, gx, gy, g);
+                        rf_back_packed<decltype(tag)::value, SG>(pset<K>(__shfl_sync(0xffffffffu, rfx, s)),
+                                                                 pset<K>(__shfl_sync(0xffffffffu, rfy, s)), b1, nb1, rb, p,
+                                                                 q, ox, oy, oz, lx, ly, lz, gx, gy, g);
                         if (a.gseg) {  // dL/d(-2 pi dt rf), summed over the warp: x into lane 0, y into lane 16
                             const Pk<K> vx = pmul(gx, b1), vy = pmul(gy, b1);
                             float v0 = active[0] ? vx.get(0) : 0.0f, v1 = active[0] ? vy.get(0) : 0.0f;
@@ -477,13 +533,11 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : 4) bp_sweep_kernel(SweepArg
             }
             chained = false;
             if (last & BP_SPOIL) lx = ly = pset<K>(0.0f);
-            const double4 k64 = a.seg64[win.x];
-            Pk<K> x0, y0, z0;  // the state at the window's start
-            if (SG) load_state(a.wstates + (size_t)(w - a.wa) * 6 * n, x0, y0, z0);
+            const double4 k64 = k64_s[w - blk];
             int cur = nseg;
             while (cur > 0) {
                 // segments [from, cur) in one step: back to the last run that starts in the window, or to its start
-                const bool at_run = next >= win.x && a.g0 != nullptr;
+                const bool at_run = next >= win.x;
                 const int from = at_run ? next - win.x + 1 : 0, reps = cur - from;
                 float v[3][K];
 #pragma unroll
@@ -512,32 +566,22 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : 4) bp_sweep_kernel(SweepArg
                         }
                     }
                     if (at_run) {  // the run's samples
-                        const size_t at = (size_t)(run - lo) * n + jk[k];
-                        const float2 g0 = active[k] ? a.g0[at] : make_float2(0.0f, 0.0f);
-                        v[0][k] += g0.x, v[1][k] += g0.y;
-                        if constexpr (SG) {
-                            const int4 rr = a.runs[run];
-                            if (rr.y >= 0) {
-                                const FreeFactors u = prop_factors(q.dt, k64, p[0], from);
-                                const float a2 = 1.0f + u.e2;
-                                const float mx = a2 * fmaf(u.ch, x0.f, -u.sh * y0.f), my = a2 * fmaf(u.sh, x0.f, u.ch * y0.f);
-                                const float2 g1 = active[0] ? a.g1[at] : make_float2(0.0f, 0.0f);
-                                const SegRec qr = a.segs[rr.y];
-                                const float re = fmaf(g1.x, mx, g1.y * my);
-                                const float gcyc = -BP_TWO_PI_F * fmaf(g1.y, mx, -g1.x * my);
-                                g[6] = fmaf(-qr.dt, re, g[6]);
-                                g[0] = fmaf(gcyc, qr.kx, g[0]), g[1] = fmaf(gcyc, qr.ky, g[1]);
-                                g[2] = fmaf(gcyc, qr.kz, g[2]), g[3] = fmaf(gcyc, qr.dt, g[3]);
-                            }
+                        v[0][k] += add0[k].x, v[1][k] += add0[k].y;
+                        if constexpr (SG) {  // and its later segments' phase and decay
+                            const FreeFactors u = prop_factors(q.dt, k64, p[0], from);
+                            const float a2 = 1.0f + u.e2;
+                            const float mx = a2 * fmaf(u.ch, x0.f, -u.sh * y0.f), my = a2 * fmaf(u.sh, x0.f, u.ch * y0.f);
+                            const float re = fmaf(add1.x, mx, add1.y * my);
+                            const float gcyc = -BP_TWO_PI_F * fmaf(add1.y, mx, -add1.x * my);
+                            g[6] = fmaf(-rq.dt, re, g[6]);
+                            g[0] = fmaf(gcyc, rq.kx, g[0]), g[1] = fmaf(gcyc, rq.ky, g[1]);
+                            g[2] = fmaf(gcyc, rq.kz, g[2]), g[3] = fmaf(gcyc, rq.dt, g[3]);
                         }
                     }
                 }
                 lx = pmake<K>(v[0]), ly = pmake<K>(v[1]), lz = pmake<K>(v[2]);
                 cur = from;
-                if (at_run) {
-                    --run;
-                    next = run >= lo ? a.runs[run].x : -1;
-                }
+                if (at_run) meet(run - 1);
             }
         }
         if (lost && lane == 0) atomicOr(a.status, BP_ERR_NO_STATE);

@@ -287,12 +287,13 @@ def pack(case, device) -> Packed:
 def run_forward(pk: Packed, state: torch.Tensor, windows_dev: torch.Tensor, w_begin: int, w_end: int,
                 raw: torch.Tensor | None, status: torch.Tensor, wstates: torch.Tensor | None = None,
                 wstate_stride: int = 1, max_ctas: int = 0, wslot: torch.Tensor | None = None,
-                whole_runs: bool = False) -> None:
+                whole_runs: bool = False) -> torch.Tensor | None:
     """The forward over windows [w_begin, w_end) from ``state``, advanced in place: ``bp_propagate``, then with
     ``raw`` (the coil sums, added to) ``bp_readout``, over as many windows at a time as keep the workspace between
     them under ``Z_BYTES``. ``wstates``: states at window starts, every ``wstate_stride``-th or by slot (``wslot``).
     ``whole_runs``: a run of samples is formed whole by the call whose windows it starts in (calls over consecutive
-    windows then give the same bits wherever they are divided); else the windows' samples alone."""
+    windows then give the same bits wherever they are divided); else the windows' samples alone. Returns the workspace
+    (the runs' first samples, [run][N] pairs) when one launch took all windows."""
     lib, stream = _lib.lib(), _lib.stream_ptr()
     runs = pk.sample_runs() if raw is not None else None
     step, cap, z = max(w_end - w_begin, 1), 0, None
@@ -324,6 +325,7 @@ def run_forward(pk: Packed, state: torch.Tensor, windows_dev: torch.Tensor, w_be
                                   ptr(windows_dev), wa, wb, ptr(runs.runs), runs.n_runs, ptr(runs.subs), runs.n_subs,
                                   ptr(z), cap, clip, ptr(raw), stream)
             _lib.check(code, "bp_readout")
+    return z if step >= w_end - w_begin else None
 
 
 def finish_signal(pk: Packed, raw: torch.Tensor) -> torch.Tensor:

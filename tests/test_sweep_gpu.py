@@ -69,14 +69,13 @@ def _loss(sig, m):
     return (sig.real.double() * w).sum() + 0.5 * (sig.imag.double() * w.flip(1)).sum() + 3.0 * (m.double() ** 2).sum()
 
 
-def _spy(monkeypatch, force=None):
+def _spy(monkeypatch):
     seen = []
     sweeps = adjoint.Checkpointed.sweeps
 
     def spy(self, *a):
-        v = sweeps(self, *a) if force is None else force
-        seen.append(v)
-        return v
+        seen.append(sweeps(self, *a))
+        return seen[-1]
 
     monkeypatch.setattr(adjoint.Checkpointed, "sweeps", spy)
     return seen
@@ -103,8 +102,9 @@ def test_against_the_oracle(n, coils, lengths, names, monkeypatch):
     got = _gradients(ph, seq, c, names, every=64)
     assert seen and all(seen)
     again = _gradients(ph, seq, c, names, every=32 * 100)
+    kept = _gradients(ph, seq, c, names)  # every state from the forward, no replay
     for k in names:  # the same bits wherever the checkpoints lie
-        assert torch.equal(got[k], again[k]), k
+        assert torch.equal(got[k], again[k]) and torch.equal(got[k], kept[k]), k
     _, want = bloch.gradients(bloch.case_from(ph, seq, c), _loss, names)
     _close(got, want, names)
 
@@ -119,6 +119,8 @@ def test_against_the_segment_sweep(n, names, monkeypatch):
         got = _gradients(ph, seq, c, names)
         assert seen and all(seen)
     with monkeypatch.context() as m:
-        _spy(m, force=False)
+        m.setattr(adjoint, "rf_relaxation_invertible", lambda pk: False)  # (bp_adjoint with a replay)
+        seen = _spy(m)
         want = _gradients(ph, seq, c, names)
+        assert seen and not any(seen)
     _close(got, want, names)
