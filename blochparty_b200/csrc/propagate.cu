@@ -79,16 +79,20 @@ __device__ __forceinline__ int first_run(const int4* __restrict__ runs, int n_ru
 #define ST_SMALL (1 << 21)  // RF: every step a small rotation (BP_SMALL)
 #define ST_SAVE (1 << 22)   // the state at its start is saved
 
-template <int CH>
+#define ST_BATCH 8  // HELP: steps whose factors are formed ahead
+
+template <int CH, bool HELP>
 __host__ __device__ constexpr size_t prop_smem() {
-    return (size_t)CH * (2 * (sizeof(SegRec) + sizeof(double4)) + sizeof(float4) + 2 * sizeof(int)) + 2 * sizeof(uint64_t);
+    return (size_t)CH * (2 * (sizeof(SegRec) + sizeof(double4)) + sizeof(float4) + 2 * sizeof(int)) +
+           2 * sizeof(uint64_t) + (HELP ? 2 * ST_BATCH * 6 * 32 * sizeof(float) : 0);
 }
 
-// K: spins per thread; NT: threads per CTA; CH: segments per chunk (a multiple of 32); NB: free steps whose factors are
-// formed together. NB = 1 where other warps fill the factors' latency; with one warp per SM quarter the factors of four
-// steps overlap: a step's chain is about 350 cycles of factors and 95 of the step itself.
-template <int K, int NT, int CH, int NB>
-__global__ void __launch_bounds__(NT, NT == 32 ? 8 : 4) bp_propagate_kernel(PropArgs a) {
+// K: spins per thread; NT: threads per CTA; CH: segments per chunk (a multiple of 32). HELP: the CTA's first warp alone
+// has spins (32), and the others form the factors of its next free steps: with few spins the chain of steps is the time,
+// and the factors (about 350 of a step's 700 cycles, in float64) do not depend on the state.
+template <int K, int NT, int CH, bool HELP>
+__global__ void __launch_bounds__(NT, NT == 32 ? 8 : HELP ? 5 : 4) bp_propagate_kernel(PropArgs a) {
+    static_assert(!HELP || (K == 1 && NT > 32), "helping warps");
     extern __shared__ __align__(128) unsigned char smem_raw[];
     static_assert(CH % 32 == 0 && CH <= 512, "chunks are whole blocks of 32 segments");
     SegRec* segbuf = reinterpret_cast<SegRec*>(smem_raw);         // [2][CH]
@@ -97,10 +101,11 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : 4) bp_propagate_kernel(Prop
     int* list = reinterpret_cast<int*>(rfx + CH);                 // [CH]: the chunk's steps
     int* slots = list + CH;                                       // [CH]: the slot that takes the state at a segment
     uint64_t* bars = reinterpret_cast<uint64_t*>(slots + CH);
+    float* ring = reinterpret_cast<float*>(bars + 2);             // HELP: [2][ST_BATCH][6][32] factors
     __shared__ int count[NT / 32 + 1], windows_in;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = a.n;
-    constexpr int TILE = NT * K;
+    constexpr int TILE = (HELP ? 32 : NT) * K;
     const int n_tiles = (n + TILE - 1) / TILE;
     const int s_begin = a.windows[a.w_begin].x, s_end = a.windows[a.w_end - 1].y;
     if (s_begin < 0 || s_end < s_begin) {  // (uniform)
@@ -137,7 +142,7 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : 4) bp_propagate_kernel(Prop
         float v[6][K], bp[K], bn[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            const int j0 = tile * TILE + (warp * K + k) * 32 + lane;
+            const int j0 = tile * TILE + ((HELP ? 0 : warp) * K + k) * 32 + lane;
             active[k] = j0 < n;
             jk[k] = active[k] ? j0 : 0;
             const Spin s = load_spin(a.spins, n, jk[k], active[k]);
@@ -253,11 +258,21 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : 4) bp_propagate_kernel(Prop
                 return e | (to - ST_SEG(e)) << 10;
             };
 
-            for (int i = 0; i < steps;) {
-                const int e = entry(i), s = ST_SEG(e), len = ST_LEN(e);
+            // HELP: the factors of steps [b0, b0 + ST_BATCH) into one half of the ring, by every warp but the first
+            auto form = [&](int b0) {
+                if (warp == 0) return;
+                for (int i = b0 + warp - 1; i < min(b0 + ST_BATCH, steps); i += NT / 32 - 1) {
+                    const int e = entry(i);
+                    if (!(e & ST_FREE)) continue;
+                    const FreeFactors f = prop_factors(q0[ST_SEG(e)].dt, k0[ST_SEG(e)], p[0], ST_LEN(e));
+                    float* r = ring + (i % (2 * ST_BATCH)) * 6 * 32 + lane;
+                    r[0] = f.ch, r[32] = f.cl, r[64] = f.sh, r[96] = f.sl, r[128] = f.e1, r[160] = f.e2;
+                }
+            };
+            auto take = [&](int i) {  // step i
+                const int e = entry(i), s = ST_SEG(e), len = ST_LEN(e), f = q0[s].flags;
                 if (e & ST_SAVE) store_state(a.wstates + (size_t)slots[s] * 6 * n);
                 if (!(e & ST_FREE)) {
-                    const int f = q0[s].flags;
                     if (s == 0 || !(f & BP_SAME_RFDT)) rf_run_relax(rr, q0[s].dt, p);
                     if (s == 0 || !(f & BP_SAME_OFF)) rf_run_offset(rr, q0[s], p);
                     auto step = [&](int t, auto tag) {
@@ -285,48 +300,46 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : 4) bp_propagate_kernel(Prop
                         }
                         if (f & BP_SPOIL) m.x = m.y = m.lx = m.ly = pset<K>(0.0f);
                     }
-                    ++i;
-                    continue;
+                    return;
                 }
-                // free pieces, the factors of NB of them formed together
-                int ent[NB];
-                FreeFactors ff[NB][K];
-                float t[NB];
+                FreeFactors ff[K];
+                if constexpr (HELP) {
+                    const float* r = ring + (i % (2 * ST_BATCH)) * 6 * 32 + lane;
+                    ff[0] = FreeFactors{r[0], r[32], r[64], r[96], r[128], r[160]};
+                } else {
 #pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    ent[b] = b == 0 ? e : entry(min(i + b, steps - 1));
-                    const int sb = ST_SEG(ent[b]);
+                    for (int k = 0; k < K; ++k) ff[k] = prop_factors(q0[s].dt, k0[s], p[k], len);
+                }
+                const bool starts = (f & BP_ADC) && c + s == next;  // a run's first sample
+                float2 z[K];
+                if (starts && len > 1) {
+                    sample(z);
 #pragma unroll
                     for (int k = 0; k < K; ++k)
-                        ff[b][k] = start_factors(q0[sb].dt, k0[sb], p[k], ST_LEN(ent[b]), t[b]);
+                        readout_advance(prop_factors(q0[s].dt, k0[s], p[k], 1), z[k].x, z[k].y);
                 }
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    if (b > 0 && (i >= steps || !(ent[b] & ST_FREE))) break;  // (uniform)
-                    const int sb = ST_SEG(ent[b]), lb = ST_LEN(ent[b]);
-                    if (b > 0 && (ent[b] & ST_SAVE)) store_state(a.wstates + (size_t)slots[sb] * 6 * n);
-                    const bool starts = (q0[sb].flags & BP_ADC) && c + sb == next;  // a run's first sample
-                    float2 z[K];
-                    if (starts && lb > 1) {
-                        sample(z);
-#pragma unroll
-                        for (int k = 0; k < K; ++k)
-                            readout_advance(prop_factors(q0[sb].dt, k0[sb], p[k], 1), z[k].x, z[k].y);
-                    }
-#pragma unroll
-                    for (int k = 0; k < K; ++k) finish_factors(ff[b][k], p[k], t[b]);
-                    free_step_packed(ff[b], p, m);
-                    if (starts) {
-                        if (lb == 1) sample(z);
-                        write_z(z);
-                    }
-                    if (q0[sb + lb - 1].flags & BP_SPOIL) m.x = m.y = m.lx = m.ly = pset<K>(0.0f);
-                    ++i;
+                free_step_packed(ff, p, m);
+                if (starts) {
+                    if (len == 1) sample(z);
+                    write_z(z);
                 }
+                if (q0[s + len - 1].flags & BP_SPOIL) m.x = m.y = m.lx = m.ly = pset<K>(0.0f);
+            };
+            if constexpr (HELP) {  // the first warp a batch behind the others
+                form(0);
+                __syncthreads();
+                for (int b0 = 0; b0 < steps; b0 += ST_BATCH) {
+                    form(b0 + ST_BATCH);
+                    if (warp == 0)
+                        for (int i = b0; i < min(b0 + ST_BATCH, steps); ++i) take(i);
+                    __syncthreads();
+                }
+            } else {
+                for (int i = 0; i < steps; ++i) take(i);
             }
             c = c_end;
         }
-        store_state(a.state);
+        if (!HELP || warp == 0) store_state(a.state);
     }
 }
 
@@ -568,19 +581,20 @@ static int num_sms() {
     return sms;
 }
 
-template <int K, int NT, int CH, int NB>
+template <int K, int NT, int CH, bool HELP>
 static int launch_propagate(const PropArgs& a, int max_ctas, cudaStream_t stream) {
-    constexpr size_t smem = prop_smem<CH>();
+    constexpr size_t smem = prop_smem<CH, HELP>();
     static_assert(smem <= 48 * 1024, "no opt-in needed");
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bp_propagate_kernel<K, NT, CH, NB>, NT, smem) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bp_propagate_kernel<K, NT, CH, HELP>, NT, smem) !=
         cudaSuccess)
         return BP_E_LAUNCH;
-    const int n_tiles = (a.n + NT * K - 1) / (NT * K);
+    constexpr int TILE = (HELP ? 32 : NT) * K;
+    const int n_tiles = (a.n + TILE - 1) / TILE;
     int grid = num_sms() * (per_sm > 0 ? per_sm : 1);
     if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
     if (grid > n_tiles) grid = n_tiles;
-    bp_propagate_kernel<K, NT, CH, NB><<<grid, NT, smem, stream>>>(a);
+    bp_propagate_kernel<K, NT, CH, HELP><<<grid, NT, smem, stream>>>(a);
     return cudaGetLastError() == cudaSuccess ? BP_OK : BP_E_LAUNCH;
 }
 
@@ -614,11 +628,12 @@ extern "C" int bp_propagate(const float* spins, int n, const void* segs, const d
     a.clip = clip;
     a.status = status;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // few spins: one warp per CTA, so that they spread over the SMs; then one spin per thread while that still leaves
-    // SM quarters with a single warp; else two
+    // while one warp of 32 spins per CTA and its three helpers fit the GPU at once (five CTAs per SM): those; then one
+    // warp per CTA, so that few spins spread over the SMs; past twice four warps per SM two spins per thread
     const int sms = num_sms();
-    if (n <= sms * 4 * 32 * 2) return launch_propagate<1, 32, 160, 4>(a, max_ctas, st);
-    return launch_propagate<2, 128, 256, 1>(a, max_ctas, st);
+    if (n <= sms * 5 * 32) return launch_propagate<1, 128, 96, true>(a, max_ctas, st);
+    if (n <= sms * 4 * 32 * 2) return launch_propagate<1, 32, 160, false>(a, max_ctas, st);
+    return launch_propagate<2, 128, 256, false>(a, max_ctas, st);
 }
 
 extern "C" int bp_readout(const float* spins, const float* sens, int n, int n_coils, const void* segs,
