@@ -69,7 +69,7 @@ BP_MAX_COILS = 32
 BP_SEG_MAX = 160
 BP_ADJ_WIN = 32
 BP_SWEEP_MAX = 2048  # segments of an interval whose RF gradient bp_sweep forms
-BP_PACK_BLOCK = 32768  # spins per block of bp_pack_spins
+BP_PACK_BLOCK = 4096  # spins per block of bp_pack_spins
 BP_MMA_MAX_COILS = 8
 BP_MLP_PARAMS = 10320
 BP_MLP_INPUTS = 2

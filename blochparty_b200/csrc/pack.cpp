@@ -56,8 +56,42 @@ inline double wrapped(double x, double period) {
     return r;
 }
 
-inline double value(const void* p, int wide, int64_t i) {
-    return wide ? static_cast<const double*>(p)[i] : (double)static_cast<const float*>(p)[i];
+// f(the array as its own type).
+template <class F>
+void typed(const void* p, int wide, F f) {
+    if (wide)
+        f(static_cast<const double*>(p));
+    else
+        f(static_cast<const float*>(p));
+}
+
+inline void convert(const void* p, int wide, int64_t at, int64_t m, float* to) {
+    typed(p, wide, [&](auto* x) {
+        for (int64_t j = 0; j < m; ++j) to[j] = (float)(double)x[at + j];
+    });
+}
+
+inline void convert_rate(const void* p, int wide, int64_t at, int64_t m, float* to) {
+    typed(p, wide, [&](auto* x) {
+        for (int64_t j = 0; j < m; ++j) to[j] = (float)(1.0 / (double)x[at + j]);
+    });
+}
+
+// rows [at, at + m) of an array of `width` columns into one run of m per column
+inline void transpose(const void* p, int wide, int64_t at, int64_t m, int width, float* to) {
+    typed(p, wide, [&](auto* x) {
+        x += at * width;
+        for (int c0 = 0; c0 < width; c0 += 8) {
+            const int w = std::min(8, width - c0);
+            if (w == 8) {
+                for (int64_t j = 0; j < m; ++j)
+                    for (int c = 0; c < 8; ++c) to[(c0 + c) * m + j] = (float)(double)x[j * width + c0 + c];
+            } else {
+                for (int64_t j = 0; j < m; ++j)
+                    for (int c = 0; c < w; ++c) to[(c0 + c) * m + j] = (float)(double)x[j * width + c0 + c];
+            }
+        }
+    });
 }
 
 }  // namespace
@@ -122,111 +156,144 @@ extern "C" int bp_pack_segments(const double* dt, const double* rf, const double
     }
 }
 
+// Blocks of spins converted by threads of their own (0: by the caller, which then needs no other thread) and the blocks
+// the staging holds. Up to four blocks (half a millisecond) new threads cost more than they save.
+static int64_t pack_threads(int64_t blocks) {
+    if (blocks <= 4) return 0;
+    const unsigned cores = std::max(2u, std::thread::hardware_concurrency());
+    return std::min<int64_t>({blocks / 2, (int64_t)cores - 1, 15});
+}
+
+static int64_t pack_slots(int64_t blocks) {
+    const int64_t t = pack_threads(blocks);
+    return t ? std::min(blocks, 2 * t) : std::max<int64_t>(blocks, 1);
+}
+
 extern "C" int64_t bp_pack_spins_staging(int64_t n, int n_coils) {
-    // one block per thread: 8 rows of the spins, 2C of the coils, 6 of the state
+    // a block: 8 rows of the spins, 2C of the coils, 6 of the state
     const int64_t block = std::min<int64_t>(n, BP_PACK_BLOCK), blocks = (n + BP_PACK_BLOCK - 1) / BP_PACK_BLOCK;
-    const unsigned cores = std::max(1u, std::thread::hardware_concurrency());
-    const int64_t threads = std::max<int64_t>(1, std::min<int64_t>({blocks, (int64_t)cores, 16}));
-    return threads * (14 + 2 * (int64_t)n_coils) * block * (int64_t)sizeof(float);
+    return pack_slots(blocks) * (14 + 2 * (int64_t)n_coils) * block * (int64_t)sizeof(float);
 }
 
 extern "C" int bp_pack_spins(const BpHostSpins* in, int64_t n, int n_coils, float* spins, float* sens, float* state,
                              float* extent, void* staging, int64_t staging_bytes, void* stream) {
     if (!in || n < 1 || n_coils < 1 || n_coils > BP_MAX_COILS || !spins || !sens || !staging) return BP_E_ARG;
     if (!in->pos || !in->pd || !in->t1 || !in->t2 || !in->db0 || !in->coils) return BP_E_ARG;
+    if (staging_bytes < bp_pack_spins_staging(n, n_coils)) return BP_E_SIZE;
     const int64_t block = std::min<int64_t>(n, BP_PACK_BLOCK), blocks = (n + BP_PACK_BLOCK - 1) / BP_PACK_BLOCK;
-    const int64_t slot = (14 + 2 * (int64_t)n_coils) * block;
-    const int64_t threads =
-        std::max<int64_t>(1, std::min<int64_t>({blocks, staging_bytes / (slot * (int64_t)sizeof(float)), 16}));
-    if (slot * (int64_t)sizeof(float) > staging_bytes) return BP_E_SIZE;
+    const int64_t slot = (14 + 2 * (int64_t)n_coils) * block, slots = pack_slots(blocks), threads = pack_threads(blocks);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return BP_E_LAUNCH;
     const int rows_padded = 16 * ((n_coils + 7) / 8);
     if (rows_padded > 2 * n_coils &&
         cudaMemsetAsync(sens + (size_t)2 * n_coils * n, 0, (size_t)(rows_padded - 2 * n_coils) * n * sizeof(float), st) !=
             cudaSuccess)
         return BP_E_LAUNCH;
-    try {
-    std::atomic<int64_t> next{0};
-    std::atomic<int> code{BP_OK};
-    std::vector<float> most(threads * 8, 0.0f);
-    auto work = [&](int64_t t, int64_t) {
-        float* base = static_cast<float*>(staging) + t * slot;
-        float* ext = most.data() + 8 * t;
-        cudaEvent_t done;
-        if (cudaSetDevice(dev) != cudaSuccess || cudaEventCreateWithFlags(&done, cudaEventDisableTiming) != cudaSuccess) {
-            code = BP_E_LAUNCH;
-            return;
-        }
-        for (int64_t b; (b = next.fetch_add(1)) < blocks && code == BP_OK;) {
-            const int64_t j0 = b * BP_PACK_BLOCK, m = std::min<int64_t>(BP_PACK_BLOCK, n - j0);
-            float *sp = base, *co = base + 8 * m, *sv = co + 2 * (int64_t)n_coils * m;
+    // block b of the spins into its slot; ext: the largest magnitudes so far, as bits (a NaN's are above every number's)
+    auto fill = [&](int64_t b, uint32_t* ext) {
+        const int64_t j0 = b * BP_PACK_BLOCK, m = std::min<int64_t>(BP_PACK_BLOCK, n - j0);
+        float* sp = static_cast<float*>(staging) + (b % slots) * slot;
+        float *co = sp + 8 * m, *sv = co + 2 * (int64_t)n_coils * m;
+        transpose(in->pos, in->wide[0], j0, m, 3, sp);
+        convert(in->pd, in->wide[1], j0, m, sp + 3 * m);
+        convert_rate(in->t1, in->wide[2], j0, m, sp + 4 * m);
+        convert_rate(in->t2, in->wide[3], j0, m, sp + 5 * m);
+        convert(in->db0, in->wide[4], j0, m, sp + 6 * m);
+        if (in->b1)
+            convert(in->b1, in->wide[5], j0, m, sp + 7 * m);
+        else
+            std::fill(sp + 7 * m, sp + 8 * m, 1.0f);
+        transpose(in->coils, in->wide[6], j0, m, 2 * n_coils, co);
+        for (int r = 0; r < 8; ++r)
             for (int64_t j = 0; j < m; ++j) {
-                const int64_t i = j0 + j;
-                sp[j] = (float)value(in->pos, in->wide[0], 3 * i);
-                sp[m + j] = (float)value(in->pos, in->wide[0], 3 * i + 1);
-                sp[2 * m + j] = (float)value(in->pos, in->wide[0], 3 * i + 2);
+                uint32_t bits;
+                std::memcpy(&bits, sp + r * m + j, 4);
+                ext[r] = std::max(ext[r], bits & 0x7fffffffu);
             }
-            for (int64_t j = 0; j < m; ++j) sp[3 * m + j] = (float)value(in->pd, in->wide[1], j0 + j);
-            for (int64_t j = 0; j < m; ++j) sp[4 * m + j] = (float)(1.0 / value(in->t1, in->wide[2], j0 + j));
-            for (int64_t j = 0; j < m; ++j) sp[5 * m + j] = (float)(1.0 / value(in->t2, in->wide[3], j0 + j));
-            for (int64_t j = 0; j < m; ++j) sp[6 * m + j] = (float)value(in->db0, in->wide[4], j0 + j);
-            for (int64_t j = 0; j < m; ++j) sp[7 * m + j] = in->b1 ? (float)value(in->b1, in->wide[5], j0 + j) : 1.0f;
-            for (int64_t j = 0; j < m; ++j)  // [spin][2C] -> [2C][spin], a block that stays in the cache
-                for (int c = 0; c < 2 * n_coils; ++c)
-                    co[c * m + j] = (float)value(in->coils, in->wide[6], (j0 + j) * 2 * n_coils + c);
-            for (int r = 0; r < 8; ++r)  // (a NaN stays: no bound holds)
-                for (int64_t j = 0; j < m && ext[r] == ext[r]; ++j) {
-                    const float v = std::fabs(sp[r * m + j]);
-                    if (!(v <= ext[r])) ext[r] = v;
+        if (!state) return;
+        std::fill(sv, sv + 6 * m, 0.0f);  // m0 in a float32 high part and its float32 remainder
+        typed(in->m0 ? in->m0 : in->pd, in->m0 ? in->wide[7] : in->wide[1], [&](auto* x) {
+            for (int c = in->m0 ? 0 : 2; c < 3; ++c)
+                for (int64_t j = 0; j < m; ++j) {
+                    const double v = (double)(in->m0 ? x[3 * (j0 + j) + c] : x[j0 + j]);
+                    const float hi = (float)v;
+                    sv[c * m + j] = hi;
+                    sv[(3 + c) * m + j] = (float)(v - (double)hi);
                 }
-            auto copy = [&](float* dst, const float* src, int rows) {
-                if (cudaMemcpy2DAsync(dst + j0, (size_t)n * sizeof(float), src, (size_t)m * sizeof(float),
-                                      (size_t)m * sizeof(float), (size_t)rows, cudaMemcpyHostToDevice, st) != cudaSuccess)
-                    code = BP_E_LAUNCH;
-            };
-            copy(spins, sp, 8);
-            copy(sens, co, 2 * n_coils);
-            if (state) {  // m0 in a float32 high part and its float32 remainder
-                for (int c = 0; c < 3; ++c)
-                    for (int64_t j = 0; j < m; ++j) {
-                        const double v = in->m0   ? value(in->m0, in->wide[7], 3 * (j0 + j) + c)
-                                         : c == 2 ? value(in->pd, in->wide[1], j0 + j)
-                                                  : 0.0;
-                        const float hi = (float)v;
-                        sv[c * m + j] = hi;
-                        sv[(3 + c) * m + j] = (float)(v - (double)hi);
-                    }
-                copy(state, sv, 6);
-            }
-            // the block's copies end before its staging is written again, or given back
-            if (cudaEventRecord(done, st) != cudaSuccess || cudaEventSynchronize(done) != cudaSuccess) code = BP_E_LAUNCH;
-        }
-        cudaEventDestroy(done);
+        });
     };
-    std::vector<std::thread> extra;
-    extra.reserve(threads);
-    for (int64_t t = 1; t < threads; ++t) {
+    auto send = [&](int64_t b) {
+        const int64_t j0 = b * BP_PACK_BLOCK, m = std::min<int64_t>(BP_PACK_BLOCK, n - j0);
+        const float* sp = static_cast<const float*>(staging) + (b % slots) * slot;
+        auto copy = [&](float* dst, const float* src, int rows) {
+            return cudaMemcpy2DAsync(dst + j0, (size_t)n * sizeof(float), src, (size_t)m * sizeof(float),
+                                     (size_t)m * sizeof(float), (size_t)rows, cudaMemcpyHostToDevice, st) == cudaSuccess;
+        };
+        return copy(spins, sp, 8) && copy(sens, sp + 8 * m, 2 * n_coils) &&
+               (!state || copy(state, sp + (8 + 2 * (int64_t)n_coils) * m, 6));
+    };
+    uint32_t most[8] = {0};
+    bool ok = true;
+    if (threads == 0) {
+        for (int64_t b = 0; b < blocks; ++b) {
+            fill(b, most);
+            ok = send(b) && ok;
+        }
+        ok = cudaStreamSynchronize(st) == cudaSuccess && ok;  // the staging is the caller's again
+    } else {
+        // workers convert blocks as they come, waiting for a slot whose copies have ended; this thread copies them in
+        // order and gives the slots back
         try {
-            extra.emplace_back(work, t, 0);
-        } catch (...) {
-            break;  // fewer threads: the others take the blocks
-        }
-    }
-    work(0, 0);
-    for (auto& x : extra) x.join();
-    if (extent) {
-        for (int r = 0; r < 8; ++r) {
-            extent[r] = 0.0f;
-            for (int64_t t = 0; t < threads && extent[r] == extent[r]; ++t) {
-                const float v = most[8 * t + r];
-                if (!(v <= extent[r])) extent[r] = v;
+            std::vector<std::atomic<int>> full(blocks);
+            for (auto& f : full) f.store(0);
+            std::atomic<int64_t> next{0}, given{slots};  // blocks below `given` may be converted
+            std::vector<uint32_t> tops(threads * 8, 0u);
+            std::vector<cudaEvent_t> events;
+            events.reserve(slots);
+            for (int64_t i = 0; i < slots && ok; ++i) {
+                cudaEvent_t e;
+                ok = cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+                if (ok) events.push_back(e);
             }
+            auto work = [&](int64_t t) {
+                for (int64_t b; (b = next.fetch_add(1)) < blocks;) {
+                    while (given.load(std::memory_order_acquire) <= b) std::this_thread::yield();
+                    fill(b, tops.data() + 8 * t);
+                    full[b].store(1, std::memory_order_release);
+                }
+            };
+            std::vector<std::thread> workers;
+            workers.reserve(threads);
+            for (int64_t t = 0; t < threads && ok; ++t) {
+                try {
+                    workers.emplace_back(work, t);
+                } catch (...) {
+                    break;  // fewer of them
+                }
+            }
+            if (workers.empty()) {  // none: this thread does their work, a slot's worth at a time
+                for (int64_t b = 0; b < blocks && ok; ++b) {
+                    fill(b, most);
+                    ok = send(b) && cudaStreamSynchronize(st) == cudaSuccess;
+                }
+            } else {
+                int64_t back = 0;  // blocks whose slots have been given back
+                for (int64_t b = 0; b < blocks; ++b) {
+                    while (!full[b].load(std::memory_order_acquire)) std::this_thread::yield();
+                    if (ok) ok = send(b) && cudaEventRecord(events[b % slots], st) == cudaSuccess;
+                    for (; back <= b - slots / 2; ++back) {  // (after a failure the workers still get through)
+                        if (ok) ok = cudaEventSynchronize(events[back % slots]) == cudaSuccess;
+                        given.store(slots + back + 1, std::memory_order_release);
+                    }
+                }
+                for (auto& w : workers) w.join();
+            }
+            ok = cudaStreamSynchronize(st) == cudaSuccess && ok;
+            for (auto& e : events) cudaEventDestroy(e);
+            for (int64_t i = 0; i < 8 * threads; ++i) most[i % 8] = std::max(most[i % 8], tops[i]);
+        } catch (...) {  // (out of host memory before any worker ran: no exception leaves the library)
+            return BP_E_SIZE;
         }
     }
-    return code;
-    } catch (...) {
-        return BP_E_SIZE;
-    }
+    if (extent) std::memcpy(extent, most, sizeof(most));
+    return ok ? BP_OK : BP_E_LAUNCH;
 }

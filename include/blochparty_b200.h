@@ -114,7 +114,7 @@ int bp_sample_runs(const int32_t* flags, int64_t n, int run_max, int32_t* runs, 
  * block of it), by several threads; every value rounded once to float32 from its float64 value. The copies are issued
  * on `stream` and have ended when the call returns. state may be NULL; extent: NULL, or float32 x 8 (host), as
  * bp_pack_segments takes it. */
-#define BP_PACK_BLOCK 32768
+#define BP_PACK_BLOCK 4096
 typedef struct {
     const void *pos, *pd, *t1, *t2, *db0, *b1, *coils, *m0; /* [n][3], [n] each, b1 NULL: 1, [n][C] complex, [n][3] or
                                                                NULL: (0, 0, pd) */

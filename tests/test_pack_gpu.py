@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 F32, F64 = torch.float32, torch.float64
 
 
-@pytest.mark.parametrize("n", [1, 127, _lib.BP_PACK_BLOCK, _lib.BP_PACK_BLOCK + 1, 5 * _lib.BP_PACK_BLOCK + 77])
+@pytest.mark.parametrize("n", [1, 127, _lib.BP_PACK_BLOCK, 4 * _lib.BP_PACK_BLOCK, 4 * _lib.BP_PACK_BLOCK + 1,
+                               70 * _lib.BP_PACK_BLOCK + 77])
 @pytest.mark.parametrize("dtype,coils,m0", [(F64, 8, False), (F32, 3, True), (F64, 13, True), (torch.float16, 1, False)])
 def test_spins(n, dtype, coils, m0):
     """Blocks of spins, one thread and several, float32, float64 and other inputs, strided and conjugated ones."""
@@ -31,7 +32,7 @@ def test_spins(n, dtype, coils, m0):
 
 
 def test_extent_keeps_a_nan():
-    n = engine._lib.BP_PACK_BLOCK * 3
+    n = engine._lib.BP_PACK_BLOCK * 12
     v = torch.ones(n, dtype=F64)
     b1 = v.clone()
     b1[7] = float("nan")
