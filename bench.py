@@ -83,11 +83,12 @@ FLOP_RF_REV, FLOP_FREE_REV, FLOP_ADC_REV_PER_COIL, FLOP_ADC_REV = 130, 30, 8, 2
 # recompute; a free segment's reverse is lambda's alone, 9 flops, and a window of free segments with one factor set
 # recomputes nothing
 FLOP_RF_REV_NO_SPIN, FLOP_RF_BACK, FLOP_FREE_LAMBDA = 103, 138, 9
-# DRAM bytes per spin-segment of the forward kernel, measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum of
-# one launch over its spins x segments): the float32 readout on the 4-echo head sequence at 96^3 x 4 TRs (14.16 GB for
-# 3,538,944 x 2,376) and the NUFFT readout at 64^3 x 4 TRs (3.015 GB for 1,048,576 x 1,864). The traffic is the
-# per-window state, spin parameters and coil sensitivities, so it scales with spins x windows.
-TRAFFIC_FP32_PER_SPIN_SEGMENT = 14.162e9 / (3538944 * 2376)
+# DRAM bytes per spin-segment of the forward kernels, measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum of
+# one forward over its spins x segments): the float32 readout (propagation and coil sums) on the 4-echo head sequence at
+# 96^3 x 4 TRs (4.929 GB for 3,538,944 x 2,376) and the NUFFT readout at 64^3 x 4 TRs (3.015 GB for 1,048,576 x 1,864).
+# The traffic is the runs' first samples and, once per 128 samples, the spin parameters and coil sensitivities (NUFFT:
+# per window, and the state), so it scales with spins x segments.
+TRAFFIC_FP32_PER_SPIN_SEGMENT = 4.929e9 / (3538944 * 2376)
 TRAFFIC_NUFFT_PER_SPIN_SEGMENT = 3.0147e9 / (1048576 * 1864)
 
 
@@ -462,8 +463,10 @@ def measure_fwd_adjoint(args, dev, pk, state0, flush, n, S):
         "states": saved_states_text(run),
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                      "traffic": None, "peak_source": "live FFMA probe (bp_ffma_peak) on this GPU",
-                     "kernel": ("bp_forward_kernel (forward" + (")" if run.saved is not None else ", replay)")
-                                + " + bp_adjoint_kernel + bp_seg_reduce_kernel"),
+                     "kernel": ("bp_propagate_kernel + bp_readout_kernel (forward" + (")" if run.saved is not None
+                                                                                     else ", replay)")
+                                + (" + bp_cotangent_kernel + bp_sweep_kernel + bp_sweep_reduce_kernel" if run.uniform
+                                   else " + bp_adjoint_kernel + bp_seg_reduce_kernel")),
                      "flops_per_spin": {"forward": fwd, "backward": bwd}},
         "gpu_launches": args.steps * (lf + lb), "clocks": clocks.summary(),
     }
@@ -698,7 +701,8 @@ def main():
         per = TRAFFIC_NUFFT_PER_SPIN_SEGMENT if nr is not None else TRAFFIC_FP32_PER_SPIN_SEGMENT
         traffic = {"bytes": per * n * S, "bytes_per_spin_segment": per,
                    "scaled_from": ("ncu capture of bp_forward_kernel with NUFFT runs, head 64^3 x 4 TRs"
-                                   if nr is not None else "ncu capture of bp_forward_kernel, head 96^3 x 4 TRs")}
+                                   if nr is not None else
+                                   "ncu capture of bp_propagate_kernel and bp_readout_kernel, head 96^3 x 4 TRs")}
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
@@ -718,14 +722,16 @@ def main():
                      "peak_source": "live FFMA probe (bp_ffma_peak) on this GPU; MEASURED_PEAKS.json has no FP32",
                      "kernel": ("bp_forward_mma_kernel" if mma is not None else
                                 "bp_forward_kernel (NUFFT runs) + bp_nufft_finish_kernel" if nr is not None
+                                else "bp_propagate_kernel + bp_readout_kernel" if replaced is None
                                 else "bp_forward_kernel"),
                      "kernel_ms": kernel_ms,
                      "flops_per_launch": flops},
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "ms_per_step": statistics.median(e2e_ms) if e2e_ms else None},
-        "gpu_launches": ((3 if nr is not None else 2) * args.steps if replaced is None else
+        "gpu_launches": ((3 if nr is not None else 2 if mma is not None
+                          else engine.forward_launches(pk, windows.shape[0]) + 1) * args.steps if replaced is None else
                          args.steps * ((len(reuse.pulses) if reuse is not None else 0) + len(replaced.spans)
-                                       + len(fwd_events) + 1)),
+                                       + 2 * len(fwd_events) + 1)),
         "clocks": clocks.summary(),
     }
     if grad_line is not None:

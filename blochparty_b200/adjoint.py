@@ -531,16 +531,18 @@ class Checkpointed:
 
     def launches(self, need_seg: bool) -> tuple[int, int]:
         """(forward, backward) kernel launches of one call each."""
-        k = len(self.plan.starts)
+        k, plan = len(self.plan.starts), self.plan
         readout = int(self.pk.n_adc > 0)
+        run = lambda windows: engine.forward_launches(self.pk, windows) if readout else 1
         swept = 2 * readout + k * (1 + readout + int(need_seg))  # the split, then per interval samples, sweep, sums
         if self.saved is not None:
-            nb = len(self.blocks())
-            return nb * (1 + readout), nb - 1 + (swept if self.uniform else k * (2 if need_seg else 1))
+            blocks = self.blocks()
+            forward = sum(run(plan.franges[kb - 1][1] - plan.franges[ka][0]) for ka, kb in blocks)
+            return forward, len(blocks) - 1 + (swept if self.uniform else k * (2 if need_seg else 1))
         if self.kept is not None:
-            return 1 + readout, swept
+            return run(plan.awin.shape[0]), swept
         rebuild = sum(kb - ka - 1 for ka, kb in self.blocks()) if self.outer else 0
-        forward = k if self.phys is not None else 1 + readout
+        forward = k if self.phys is not None else run(plan.fwin.shape[0])
         return forward, rebuild + (k + swept if self.uniform else k * (3 if need_seg else 2))
 
     def check(self, what: str = "bp_forward / bp_adjoint") -> None:

@@ -1,8 +1,8 @@
 // Forward propagation with the coil readout on the tensor cores (tcgen05, split bfloat16, float32 accumulation).
 //
 // The propagation's steps are those of bp_propagate_kernel (windows, persistent CTAs over 128-spin tiles, TMA-staged
-// segment blocks, compensated float32 state). The readout differs: the coil sum of a block of 16 ADC samples over a tile's 128
-// spins is one small matrix product on the tensor cores,
+// segment blocks, compensated float32 state). The readout differs: the coil sum of a block of 16 ADC samples over a
+// tile's 128 spins is one small matrix product on the tensor cores,
 //     D[m][t] += sum_k A[m][k] B[t][k],   k = 2 j + {0, 1} (spin j's Mx, My),
 // with A the tile's coil sensitivities (row m = 2c: (s_r, -s_i), row 2c + 1: (s_i, s_r) per spin, coil c) and B
 // the 16 samples' magnetization. Both are split into bfloat16 high and low parts and D accumulates

@@ -104,53 +104,54 @@ extern "C" int bp_pack_segments(const double* dt, const double* rf, const double
                                       !flags || !psi)))
         return BP_E_ARG;
     try {
-    Record* rec = static_cast<Record*>(records);
-    parallel(n, 1 << 13, 16, [&](int64_t a, int64_t b) {
-        for (int64_t s = a; s < b; ++s) {
-            const double w = -kTwoPi * dt[s], beta = (b0 ? b0[s] : 0.0) * dt[s];
-            const double k[3] = {grad[3 * s] * dt[s], grad[3 * s + 1] * dt[s], grad[3 * s + 2] * dt[s]};
-            Record& r = rec[s];
-            r.dt = (float)dt[s];
-            r.wx = (float)(w * rf[2 * s]), r.wy = (float)(w * rf[2 * s + 1]);
-            r.kx = (float)k[0], r.ky = (float)k[1], r.kz = (float)k[2], r.beta = (float)beta;
-            seg64[4 * s] = k[0], seg64[4 * s + 1] = k[1], seg64[4 * s + 2] = k[2], seg64[4 * s + 3] = beta;
-            r.flags = (is_rf[s] ? RF : 0) | (adc[s] ? ADC : 0) | (spoil[s] ? SPOIL : 0);
-        }
-    });
-    // what a segment shares with the one before it, and whether its rotation is small for every spin: extent holds the
-    // largest |x| |y| |z| pd r1 r2 |dB0| |b1| (NULL: not marked)
-    parallel(n, 1 << 13, 16, [&](int64_t a, int64_t b) {
-        for (int64_t s = a; s < b; ++s) {
-            Record& r = rec[s];
-            int32_t f = r.flags & (RF | ADC | SPOIL);
-            if (s > 0) {
-                const Record& q = rec[s - 1];
-                const double *u = seg64 + 4 * s, *v = u - 4;
-                const bool rf0 = is_rf[s - 1] != 0, rf1 = is_rf[s] != 0, same_dt = r.dt == q.dt;
-                if (!rf0 && !rf1 && same_dt && u[0] == v[0] && u[1] == v[1] && u[2] == v[2] && u[3] == v[3])
-                    f |= SAME_FREE;
-                if (rf0 && rf1 && same_dt) {
-                    f |= SAME_RFDT;
-                    if (r.kx == q.kx && r.ky == q.ky && r.kz == q.kz && r.beta == q.beta) f |= SAME_OFF;
+        Record* rec = static_cast<Record*>(records);
+        parallel(n, 1 << 13, 16, [&](int64_t a, int64_t b) {
+            for (int64_t s = a; s < b; ++s) {
+                const double w = -kTwoPi * dt[s], beta = (b0 ? b0[s] : 0.0) * dt[s];
+                const double k[3] = {grad[3 * s] * dt[s], grad[3 * s + 1] * dt[s], grad[3 * s + 2] * dt[s]};
+                Record& r = rec[s];
+                r.dt = (float)dt[s];
+                r.wx = (float)(w * rf[2 * s]), r.wy = (float)(w * rf[2 * s + 1]);
+                r.kx = (float)k[0], r.ky = (float)k[1], r.kz = (float)k[2], r.beta = (float)beta;
+                seg64[4 * s] = k[0], seg64[4 * s + 1] = k[1], seg64[4 * s + 2] = k[2], seg64[4 * s + 3] = beta;
+                r.flags = (is_rf[s] ? RF : 0) | (adc[s] ? ADC : 0) | (spoil[s] ? SPOIL : 0);
+            }
+        });
+        // what a segment shares with the one before it, and whether its rotation is small for every spin: extent holds
+        // the largest |x| |y| |z| pd r1 r2 |dB0| |b1| (NULL: not marked)
+        parallel(n, 1 << 13, 16, [&](int64_t a, int64_t b) {
+            for (int64_t s = a; s < b; ++s) {
+                Record& r = rec[s];
+                int32_t f = r.flags & (RF | ADC | SPOIL);
+                if (s > 0) {
+                    const Record& q = rec[s - 1];
+                    const double *u = seg64 + 4 * s, *v = u - 4;
+                    const bool rf0 = is_rf[s - 1] != 0, rf1 = is_rf[s] != 0, same_dt = r.dt == q.dt;
+                    if (!rf0 && !rf1 && same_dt && u[0] == v[0] && u[1] == v[1] && u[2] == v[2] && u[3] == v[3])
+                        f |= SAME_FREE;
+                    if (rf0 && rf1 && same_dt) {
+                        f |= SAME_RFDT;
+                        if (r.kx == q.kx && r.ky == q.ky && r.kz == q.kz && r.beta == q.beta) f |= SAME_OFF;
+                    }
                 }
+                if (extent && (f & RF)) {
+                    const double wz =
+                        kTwoPi * (std::fabs((double)r.kx) * extent[0] + std::fabs((double)r.ky) * extent[1] +
+                                  std::fabs((double)r.kz) * extent[2] + std::fabs((double)r.dt) * extent[6] +
+                                  std::fabs((double)r.beta));
+                    const double b1 = extent[7], wx = r.wx, wy = r.wy;
+                    if (b1 * b1 * (wx * wx + wy * wy) + wz * wz < 0.0624) f |= SMALL;
+                }
+                flags[s] = f;
             }
-            if (extent && (f & RF)) {
-                const double wz = kTwoPi * (std::fabs((double)r.kx) * extent[0] + std::fabs((double)r.ky) * extent[1] +
-                                            std::fabs((double)r.kz) * extent[2] + std::fabs((double)r.dt) * extent[6] +
-                                            std::fabs((double)r.beta));
-                const double b1 = extent[7], wx = r.wx, wy = r.wy;
-                if (b1 * b1 * (wx * wx + wy * wy) + wz * wz < 0.0624) f |= SMALL;
-            }
-            flags[s] = f;
+        });
+        int64_t rows = 0;
+        for (int64_t s = 0; s < n; ++s) {
+            rec[s].flags = flags[s];
+            if (adc[s]) psi[rows++] = wrapped(phase[s], kTwoPi);
         }
-    });
-    int64_t rows = 0;
-    for (int64_t s = 0; s < n; ++s) {
-        rec[s].flags = flags[s];
-        if (adc[s]) psi[rows++] = wrapped(phase[s], kTwoPi);
-    }
-    *n_adc = rows;
-    return BP_OK;
+        *n_adc = rows;
+        return BP_OK;
     } catch (...) {  // (out of host memory: no exception leaves the library)
         return BP_E_SIZE;
     }

@@ -284,6 +284,25 @@ def pack(case, device) -> Packed:
     return pack_with_state(case, device)[0]
 
 
+def _window_step(pk: Packed, windows: int) -> tuple[int, int]:
+    """(windows per launch, runs the workspace holds) of a forward with a readout over ``windows`` windows: all of them
+    where the runs' first samples fit ``Z_BYTES``, else as many as keep any launch's runs under it."""
+    runs, step = pk.sample_runs(), max(windows, 1)
+    cap, room = runs.n_runs, max(Z_BYTES // (8 * max(pk.n, 1)), 1)
+    if cap > room:
+        step = max(1, step * room // cap)
+        while step > 1 and runs.most_in(step * _lib.BP_SEG_MAX) + 1 > room:
+            step = (step + 1) // 2
+        cap = min(cap, runs.most_in(step * _lib.BP_SEG_MAX) + 1)
+    return step, cap
+
+
+def forward_launches(pk: Packed, windows: int) -> int:
+    """Kernel launches of ``run_forward`` with a readout over ``windows`` windows."""
+    step, cap = _window_step(pk, windows)
+    return -(-windows // step) * (2 if cap else 1)
+
+
 def run_forward(pk: Packed, state: torch.Tensor, windows_dev: torch.Tensor, w_begin: int, w_end: int,
                 raw: torch.Tensor | None, status: torch.Tensor, wstates: torch.Tensor | None = None,
                 wstate_stride: int = 1, max_ctas: int = 0, wslot: torch.Tensor | None = None,
@@ -296,16 +315,8 @@ def run_forward(pk: Packed, state: torch.Tensor, windows_dev: torch.Tensor, w_be
     (the runs' first samples, [run][N] pairs) when one launch took all windows."""
     lib, stream = _lib.lib(), _lib.stream_ptr()
     runs = pk.sample_runs() if raw is not None else None
-    step, cap, z = max(w_end - w_begin, 1), 0, None
-    if runs is not None and runs.n_runs:
-        room = max(Z_BYTES // (8 * max(pk.n, 1)), 1)
-        cap = runs.n_runs
-        if cap > room:  # fewer windows at a time
-            step = max(1, step * room // cap)
-            while step > 1 and runs.most_in(step * _lib.BP_SEG_MAX) + 1 > room:
-                step = (step + 1) // 2
-            cap = min(cap, runs.most_in(step * _lib.BP_SEG_MAX) + 1)
-        z = torch.empty(cap, pk.n, 2, dtype=F32, device=pk.device)
+    step, cap = _window_step(pk, w_end - w_begin) if runs is not None else (max(w_end - w_begin, 1), 0)
+    z = torch.empty(cap, pk.n, 2, dtype=F32, device=pk.device) if cap else None
     for wa in range(w_begin, w_end, step):
         wb = min(wa + step, w_end)
         clip = 0 if whole_runs else ((_lib.BP_CLIP_BEGIN if wa == w_begin else 0)
