@@ -79,7 +79,9 @@ __device__ __forceinline__ int first_run(const int4* __restrict__ runs, int n_ru
 #define ST_SMALL (1 << 21)  // RF: every step a small rotation (BP_SMALL)
 #define ST_SAVE (1 << 22)   // the state at its start is saved
 
-#define ST_BATCH 8  // HELP: steps whose factors are formed ahead
+// HELP: steps whose factors are formed ahead. Eight left the first warp waiting longer at a chunk's start: 0.767 -> 0.735
+// ms for 4,096 spins x 264 TRs (six 0.740), 0.434 -> 0.419 for 9,025 x 115; the same where help is off.
+#define ST_BATCH 4
 
 template <int CH, bool HELP>
 __host__ __device__ constexpr size_t prop_smem() {
@@ -419,10 +421,13 @@ __global__ void __launch_bounds__(RO_THREADS, 3) bp_readout_kernel(ReadArgs a) {
     __syncthreads();
     if (sub[0].x == 0 && sub[1].x == 0 && sub[2].x == 0 && sub[3].x == 0) return;
 
-    uint2* sens = reinterpret_cast<uint2*>(sm[warp]);              // [32][8], split and swizzled
-    float2* tab = reinterpret_cast<float2*>(sens + 32 * 8);        // [RO_ROWS][RO_TAB_STRIDE]: q^0 .. q^7 per spin
-    float2* step8 = tab + RO_ROWS * RO_TAB_STRIDE;                 // [32]: q^8
-    float2* first = step8 + 32;                                    // [32]: the block's first sample, scaled
+    uint4* sens = reinterpret_cast<uint4*>(sm[warp]);              // [32][8], split and swizzled
+    float* tab = reinterpret_cast<float*>(sens + 32 * 8);          // [RO_ROWS][RO_TAB_ROW]: q^0 .. q^7, in pairs of spins
+    float* step8 = tab + RO_ROWS * RO_TAB_ROW;                     // [16][4]: q^8, in pairs
+    float* first = step8 + 16 * 4;                                 // [16][4]: the block's first sample, scaled, in pairs
+    float2* nstep = reinterpret_cast<float2*>(first + 16 * 4);     // [16]: -im of the pairs of step8
+    float2* nfirst = nstep + 16;                                   // and of first
+    const int pw = pair_word(lane);                                // this lane's spin's place in its pair
     const int r = lane >> 2, t = lane & 3;
     float acc[RO_SUBS][2][2][4];  // block, 16 samples, real and imaginary, fragment
 #pragma unroll
@@ -478,10 +483,8 @@ __global__ void __launch_bounds__(RO_THREADS, 3) bp_readout_kernel(ReadArgs a) {
             float scale;
             warp_scale(mag, scale, sens_inv);
 #pragma unroll
-            for (int c = 0; c < 8; c += 2) {
-                const uint2 x = split_sens(v[2 * c] * scale, v[2 * c + 1] * scale);
-                const uint2 y = split_sens(v[2 * c + 2] * scale, v[2 * c + 3] * scale);
-                *reinterpret_cast<uint4*>(sens + sens_slot(lane, c)) = make_uint4(x.x, x.y, y.x, y.y);
+            for (int c = 0; c < 8; ++c) {
+                sens[sens_slot(lane, c)] = split_sens(v[2 * c] * scale, v[2 * c + 1] * scale);
             }
         }
         float2 q32 = make_float2(1.0f, 0.0f), z = make_float2(0.0f, 0.0f);
@@ -495,13 +498,13 @@ __global__ void __launch_bounds__(RO_THREADS, 3) bp_readout_kernel(ReadArgs a) {
                 float2 q8;
                 factor_powers(f, q8, q32);
                 float zr = 1.0f, zi = 0.0f;
-                tab[lane] = make_float2(zr, zi);
 #pragma unroll
-                for (int i = 1; i < RO_ROWS; ++i) {
-                    readout_advance(f, zr, zi);
-                    tab[i * RO_TAB_STRIDE + lane] = make_float2(zr, zi);
+                for (int i = 0; i < RO_ROWS; ++i) {
+                    tab[i * RO_TAB_ROW + pw] = zr, tab[i * RO_TAB_ROW + pw + 2] = zi;
+                    if (i + 1 < RO_ROWS) readout_advance(f, zr, zi);
                 }
-                step8[lane] = q8;
+                step8[pw] = q8.x, step8[pw + 2] = q8.y;
+                reinterpret_cast<float*>(nstep)[(pw >> 2) * 2 + (pw & 1)] = -q8.y;
             }
             if (slot != sb.y || part > sb.z) {
                 z = zin[b];
@@ -512,30 +515,24 @@ __global__ void __launch_bounds__(RO_THREADS, 3) bp_readout_kernel(ReadArgs a) {
             float scale, inverse;
             const uint32_t u = __float_as_uint(fmaxf(fabsf(z.x), fabsf(z.y)));
             warp_scale(u, scale, inverse);
-            first[lane] = make_float2(z.x * scale, z.y * scale);
+            first[pw] = z.x * scale, first[pw + 2] = z.y * scale;
+            reinterpret_cast<float*>(nfirst)[(pw >> 2) * 2 + (pw & 1)] = -(z.y * scale);
             __syncwarp();
             float dr[2][4], di[2][4];
 #pragma unroll
             for (int i = 0; i < 8; ++i) dr[i >> 2][i & 3] = di[i >> 2][i & 3] = 0.0f;
 #pragma unroll 2
             for (int g = 0; g < 4; ++g) {  // eight spins: 8 g + t and 8 g + 4 + t are this lane's
-                const int s0 = 8 * g + t, s1 = s0 + 4;
-                const uint2 br[2] = {sens[sens_slot(s0, r)], sens[sens_slot(s1, r)]};
-                const uint2 bi[2] = {make_uint2(turn_half(br[0].x), turn_half(br[0].y)),
-                                     make_uint2(turn_half(br[1].x), turn_half(br[1].y))};
-                const float2 fa = first[s0], fb = first[s1];
-                const float2 ta = tab[r * RO_TAB_STRIDE + s0], tb = tab[r * RO_TAB_STRIDE + s1];
-                const CPair z0 = cmul2(CPair{make_float2(fa.x, fb.x), make_float2(fa.y, fb.y)},
-                                       CPair{make_float2(ta.x, tb.x), make_float2(ta.y, tb.y)},
-                                       make_float2(-ta.y, -tb.y));
-                const float2 qa = step8[s0], qb = step8[s1];
-                const CPair step{make_float2(qa.x, qb.x), make_float2(qa.y, qb.y)};
-                const float2 nim = make_float2(-qa.y, -qb.y);
+                const int pr = 4 * g + t;
+                const uint4 sa = sens[sens_slot(8 * g + t, r)], sc = sens[sens_slot(8 * g + 4 + t, r)];
+                const CPair step = load_pair(step8 + 4 * pr);
+                const float2 nim = nstep[pr];
+                const CPair z0 = cmul2(load_pair(tab + r * RO_TAB_ROW + 4 * pr), load_pair(first + 4 * pr), nfirst[pr]);
                 const CPair z1 = cmul2(z0, step, nim);
-                readout_mma(z0, z1, br, bi, dr[0], di[0]);
+                readout_mma(z0, z1, sa, sc, dr[0], di[0]);
                 if (sb.x > 16) {
                     const CPair z2 = cmul2(z1, step, nim);
-                    readout_mma(z2, cmul2(z2, step, nim), br, bi, dr[1], di[1]);
+                    readout_mma(z2, cmul2(z2, step, nim), sa, sc, dr[1], di[1]);
                 }
             }
             __syncwarp();  // the operands' reads have ended

@@ -40,7 +40,8 @@ __global__ void bp_h_most_kernel(const float* __restrict__ h, int64_t n, uint32_
     if ((threadIdx.x & 31) == 0 && m) atomicMax(most, m);
 }
 
-// hs [rows][8 ncg]: the halves of (h0, -h1) of every row and coil, scaled; zero coils to pad.
+// hs [rows][8 ncg]: the halves of (h0, -h1) of every row and coil, scaled; zero coils to pad. (With the turned halves
+// too, as the readout's, bp_cotangent read twice the bytes: 0.83 -> 0.89 ms at 1,048,576 spins x 512 samples.)
 __global__ void bp_h_split_kernel(const float* __restrict__ h, int rows, int n_coils, int width, const uint32_t* most,
                                   uint2* __restrict__ hs) {
     float scale, inverse;
@@ -50,12 +51,16 @@ __global__ void bp_h_split_kernel(const float* __restrict__ h, int rows, int n_c
     const int64_t r = i / width;
     const int c = (int)(i - r * width);
     uint2 v = make_uint2(0u, 0u);
-    if (c < n_coils) v = split_sens(h[r * 2 * n_coils + 2 * c] * scale, h[r * 2 * n_coils + 2 * c + 1] * scale);
+    if (c < n_coils) {
+        const uint4 u = split_sens(h[r * 2 * n_coils + 2 * c] * scale, h[r * 2 * n_coils + 2 * c + 1] * scale);
+        v = make_uint2(u.x, u.y);
+    }
     hs[i] = v;
 }
 
 #define CO_THREADS 128
 #define CO_WARPS (CO_THREADS / 32)
+#define CO_TAB_STRIDE 36  // float2 per row of the powers (32 spins + 4)
 #define CO_ONE 128.0f  // the powers' scale: a power of two that keeps their low halves normal, and 255 times them a half
 
 struct CotArgs {
@@ -92,7 +97,7 @@ __device__ __forceinline__ int run_from(const int4* __restrict__ runs, int n_run
 // gridDim.y-th run (one part with coil gradients: they are summed over the runs, last to first).
 template <bool WANT1>
 __global__ void __launch_bounds__(CO_THREADS, WANT1 ? 3 : 4) bp_cotangent_kernel(CotArgs a) {
-    __shared__ float2 tabs[CO_WARPS][RO_ROWS * RO_TAB_STRIDE];  // conj(q)^0 .. conj(q)^7 per spin
+    __shared__ float2 tabs[CO_WARPS][RO_ROWS * CO_TAB_STRIDE];  // conj(q)^0 .. conj(q)^7 per spin
     __shared__ float2 steps[CO_WARPS][2][32];                   // conj(q)^8, conj(q)^32
     __shared__ float2 firsts[CO_WARPS][32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -128,7 +133,7 @@ __global__ void __launch_bounds__(CO_THREADS, WANT1 ? 3 : 4) bp_cotangent_kernel
 #pragma unroll
             for (int i = 1; i < RO_ROWS; ++i) {
                 readout_advance(f, zr, zi);
-                tab[i * RO_TAB_STRIDE + lane] = make_float2(zr, zi);
+                tab[i * CO_TAB_STRIDE + lane] = make_float2(zr, zi);
             }
             steps[warp][0][lane] = q8;
             steps[warp][1][lane] = q32;
@@ -146,8 +151,8 @@ __global__ void __launch_bounds__(CO_THREADS, WANT1 ? 3 : 4) bp_cotangent_kernel
                 float tr[4] = {0.f, 0.f, 0.f, 0.f}, ti[4] = {0.f, 0.f, 0.f, 0.f};
                 float ur[4] = {0.f, 0.f, 0.f, 0.f}, ui[4] = {0.f, 0.f, 0.f, 0.f};
                 // samples t and t + 4 of the block of 32, two spins; their steps by eight and by 32
-                const float2 ta = tab[t * RO_TAB_STRIDE + sa], ta4 = tab[(t + 4) * RO_TAB_STRIDE + sa];
-                const float2 tb = tab[t * RO_TAB_STRIDE + sb], tb4 = tab[(t + 4) * RO_TAB_STRIDE + sb];
+                const float2 ta = tab[t * CO_TAB_STRIDE + sa], ta4 = tab[(t + 4) * CO_TAB_STRIDE + sa];
+                const float2 tb = tab[t * CO_TAB_STRIDE + sb], tb4 = tab[(t + 4) * CO_TAB_STRIDE + sb];
                 CPair wa{make_float2(ta.x, ta4.x), make_float2(ta.y, ta4.y)};
                 CPair wb{make_float2(tb.x, tb4.x), make_float2(tb.y, tb4.y)};
                 const float2 ea = steps[warp][0][sa], eb = steps[warp][0][sb];
@@ -276,7 +281,7 @@ struct SweepArgs {
 // bp_adjoint's rf_back, with the per-spin gradients of rf_reverse where SG. gx, gy: dL/d(-2 pi dt rf).
 template <int K>
 struct BackRun {
-    Pk<K> a1, a2, ia1, ia2, pe, npe;  // half-step factors and their inverses, pd expm1(-dt r1 / 2) and its negative
+    Pk<K> a1, a2, ia1, ia2, pe;  // half-step factors and their inverses, pd expm1(-dt r1 / 2)
     Pk<K> wz, nwz, wz2;
 };
 
@@ -468,19 +473,19 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : 4) bp_sweep_kernel(SweepArg
                         load_state(a.wstates + (size_t)sl * 6 * n, ox, oy, oz);
                 }
                 BackRun<K> rb;
-                float a1[K], a2[K], i1[K], i2[K], pe[K], npe[K], wz[K], nwz[K], wz2[K];
+                float a1[K], a2[K], i1[K], i2[K], pe[K], wz[K], nwz[K], wz2[K];
                 bool small = true;
 #pragma unroll
                 for (int k = 0; k < K; ++k) {
                     const float e1h = relax_expm1(-0.5f * q.dt * p[k].r1), e2h = relax_expm1(-0.5f * q.dt * p[k].r2);
                     a1[k] = 1.0f + e1h, a2[k] = 1.0f + e2h, i1[k] = 1.0f / a1[k], i2[k] = 1.0f / a2[k];
-                    pe[k] = p[k].pd * e1h, npe[k] = -pe[k];
+                    pe[k] = p[k].pd * e1h;
                     Spin s{};
                     s.px = (float)p[k].x, s.py = (float)p[k].y, s.pz = (float)p[k].z, s.db0 = (float)p[k].db0;
                     wz[k] = rf_wz(q, s), nwz[k] = -wz[k], wz2[k] = wz[k] * wz[k];
                 }
                 rb.a1 = pmake<K>(a1), rb.a2 = pmake<K>(a2), rb.ia1 = pmake<K>(i1), rb.ia2 = pmake<K>(i2);
-                rb.pe = pmake<K>(pe), rb.npe = pmake<K>(npe);
+                rb.pe = pmake<K>(pe);
                 rb.wz = pmake<K>(wz), rb.nwz = pmake<K>(nwz), rb.wz2 = pmake<K>(wz2);
                 // the window's RF, a segment per lane (its other values are the first segment's); every rotation small for
                 // every spin of the warp: |w|^2 <= b1^2 max(wx0^2 + wy0^2) + wz^2
