@@ -651,16 +651,21 @@ extern "C" int bp_surrogate_pulse(const float* spins, float* state, int n, const
 
 // ---- inference on the tensor cores: all four layers as tcgen05 matrix products ----
 //
-// Per CTA tile of 128 spins (thread t = spin row t = tensor-memory lane t), four rounds, one per layer: every
+// A CTA is two groups of four warps, each with tiles of its own, that share one copy of the weights: with a copy per tile
+// the shared memory held three tiles per SM, now four. The GELU's arithmetic runs on paired instructions with one
+// reciprocal for two values (the special-function unit was its bound). One 300-step pulse over 393,216 spins: 0.0924 ms
+// before; 0.0782 with the pairs and one group in each of three CTAs, 0.0761 with two blocks of columns in flight, 0.0739
+// with two groups in each of two CTAs; five groups in one CTA 0.0787, four 0.086.
+// Per tile of 128 spins (a group's thread t = spin row t = tensor-memory lane t), four rounds, one per layer: every
 // thread stores its row of the layer's input, split into bfloat16 high and low parts, as the A operand (K-major),
 // one thread issues D = A_hi W_hi^T + A_hi W_lo^T + A_lo W_hi^T (M = 128, float32 accumulation in tensor memory),
 // and every thread reads its row of D back (tcgen05.ld) and adds the bias (and GELU for layers 1 to 3):
 //   layer 1: the 14 input features, zero-padded to K = 16 (one K step), N = 64, D in columns [0, 64);
 //   layers 2 and 3: K = 64 (4 steps), N = 64, D in columns [0, 64);
-//   layer 4: K = 64, N = 16, D in columns [64, 80).
+//   layer 4: K = 64, N = 16, D in columns [0, 16) (every thread has read layer 3's).
 // Shared memory: W2 hi, W2 lo, W3 hi, W3 lo (8192 bytes each, [0, 32768)), W1 hi, W1 lo ([32768, 36864)), W4 hi,
-// W4 lo ([36864, 40960)), A hi and A lo (16384 each, [40960, 73728)), the fallback queue, mbarriers. The biases
-// travel in the kernel's arguments (the constant bank). Layout of every operand: core matrices of 8 rows x 16
+// W4 lo ([36864, 40960)), every group's A hi and A lo (16384 each), their fallback queues, mbarriers. The biases travel
+// in the kernel's arguments (the constant bank). Layout of every operand: core matrices of 8 rows x 16
 // bytes, K-adjacent ones 128 bytes apart, 8-row groups 1024 bytes apart (W1: 256, its rows being 16 wide); a thread
 // writes its row 16 bytes at a time, so the 8 lanes of each store phase fill one 128-byte line.
 #include "tcgen05.cuh"
@@ -673,19 +678,53 @@ extern "C" int bp_surrogate_pulse(const float* spins, float* state, int n, const
 #define SI_WT_BYTES (SI_OFF_W4 + 2 * SI_W4_BYTES)  // 40960: every weight tile, one bulk copy
 #define SI_OFF_A SI_WT_BYTES
 #define SI_A_BYTES 16384
-#define SI_OFF_LIST (SI_OFF_A + 2 * SI_A_BYTES)  // queued fallback spins (256 ints), after the A operand
+#define SI_GROUPS 2                              // tiles in flight per CTA (32 KB of A operand each), two CTAs per SM
+#define SI_THREADS (128 * SI_GROUPS)
+#define SI_OFF_LIST (SI_OFF_A + SI_GROUPS * 2 * SI_A_BYTES)  // queued fallback spins (256 ints per group)
 #define SI_LIST 256
-#define SI_OFF_BAR (SI_OFF_LIST + SI_LIST * 4)
-#define SI_SMEM (SI_OFF_BAR + 64)
+#define SI_OFF_BAR (SI_OFF_LIST + SI_GROUPS * SI_LIST * 4)  // mbarriers: the weights', a group's MMAs; then the rest
+#define SI_SMEM (SI_OFF_BAR + (1 + SI_GROUPS) * 8 + (1 + SI_GROUPS) * 4)
 #define SI_LBO 128
 #define SI_SBO 1024
 #define SI_SBO_W1 256
-#define SI_COLS 128   // tensor-memory columns: D of layers 1 to 3 in [0, 64), of layer 4 in [64, 80)
-#define SI_D4 64
+#define SI_COLS 128   // tensor-memory columns: a group's D in its 64
+#define SI_D 64
 #define SI_K1 16      // layer 1's K: the features, zero-padded
 
 static_assert(SI_OFF_A % 1024 == 0 && SI_OFF_W1 % 16 == 0 && SI_OFF_W4 % 16 == 0, "operand alignment");
 static_assert(MLP_IN <= SI_K1, "layer 1 fits one K step");
+static_assert(SI_GROUPS * SI_D <= SI_COLS, "tensor memory");
+
+// The group's 128 threads meet (named barrier 1 + group); with a predicate: whether any of them has it set.
+__device__ __forceinline__ void group_sync(int group) {
+    asm volatile("barrier.cta.sync %0, 128;" ::"r"(1 + group) : "memory");
+}
+__device__ __forceinline__ bool group_sync_or(int group, bool pred) {
+    uint32_t any;
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n barrier.cta.red.or.pred q, %2, 128, p;\n"
+        " selp.u32 %0, 1, 0, q;\n}"
+        : "=r"(any)
+        : "r"((uint32_t)pred), "r"(1 + group)
+        : "memory");
+    return any != 0;
+}
+
+// gelu_f of two values: its arithmetic on paired instructions, exp2 and the reciprocal without the handling of
+// denormals (1 + exp(-2u) is never one, and an exp(-2u) that is one does not change the sum).
+__device__ __forceinline__ float2 gelu_pair(const float2& x) {
+    const float k = -2.0f * 0.7978845608028654f * 1.4426950408889634f;  // -2 c log2(e)
+    const float2 t = __ffma2_rn(__fmul2_rn(x, make_float2(0.044715f, 0.044715f)), __fmul2_rn(x, x), x);
+    float2 u = __fmul2_rn(t, make_float2(k, k)), e, s;
+    u.x = fminf(u.x, 60.0f), u.y = fminf(u.y, 60.0f);  // (the product of the denominators stays finite)
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(u.x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(u.y));
+    const float2 d = __fadd2_rn(e, make_float2(1.0f, 1.0f));
+    float both;  // one reciprocal for the two: 1 / x = y / (x y)
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(both) : "f"(d.x * d.y));
+    s = __fmul2_rn(make_float2(d.y, d.x), make_float2(both, both));
+    return __fmul2_rn(x, s);
+}
 
 // NCH x 8 values of this thread's row -> A hi and A lo rows, chunks [chunk0, chunk0 + NCH) (16-byte stores)
 template <int NCH>
@@ -699,7 +738,8 @@ __device__ __forceinline__ void store_row_bf16x2(unsigned char* ahi, unsigned ch
             const float v0 = v[8 * c + 2 * w], v1 = v[8 * c + 2 * w + 1];
             const __nv_bfloat162 hp = __floats2bfloat162_rn(v0, v1);
             const float2 hf = __bfloat1622float2(hp);
-            const __nv_bfloat162 lp = __floats2bfloat162_rn(v0 - hf.x, v1 - hf.y);
+            const float2 rest = __ffma2_rn(hf, make_float2(-1.0f, -1.0f), make_float2(v0, v1));
+            const __nv_bfloat162 lp = __floats2bfloat162_rn(rest.x, rest.y);
             h[w] = *reinterpret_cast<const uint32_t*>(&hp);
             l[w] = *reinterpret_cast<const uint32_t*>(&lp);
         }
@@ -723,40 +763,40 @@ struct PulseMmaArgs {
 };
 
 // (__grid_constant__: the biases are indexed in place in the parameter space, not copied to the stack)
-__global__ void __launch_bounds__(128, 3) bp_surrogate_pulse_mma_kernel(const __grid_constant__ PulseMmaArgs args) {
+__global__ void __launch_bounds__(SI_THREADS, 2) bp_surrogate_pulse_mma_kernel(const __grid_constant__ PulseMmaArgs args) {
     extern __shared__ __align__(1024) unsigned char smb[];
     const PulseArgs& a = args.p;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smb + SI_OFF_BAR);  // [0] weights, [1] MMA
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smb + SI_OFF_BAR + 2 * sizeof(uint64_t));
-    int* queued = reinterpret_cast<int*>(smb + SI_OFF_BAR + 3 * sizeof(uint64_t));
-    int* flist = reinterpret_cast<int*>(smb + SI_OFF_LIST);
-    unsigned char* ahi = smb + SI_OFF_A;
-    unsigned char* alo = smb + SI_OFF_A + SI_A_BYTES;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int group = threadIdx.x >> 7, tid = threadIdx.x & 127, warp = tid >> 5;  // (within the group)
+    uint64_t* wbar = reinterpret_cast<uint64_t*>(smb + SI_OFF_BAR);  // the weights'
+    uint64_t* bar = wbar + 1 + group;                                // the group's MMAs'
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wbar + 1 + SI_GROUPS);
+    int* queued = reinterpret_cast<int*>(tmem_slot + 1) + group;
+    int* flist = reinterpret_cast<int*>(smb + SI_OFF_LIST) + group * SI_LIST;
+    unsigned char* ahi = smb + SI_OFF_A + group * 2 * SI_A_BYTES;
+    unsigned char* alo = ahi + SI_A_BYTES;
     const uint32_t sW = smem_u32(smb), sA = smem_u32(ahi);
 
     const float* bias = args.net.bias;
-    if (tid == 0) {
-        *queued = 0;
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
+    if (threadIdx.x == 0) {
+        for (int g = 0; g < SI_GROUPS; ++g) queued[g] = 0;
+        for (int g = 0; g <= SI_GROUPS; ++g) mbar_init(&wbar[g], 1);
         fence_mbar_init();
         fence_proxy_async_smem();
-        mbar_expect_tx(&bars[0], SI_WT_BYTES);
-        tma_load_1d(smb, args.wtiles, SI_WT_BYTES, &bars[0]);
+        mbar_expect_tx(wbar, SI_WT_BYTES);
+        tma_load_1d(smb, args.wtiles, SI_WT_BYTES, wbar);
     }
-    if (warp == 0) tmem_alloc(tmem_slot, SI_COLS);
+    if (threadIdx.x < 32) tmem_alloc(tmem_slot, SI_COLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem_base = *tmem_slot, tmem = tmem_base + group * SI_D;
     const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
 
     uint32_t mma_phase = 0;
     bool w_ready = false, fail = false, err = false, mma_out = false;
     const int n_tiles = (a.n + 127) / 128;
 
-    for (int tile = blockIdx.x; tile < n_tiles && !fail; tile += gridDim.x) {
+    for (int tile = blockIdx.x + group * gridDim.x; tile < n_tiles && !fail; tile += SI_GROUPS * gridDim.x) {
         const int j0 = tile * 128 + tid;
         const bool active = j0 < a.n;
         const int j = active ? j0 : 0;
@@ -764,90 +804,7 @@ __global__ void __launch_bounds__(128, 3) bp_surrogate_pulse_mma_kernel(const __
         const float df = p.db0 + a.b0off;
         const float zr = (float)(((double)p.pz - a.z0) / a.thickness);
         const bool inside = active && fabsf(df) <= a.dom_df && fabsf(p.b1 - 1.0f) <= a.dom_b1 && fabsf(zr) <= a.dom_z;
-        float y[MLP_OUT];
-        {   // layer 1's input: the features, zero-padded to 16, as the A operand's first two chunks
-            float xin[MLP_X], g[SI_K1];
-            pulse_inputs(a, p, df, xin);
-            mlp_features(xin[0], xin[1], g);
-#pragma unroll
-            for (int i = MLP_IN; i < SI_K1; ++i) g[i] = 0.0f;
-            store_row_bf16x2<SI_K1 / 8>(ahi, alo, tid, g, 0);
-        }
-#pragma unroll 1
-        for (int layer = 0; layer < 4; ++layer) {  // a real loop: one copy of the code serves the four layers
-            fence_proxy_async_smem();
-            tc_fence_before();
-            if (__syncthreads_or(err)) {
-                fail = true;
-                break;
-            }
-            if (tid == 0) {
-                if (!w_ready && !mbar_wait_bounded(&bars[0], 0)) err = true;
-                w_ready = true;
-                if (!err) {
-                    tc_fence_after();
-                    const uint32_t wh = layer == 0 ? sW + SI_OFF_W1
-                                      : layer == 3 ? sW + SI_OFF_W4
-                                                   : sW + (uint32_t)(2 * (layer - 1)) * SI_W_BYTES;
-                    const uint32_t wl = wh + (layer == 0 ? SI_W1_BYTES : layer == 3 ? SI_W4_BYTES : SI_W_BYTES);
-                    const uint32_t sbo_w = layer == 0 ? SI_SBO_W1 : SI_SBO;
-                    const uint32_t idesc = umma_idesc_bf16_f32(128, layer == 3 ? MLP_OUT : MLP_H);
-                    const uint32_t d = tmem + (layer == 3 ? SI_D4 : 0u);
-                    uint64_t ah_d = umma_desc(sA, SI_LBO, SI_SBO), al_d = umma_desc(sA + SI_A_BYTES, SI_LBO, SI_SBO);
-                    uint64_t bh_d = umma_desc(wh, SI_LBO, sbo_w), bl_d = umma_desc(wl, SI_LBO, sbo_w);
-                    const int k_steps = layer == 0 ? SI_K1 / 16 : MLP_H / 16;
-                    for (int kk = 0; kk < k_steps; ++kk) {
-                        umma_bf16(d, ah_d, bh_d, idesc, kk > 0 ? 1u : 0u);
-                        umma_bf16(d, ah_d, bl_d, idesc, 1u);
-                        umma_bf16(d, al_d, bh_d, idesc, 1u);
-                        ah_d += 2 * SI_LBO / 16, al_d += 2 * SI_LBO / 16, bh_d += 2 * SI_LBO / 16, bl_d += 2 * SI_LBO / 16;
-                    }
-                    umma_commit(&bars[1]);
-                }
-            }
-            mma_out = true;
-            if (mbar_wait_bounded(&bars[1], mma_phase)) {
-                mma_phase ^= 1u;
-                mma_out = false;
-            } else {
-                err = true;
-            }
-            if (__syncthreads_or(err)) {
-                fail = true;
-                break;
-            }
-            tc_fence_after();
-            if (layer < 3) {
-                // the layer's output 16 columns at a time: bias and GELU, split straight into the next A operand
-                // (the MMA that read the A operand has completed)
-                const float* b = bias + layer * MLP_H;
-#pragma unroll 1
-                for (int c0 = 0; c0 < MLP_H; c0 += 16) {
-                    float d[16];
-                    tmem_ld16(lane_addr + (uint32_t)c0, d);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) d[i] = gelu_f(d[i] + b[c0 + i]);
-                    store_row_bf16x2<2>(ahi, alo, tid, d, c0 / 8);
-                }
-            } else {
-                float d[16];
-                tmem_ld16(lane_addr + (uint32_t)SI_D4, d);
-                tmem_ld_wait();
-#pragma unroll
-                for (int o = 0; o < MLP_OUT; ++o) y[o] = d[o] + bias[3 * MLP_H + o];
-            }
-            tc_fence_before();
-        }
-        if (fail) break;
-        if (inside) {
-            float mx = a.state[j], my = a.state[a.n + j], mz = a.state[2 * a.n + j];
-            float lx = a.state[3 * a.n + j], ly = a.state[4 * a.n + j], lz = a.state[5 * a.n + j];
-            apply_pulse_map(y, a, p, df, mx, my, mz, lx, ly, lz);
-            a.state[j] = mx, a.state[a.n + j] = my, a.state[2 * a.n + j] = mz;
-            a.state[3 * a.n + j] = lx, a.state[4 * a.n + j] = ly, a.state[5 * a.n + j] = lz;
-        }
-        // spins outside the domain join the CTA's queue; whenever it holds 128, all threads step them (full warps
+        // spins outside the domain join the group's queue; whenever it holds 128, its threads step them (full warps
         // whatever the spins' order)
         const unsigned in_mask = __ballot_sync(0xffffffffu, inside);
         const unsigned out_mask = __ballot_sync(0xffffffffu, active && !inside);
@@ -861,25 +818,111 @@ __global__ void __launch_bounds__(128, 3) bp_surrogate_pulse_mma_kernel(const __
             base = __shfl_sync(0xffffffffu, base, 0);
             if (active && !inside) flist[base + __popc(out_mask & ((1u << (tid & 31)) - 1u))] = j;
         }
-        __syncthreads();
-        const int nq = *queued;
+        float y[MLP_OUT];
+        {   // layer 1's input: the features, zero-padded to 16, as the A operand's first two chunks
+            float xin[MLP_X], g[SI_K1];
+            pulse_inputs(a, p, df, xin);
+            mlp_features(xin[0], xin[1], g);
+#pragma unroll
+            for (int i = MLP_IN; i < SI_K1; ++i) g[i] = 0.0f;
+            store_row_bf16x2<SI_K1 / 8>(ahi, alo, tid, g, 0);
+        }
+#pragma unroll 1
+        for (int layer = 0; layer < 4; ++layer) {  // a real loop: one copy of the code serves the four layers
+            fence_proxy_async_smem();
+            tc_fence_before();
+            if (group_sync_or(group, err)) {
+                fail = true;
+                break;
+            }
+            if (tid == 0) {
+                if (!w_ready && !mbar_wait_bounded(wbar, 0)) err = true;
+                w_ready = true;
+                if (!err) {
+                    tc_fence_after();
+                    const uint32_t wh = layer == 0 ? sW + SI_OFF_W1
+                                      : layer == 3 ? sW + SI_OFF_W4
+                                                   : sW + (uint32_t)(2 * (layer - 1)) * SI_W_BYTES;
+                    const uint32_t wl = wh + (layer == 0 ? SI_W1_BYTES : layer == 3 ? SI_W4_BYTES : SI_W_BYTES);
+                    const uint32_t sbo_w = layer == 0 ? SI_SBO_W1 : SI_SBO;
+                    const uint32_t idesc = umma_idesc_bf16_f32(128, layer == 3 ? MLP_OUT : MLP_H);
+                    uint64_t ah_d = umma_desc(sA, SI_LBO, SI_SBO), al_d = umma_desc(sA + SI_A_BYTES, SI_LBO, SI_SBO);
+                    uint64_t bh_d = umma_desc(wh, SI_LBO, sbo_w), bl_d = umma_desc(wl, SI_LBO, sbo_w);
+                    const int k_steps = layer == 0 ? SI_K1 / 16 : MLP_H / 16;
+                    for (int kk = 0; kk < k_steps; ++kk) {
+                        umma_bf16(tmem, ah_d, bh_d, idesc, kk > 0 ? 1u : 0u);
+                        umma_bf16(tmem, ah_d, bl_d, idesc, 1u);
+                        umma_bf16(tmem, al_d, bh_d, idesc, 1u);
+                        ah_d += 2 * SI_LBO / 16, al_d += 2 * SI_LBO / 16, bh_d += 2 * SI_LBO / 16, bl_d += 2 * SI_LBO / 16;
+                    }
+                    umma_commit(bar);
+                }
+            }
+            mma_out = true;
+            if (mbar_wait_bounded(bar, mma_phase)) {
+                mma_phase ^= 1u;
+                mma_out = false;
+            } else {
+                err = true;  // (seen by all at the next barrier; what is stored until then is not used)
+            }
+            tc_fence_after();
+            if (layer < 3) {
+                // the layer's output 16 columns at a time: bias and GELU, split straight into the next A operand
+                // (the MMA that read the A operand has completed)
+                const float* b = bias + layer * MLP_H;
+#pragma unroll 2
+                for (int c0 = 0; c0 < MLP_H; c0 += 16) {
+                    float d[16];
+                    tmem_ld16(lane_addr + (uint32_t)c0, d);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 16; i += 2) {
+                        const float2 g = gelu_pair(__fadd2_rn(make_float2(d[i], d[i + 1]),
+                                                              make_float2(b[c0 + i], b[c0 + i + 1])));
+                        d[i] = g.x, d[i + 1] = g.y;
+                    }
+                    store_row_bf16x2<2>(ahi, alo, tid, d, c0 / 8);
+                }
+            } else {
+                float d[16];
+                tmem_ld16(lane_addr, d);
+                tmem_ld_wait();
+#pragma unroll
+                for (int o = 0; o < MLP_OUT; ++o) y[o] = d[o] + bias[3 * MLP_H + o];
+            }
+            tc_fence_before();
+        }
+        if (fail) break;
+        const int nq = *queued;  // (no thread adds to it between the first layer's barrier and the next)
+        if (group_sync_or(group, err)) {
+            fail = true;
+            break;
+        }
+        if (inside) {
+            float mx = a.state[j], my = a.state[a.n + j], mz = a.state[2 * a.n + j];
+            float lx = a.state[3 * a.n + j], ly = a.state[4 * a.n + j], lz = a.state[5 * a.n + j];
+            apply_pulse_map(y, a, p, df, mx, my, mz, lx, ly, lz);
+            a.state[j] = mx, a.state[a.n + j] = my, a.state[2 * a.n + j] = mz;
+            a.state[3 * a.n + j] = lx, a.state[4 * a.n + j] = ly, a.state[5 * a.n + j] = lz;
+        }
         if (nq >= 128) {
             fallback_spin(a, flist[nq - 128 + tid]);
-            __syncthreads();
+            group_sync(group);
             if (tid == 0) *queued = nq - 128;
+            group_sync(group);
         }
-        __syncthreads();
     }
+    group_sync(group);
     if (!fail && tid < *queued) fallback_spin(a, flist[tid]);
     // leave no copy or MMA in flight (failure paths), then free the tensor memory
-    if (tid == 0 && !w_ready) mbar_wait_bounded(&bars[0], 0);
-    if (mma_out) mbar_wait_bounded(&bars[1], mma_phase);
+    if (tid == 0 && !w_ready) mbar_wait_bounded(wbar, 0);
+    if (mma_out) mbar_wait_bounded(bar, mma_phase);
     if ((fail || err) && tid == 0 && args.status) atomicOr(args.status, BP_ERR_TMA_TIMEOUT);
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) {
+    if (threadIdx.x < 32) {
         tc_fence_after();
-        tmem_dealloc(tmem, SI_COLS);
+        tmem_dealloc(tmem_base, SI_COLS);
     }
 }
 
@@ -949,9 +992,9 @@ static int pulse_mma_grid(int n, int max_ctas, int* grid_out) {
         cudaFuncGetAttributes(&fa, bp_surrogate_pulse_mma_kernel) != cudaSuccess)
         return BP_E_LAUNCH;
     int per_sm = smem_sm / (SI_SMEM + smem_res);
-    const int regs_block = ((fa.numRegs * 32 + 255) / 256) * 256 * 4;
+    const int regs_block = ((fa.numRegs * 32 + 255) / 256) * 256 * (SI_THREADS / 32);
     if (regs_block > 0 && regs_sm / regs_block < per_sm) per_sm = regs_sm / regs_block;
-    if (thr_sm / 128 < per_sm) per_sm = thr_sm / 128;
+    if (thr_sm / SI_THREADS < per_sm) per_sm = thr_sm / SI_THREADS;
     if (per_sm > 512 / SI_COLS) per_sm = 512 / SI_COLS;
     if (per_sm < 1) per_sm = 1;
     const int n_tiles = (n + 127) / 128;
@@ -988,6 +1031,6 @@ extern "C" int bp_surrogate_pulse_mma(const float* spins, float* state, int n, c
     std::memcpy(a.net.bias + MLP_H, params_host + P_B2, MLP_H * sizeof(float));
     std::memcpy(a.net.bias + 2 * MLP_H, params_host + P_B3, MLP_H * sizeof(float));
     std::memcpy(a.net.bias + 3 * MLP_H, params_host + P_B4, MLP_OUT * sizeof(float));
-    bp_surrogate_pulse_mma_kernel<<<grid, 128, SI_SMEM, static_cast<cudaStream_t>(stream)>>>(a);
+    bp_surrogate_pulse_mma_kernel<<<grid, SI_THREADS, SI_SMEM, static_cast<cudaStream_t>(stream)>>>(a);
     return cudaGetLastError() == cudaSuccess ? BP_OK : BP_E_LAUNCH;
 }

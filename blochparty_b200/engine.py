@@ -404,9 +404,23 @@ def forward_spans(pk: Packed, state: torch.Tensor, plan, spans, raw: torch.Tenso
         return
     rng = np.ascontiguousarray(np.asarray(ranges, dtype=np.int32).reshape(-1, 2))
     n_spans = rng.shape[0] - 1
+    # the first sample of every run of samples, of as many ranges at a time as Z_BYTES holds
+    runs, z, run_at, cap = None, None, None, 0
+    if raw is not None:
+        runs = pk.sample_runs()
+        starts = plan[0][:, 0]
+        first = [int(starts[wa]) if wa < len(starts) else pk.flags.shape[0] for wa, _ in ranges] + [pk.flags.shape[0]]
+        run_at = np.ascontiguousarray(np.searchsorted(runs.starts, first), dtype=np.int32)
+        cap = min(runs.n_runs, max(Z_BYTES // (8 * max(pk.n, 1)), 1))
+        if 0 < int(np.diff(run_at).max()) <= cap:
+            z = torch.empty(cap, pk.n, 2, dtype=F32, device=pk.device)
     code = _lib.lib().bp_forward_spans(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64),
                                        ptr(wdev), rng.ctypes.data, n_spans, ctypes.addressof(spans) if n_spans else None,
-                                       ptr(state), ptr(raw), max_ctas, ptr(status), _lib.stream_ptr())
+                                       ptr(state), ptr(raw), max_ctas, ptr(runs.runs) if z is not None else None,
+                                       runs.n_runs if z is not None else 0, ptr(runs.subs) if z is not None else None,
+                                       runs.n_subs if z is not None else 0,
+                                       run_at.ctypes.data if z is not None else None, ptr(z), cap, ptr(status),
+                                       _lib.stream_ptr())
     _lib.check(code, "bp_forward_spans")
 
 

@@ -126,10 +126,9 @@ class Reuse:
 
 def forward_with_reuse(inp, device, max_ctas: int = 0, memory: int = PULSE_MEMORY):
     """``simulate(..., pulses="reuse")``: signal (C, A) complex64 and m (N, 3) float32 on the CPU."""
-    pk = engine.pack(inp, device)
+    pk, state = engine.pack_with_state(inp, device)
     reuse = Reuse(inp, pk, memory)
     reuse.make_maps(pk)
-    state = engine.initial_state(inp.pd, inp.m_init, device)
     raw = torch.zeros(max(pk.n_adc, 1), 2 * pk.n_coils, dtype=F64, device=device)
     status = torch.zeros(1, dtype=torch.int32, device=device)
     reuse.run(pk, state, raw if pk.n_adc else None, status, max_ctas)

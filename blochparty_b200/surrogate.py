@@ -384,9 +384,8 @@ def run_with_surrogates(inp, device, surrogates, inference: str = "mma"):
     """The forward with every matched pulse occurrence through its surrogate; returns (signal, m, counts).
     ``inference``: "mma" (layers 2 and 3 on the tensor cores, ``bp_surrogate_pulse_mma``) or "fp32" (the whole
     network on the CUDA cores, ``bp_surrogate_pulse``)."""
-    pk = engine.pack(inp, device)
+    pk, state = engine.pack_with_state(inp, device)
     plan = SurrogateRun(inp, pk, surrogates, inference)
-    state = engine.initial_state(inp.pd, inp.m_init, device)
     raw = torch.zeros(max(pk.n_adc, 1), 2 * pk.n_coils, dtype=F64, device=device)
     status = torch.zeros(1, dtype=torch.int32, device=device)
     counts = torch.zeros(2, dtype=torch.int32, device=device)

@@ -448,14 +448,17 @@ int bp_surrogate_pulse_mma(const float* spins, float* state, int n, const float*
 
 /* ---- a forward with pulse occurrences replaced (the launch loop of pulses="reuse" / "surrogate") ----
  * bp_forward_spans steps windows ranges[0] = [w0, w1), then replaces span 0, steps ranges[1], replaces span 1, ...,
- * and steps ranges[n_spans] last: 2 n_spans + 1 launches issued from host code in one call (ranges: host int32
+ * and steps ranges[n_spans] last, all launches issued from host code in one call (ranges: host int32
  * [n_spans + 1][2]; spans: host array). Every span replaces the segments [seg0, seg0 + k_steps) it names, which
  * the windows leave out. A span is one of:
  *   BP_SPAN_MAP      bp_pulse_apply(map, n, state, phase)                 (map: device [12][n] float64)
  *   BP_SPAN_NET_MMA  bp_surrogate_pulse_mma(..., params (host), wtiles, ...)
  *   BP_SPAN_NET_F32  bp_surrogate_pulse(..., params (device), ...)
- * with phase = the RF phase (phi0 of a network), and the network fields as in those calls. Returns the first
- * failing call's status (launches before it stay queued). */
+ * with phase = the RF phase (phi0 of a network), and the network fields as in those calls. With a workspace z
+ * [z_cap][n] pairs the windows are stepped by bp_propagate, with one bp_readout (runs, subs as there) over as many
+ * ranges as z holds the runs of, and once at the end; run_at (host int32 [n_spans + 2]): the runs that start before
+ * each range, then all; no range may have more than z_cap of them. With z = NULL and raw they are stepped by
+ * bp_forward. Returns the first failing call's status (launches before it stay queued). */
 #define BP_SPAN_MAP 0
 #define BP_SPAN_NET_MMA 1
 #define BP_SPAN_NET_F32 2
@@ -472,7 +475,9 @@ typedef struct {
 } BpSpan;
 int bp_forward_spans(const float* spins, const float* sens, int n, int n_coils, const void* segs,
                      const double* seg64, const int32_t* windows, const int32_t* ranges, int n_spans,
-                     const BpSpan* spans, float* state, double* raw, int max_ctas, int32_t* status, void* stream);
+                     const BpSpan* spans, float* state, double* raw, int max_ctas, const int32_t* runs, int n_runs,
+                     const int32_t* subs, int n_subs, const int32_t* run_at, float* z, int z_cap, int32_t* status,
+                     void* stream);
 
 /* Measurement kernel (the roofline denominator): 4 CTAs x 256 threads per SM, each thread `iters` x 128
  * independent FFMAs; `*flops` receives the flop count of the launch, which the caller divides by the launch's
