@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : HELP ? 5 : 4) bp_propagate_
     int* slots = list + CH;                                       // [CH]: the slot that takes the state at a segment
     uint64_t* bars = reinterpret_cast<uint64_t*>(slots + CH);
     float* ring = reinterpret_cast<float*>(bars + 2);             // HELP: [2][ST_BATCH][6][32] factors
-    __shared__ int count[NT / 32 + 1], windows_in;
+    __shared__ int count[NT / 32 + 1];
+    __shared__ int windows_in[2];  // windows that start in a chunk, by the chunk's parity
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = a.n;
     constexpr int TILE = (HELP ? 32 : NT) * K;
@@ -121,6 +122,7 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : HELP ? 5 : 4) bp_propagate_
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
         fence_mbar_init();
+        windows_in[0] = windows_in[1] = 0;
     }
     __syncthreads();
     auto issue = [&](int c, int buf) {
@@ -190,12 +192,12 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : HELP ? 5 : 4) bp_propagate_
             const bool ok = mbar_wait_bounded(&bars[buf], (it >> 1) & 1);
             const SegRec* q0 = segbuf + buf * CH;
             const double4* k0 = k64buf + buf * CH;
-            if (tid == 0) windows_in = 0;
             if (__syncthreads_or(!ok)) {  // (and every thread is done with the chunk before this one)
                 if (tid == 0) atomicOr(a.status, BP_ERR_TMA_TIMEOUT);
                 return;
             }
             if (tid == 0) {  // the next chunk, of this tile or the next one, after the check: nothing left in flight
+                windows_in[(it + 1) & 1] = 0;  // (every thread has read the chunk before's, which the next one takes)
                 if (c_end < s_end)
                     issue(c_end, buf ^ 1);
                 else if (tile + (int)gridDim.x < n_tiles)
@@ -210,7 +212,7 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : HELP ? 5 : 4) bp_propagate_
                     const int i = w - a.w_begin;
                     if (x >= 0)
                         slots[x] = a.wslot ? a.wslot[w] : (i % a.wstate_stride) == 0 ? i / a.wstate_stride : -1;
-                    atomicAdd(&windows_in, 1);
+                    atomicAdd(&windows_in[it & 1], 1);
                 }
                 __syncthreads();
             }
@@ -253,7 +255,7 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : HELP ? 5 : 4) bp_propagate_
                 if (start) list[at + __popc(starts & ((1u << lane) - 1u))] = s | kind;
             }
             __syncthreads();
-            if (a.wstates) w_at += windows_in;
+            if (a.wstates) w_at += windows_in[it & 1];
             // a step ends where the next one starts
             auto entry = [&](int i) {
                 const int e = list[i], to = i + 1 < steps ? ST_SEG(list[i + 1]) : nseg;

@@ -119,3 +119,24 @@ def test_divided_forward(n, room, monkeypatch):
     for i, s in enumerate(states):
         assert torch.equal(saved[i], s), i
     _lib.check_status(status, "bp_propagate")
+
+
+@pytest.mark.parametrize("n", [1000, 30000, 38000])
+def test_states_saved_over_many_chunks(n):
+    """A state saved at every window of a sequence of many chunks (one warp with helpers, one warp, four warps per
+    CTA; no barrier between a chunk's steps in the last two), again and again: each the state a division passes on."""
+    ph, seq = _phantom(n, 5), _sequence((64, 95) * 6, 6)
+    pk, _, _, state0 = _packed(ph, seq, bpb.birdcage_sensitivities(ph.pos, 1))
+    win = engine.plan_windows(pk.flags, 32, seg_max=32)
+    wdev, W = torch.from_numpy(win).to(pk.device), win.shape[0]
+    assert pk.flags.shape[0] > 6 * 256 and W > 60
+    status = torch.zeros(1, dtype=torch.int32, device=pk.device)
+    want, state = [], state0.clone()
+    for w in range(W):
+        want.append(state.clone())
+        engine.run_forward(pk, state, wdev, w, w + 1, None, status)
+    for _ in range(3):
+        saved = torch.full((W, 6, n), -1.0, device=pk.device)
+        engine.run_forward(pk, state0.clone(), wdev, 0, W, None, status, wstates=saved)
+        assert torch.equal(saved, torch.stack(want))
+    _lib.check_status(status, "bp_propagate")
