@@ -126,6 +126,7 @@ def _upload_spins(pos, pd, t1, t2, db0, b1, coils, m_init, device, want_state: b
     rows = [_host(t.expand(n)) for t in (pd, t1, t2, db0)]
     pos = _host(pos.expand(n, 3))
     b1 = None if b1 is None else _host(b1.expand(n))
+    coils = coils.reshape(n, n_coils)  # (raises where it has other than n rows: the packer reads n of them)
     coils = _host(coils if coils.dtype in (torch.complex64, torch.complex128) else coils.to(torch.complex128))
     m0 = None if m_init is None else _host(m_init.expand(n, 3))
     spins = torch.empty(8, n, dtype=F32, device=device)

@@ -491,6 +491,18 @@ def test_sample_runs(seed):
     assert got.most_in(500) == most
 
 
+@pytest.mark.parametrize("rows", [1, 4, 6])
+def test_packing_refuses_coils_of_another_number_of_spins(rows):
+    """The native packer reads one row of coils per spin: fewer rows would be read past their end, more ignored."""
+    v = torch.ones(5, dtype=F64)
+    with pytest.raises(RuntimeError, match="invalid for input of size"):
+        engine._upload_spins(torch.ones(5, 3, dtype=F64), v, v, v, v, None, torch.ones(rows, 2, dtype=torch.complex64),
+                             None, "cpu", False)
+    with pytest.raises(RuntimeError, match="invalid for input of size"):  # the same on the CPU
+        engine.pack_spins(torch.ones(5, 3, dtype=F64), v, v, v, v, None, torch.ones(rows, 2, dtype=torch.complex64),
+                          "cpu")
+
+
 @pytest.mark.parametrize("S,b0", [(1, False), (5, True), (9000, True), (40000, False)])
 def test_native_segment_records(S, b0):
     """The records, moments, flags and receiver phases of the native packer against their definition in numpy, and
