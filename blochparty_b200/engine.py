@@ -174,15 +174,23 @@ def pack_spins(pos, pd, t1, t2, db0, b1, coils, device):
 def pack_segments(dt, rf, grad, b0_offset, adc_phase, is_rf, adc, spoil, device, extent: np.ndarray | None = None):
     """Segment records (float64 arithmetic, one rounding to float32), the float64 moments, psi, the flags (host) and
     the number of samples, by the native packer into one buffer and, on a GPU, one copy from page-locked memory.
-    ``extent``: the spins' extents (``_upload_spins``), to set SMALL as ``mark_small_rf`` does."""
-    arrays = [np.ascontiguousarray(_np64(t)) for t in (dt, rf, grad, adc_phase)]
-    dt, rf, grad, phase = arrays
+    ``extent``: the spins' extents (``_upload_spins``), to set SMALL as ``mark_small_rf`` does. The RF, the gradient and
+    the offset are broadcast over the segments (one offset for all of them, say); the RF's first two columns count."""
+    dt, rf = _np64(dt), _np64(rf)
     S = dt.shape[0]
-    b0 = None if b0_offset is None else np.ascontiguousarray(_np64(b0_offset))
-    shapes = ((dt, (S,)), (rf, (S, 2)), (grad, (S, 3)), (phase, (S,)), (b0, (S,)))
-    for t, shape in shapes:
-        if t is not None and t.shape != shape:
-            raise ValueError(f"a sequence of {S} segments takes an array {shape}, got {t.shape}")
+    if rf.ndim != 2 or rf.shape[1] < 2:
+        raise ValueError(f"the RF takes two columns, got {rf.shape}")
+
+    def rows(t, *shape):
+        if t.shape != shape:
+            t = np.broadcast_to(t, shape)  # (raises where it cannot)
+        return np.ascontiguousarray(t)
+
+    phase = _np64(adc_phase)
+    if dt.shape != (S,) or phase.shape != (S,):
+        raise ValueError(f"a sequence of {S} segments takes a duration and a phase for each, got {dt.shape}, {phase.shape}")
+    dt, rf, grad, phase = rows(dt, S), rows(rf[:, :2], S, 2), rows(_np64(grad), S, 3), rows(phase, S)
+    b0 = None if b0_offset is None else rows(_np64(b0_offset), S)
     marks = [np.ascontiguousarray(_bools(f, S)).view(np.uint8) for f in (is_rf, adc, spoil)]
     n_adc = int(np.count_nonzero(marks[1]))
     flags = np.empty(S, dtype=np.int32)

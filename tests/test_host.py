@@ -503,6 +503,24 @@ def test_packing_refuses_coils_of_another_number_of_spins(rows):
                           "cpu")
 
 
+def test_segment_packing_broadcasts():
+    """One offset, one gradient or one RF row for all segments, and columns past the RF's two, pack as the arrays
+    written out; what does not fit is refused."""
+    S = 6
+    g = torch.Generator().manual_seed(0)
+    rnd = lambda *s: torch.rand(*s, generator=g, dtype=F64)
+    dt, rf, grad, phase = rnd(S) * 1e-4, rnd(1, 3), rnd(1, 3), rnd(S)
+    marks = ([True] * S, [False, True] * 3, [False] * S)
+    pack = lambda rf, grad, b0: engine.pack_segments(dt, rf, grad, b0, phase, *marks, "cpu")
+    want = pack(rf[:, :2].expand(S, 2), grad.expand(S, 3), torch.full((S,), 7.0, dtype=F64))
+    for b0 in (torch.tensor(7.0, dtype=F64), torch.tensor([7.0], dtype=F64)):
+        got = pack(rf, grad, b0)
+        assert all(torch.equal(a, b) for a, b in zip(got[:3], want[:3])) and (got[3] == want[3]).all()
+    for bad in ((rnd(S, 1), grad, None), (rnd(S - 1, 2), grad, None), (rf, rnd(S, 2), None), (rf, grad, rnd(S - 1))):
+        with pytest.raises((ValueError, IndexError)):
+            pack(*bad)
+
+
 @pytest.mark.parametrize("S,b0", [(1, False), (5, True), (9000, True), (40000, False)])
 def test_native_segment_records(S, b0):
     """The records, moments, flags and receiver phases of the native packer against their definition in numpy, and
