@@ -145,6 +145,26 @@ def rf_relaxation_invertible(pk: engine.Packed) -> bool:
     return dt * r <= 1.35
 
 
+# A stretch of RF segments is integrated backward over a duration t only while t r <= 2 for the largest rate r: the
+# states' rounding errors grow by exp(t r) on the way. One window of 32 steps of 10 us with per-spin gradients, relative
+# error of dL/dR2 against float64: 7e-7 with the states recomputed forward at any T2; integrated backward 1e-6 at
+# T2 = 100 us (t r = 3.2), 2e-5 at 50 us, 3e-2 at 20 us, meaningless at 10 us.
+MAX_DECAY = 2.0
+
+
+def rf_decay(pk: engine.Packed, awin: np.ndarray) -> tuple[float, float]:
+    """(t r of the longest RF window, of the longest run of RF windows) for the adjoint windows ``awin``, each of RF or
+    of free segments (``SavedStates``): the duration times the largest relaxation rate of any spin (NaN if one is)."""
+    if awin.shape[0] == 0 or pk.n == 0:
+        return 0.0, 0.0
+    rf = (pk.flags[awin[:, 0]] & engine.RF) != 0
+    t = np.add.reduceat(pk.segs[:, 0].cpu().numpy().astype(np.float64), awin[:, 0]) * rf
+    total = np.cumsum(t)
+    run = total - np.maximum.accumulate(np.where(rf, 0.0, total))  # since the last free window
+    r = float(torch.maximum(pk.spins[4], pk.spins[5]).max())
+    return float(t.max()) * r, float(run.max()) * r
+
+
 def saved_layout(plan, state_bytes: int, budget_bytes: int):
     """(intervals per block, slots) of the backward from saved states for ``plan`` (a ``Plan`` with its
     ``saved``), or None when no layout fits ``budget_bytes`` (``state_bytes`` per stored state): every interval in
@@ -235,6 +255,9 @@ class Checkpointed:
         invertible = phys is None and rf_relaxation_invertible(pk)
         want = saved and invertible
         plan = Plan(pk, min(every, 2048), device, saved=True) if want else None
+        # (and where the pulses are short next to the relaxation: they are integrated backward whole)
+        if plan is not None and plan.saved is not None and not rf_decay(pk, plan.awin)[1] <= MAX_DECAY:
+            plan = None
         self.layout = None  # saved: (intervals per block, slots)
         if plan is not None and plan.saved is not None:
             if budget_bytes is None:
@@ -247,18 +270,16 @@ class Checkpointed:
         if self.layout is None and keep and invertible:
             plan = Plan(pk, _lib.BP_SWEEP_MAX, device)
             room = torch.cuda.mem_get_info(device)[0] // 4 if torch.cuda.is_available() else 0
-            uniform = SavedStates.of(pk.flags, plan.awin) is not None
-            if (uniform and 24 * pk.n * (plan.awin.shape[0] + 1) <= room
+            if (self.sweepable(plan) and 24 * pk.n * (plan.awin.shape[0] + 1) <= room
                     and 8 * pk.n * pk.sample_runs().n_runs <= min(engine.Z_BYTES, room)):
                 self.kept = torch.empty(plan.awin.shape[0] + 1, 6, pk.n, dtype=F32, device=device)
         if self.layout is None and self.kept is None:
             plan = Plan(pk, every, device)
         self.plan = plan
         self.saved = plan.saved
-        # whether every adjoint window is one run of RF or of free segments: then the gradients that need no
-        # per-segment sums but the RF waveform's take a window in one step (bp_cotangent, bp_sweep)
-        self.uniform = invertible and (plan.saved is not None or self.kept is not None
-                                       or SavedStates.of(pk.flags, plan.awin) is not None)
+        # whether every adjoint window is one run of RF or of free segments and can be integrated backward: then the
+        # gradients that need no per-segment sums but the RF waveform's take a window in one step (bp_cotangent, bp_sweep)
+        self.uniform = invertible and (plan.saved is not None or self.kept is not None or self.sweepable(plan))
         k = len(plan.starts)
         self.outer = outer if outer > 1 and k > outer and self.saved is None and self.kept is None else 0
         fws = _lib.forward_workspace(pk.n, pk.n_adc, pk.n_coils)
@@ -293,6 +314,11 @@ class Checkpointed:
         self.raw = sized(fws.raw, (max(pk.n_adc, 1), 2 * pk.n_coils), F64, device, zero=True)
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
         self._bufs = None
+
+    def sweepable(self, plan: "Plan") -> bool:
+        """Whether the sweep over runs can take ``plan``'s windows with per-spin gradients: each of RF or of free segments,
+        and the RF windows short next to the relaxation (their states are integrated backward from the window's end)."""
+        return SavedStates.of(self.pk.flags, plan.awin) is not None and rf_decay(self.pk, plan.awin)[0] <= MAX_DECAY
 
     def blocks(self):
         """[(first interval, end interval)] of the outer blocks (one block of every interval on two levels), or of

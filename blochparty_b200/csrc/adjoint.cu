@@ -40,6 +40,7 @@
 // !SG: the RF gradient of an interval of at most this many segments is summed over the CTA's tiles in shared memory
 // ([ADJ_SACC_MAX][2] floats) and written to gseg once, instead of added to gseg after every window
 #define ADJ_SACC_MAX 2048
+#define BP_MAX_DECAY 2.0f  // (blochparty_b200/adjoint.py MAX_DECAY, where the reason stands)
 // the sweep's own bits in a staged record's flags (above the record's): the segment before it (in the window)
 // spoils; the segment after it (in the window, swept just before) shares its RF relaxation, its RF off-resonance,
 // or its free factors, so the sweep keeps them
@@ -661,7 +662,10 @@ __global__ void __launch_bounds__(ADJ_THREADS, SG ? (NCG == 1 ? 4 : 3) : (NCG ==
                     const RevRelax rb = rev_relax(wrec[0].dt, p);
                     const float wzb = wz_of(wrec[0], win.x);
                     const bool from_chain = saved && chain_in_w;
-                    if (!(wrec[nseg - 1].flags & BP_SPOIL) && __all_sync(0xffffffffu, rb.invert) &&
+                    // rounding grows by exp(t r) on the way back over t: up to 7.4, else the states are recomputed (saved:
+                    // there is nothing to recompute them from; the caller sees to it that its pulses are short)
+                    const bool calm = saved || (float)nseg * wrec[0].dt * fmaxf(p.r1, p.r2) <= BP_MAX_DECAY;
+                    if (!(wrec[nseg - 1].flags & BP_SPOIL) && __all_sync(0xffffffffu, rb.invert && calm) &&
                         (from_chain || we != nullptr)) {
                         float ox = from_chain ? cx : mex, oy = from_chain ? cy : mey, oz = from_chain ? cz : mez;
                         for (int s = nseg - 1; s >= 0; --s) {

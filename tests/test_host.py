@@ -331,6 +331,32 @@ def test_saved_states_plan():
     assert sv2 is not None and sv2.final and sv2.n_slots == 2 and list(sv2.points) == [pulse_ends[0]]
 
 
+def test_backward_integration_is_bounded_by_the_decay():
+    """rf_decay: the longest RF window and the longest run of them, times the largest rate of any spin; what a sweep may
+    integrate backward is decided on it, not on one step."""
+    from types import SimpleNamespace
+
+    from blochparty_b200 import adjoint
+
+    b = sequences.SequenceBuilder()
+    for k in (10, 200, 40):
+        b.rf_waveform(np.ones((k, 2)), 10e-6).delay(1e-3)
+    seq = b.build()
+    rec, _, _, flags, _ = engine.pack_segments(seq.dt, seq.rf, seq.grad, None, seq.adc_phase, list(seq.is_rf), list(seq.adc),
+                                               list(seq.spoil), "cpu")
+    w = _lib.BP_ADJ_WIN
+    awin = engine.plan_windows(flags, w, seg_max=w, breaks=adjoint.run_breaks(flags))
+    spins = torch.zeros(8, 2)
+    spins[4], spins[5] = torch.tensor([1.0, 3.0]), torch.tensor([1000.0, 2000.0])
+    pk = SimpleNamespace(segs=rec, spins=spins, flags=flags, n=2)
+    window, run = adjoint.rf_decay(pk, awin)
+    assert abs(window - 32 * 10e-6 * 2000) < 1e-5 and abs(run - 200 * 10e-6 * 2000) < 1e-5
+    assert window <= adjoint.MAX_DECAY < run and adjoint.rf_relaxation_invertible(pk)  # (one step alone would let it pass)
+    spins[5, 0] = float("nan")
+    assert not adjoint.rf_decay(pk, awin)[0] <= adjoint.MAX_DECAY
+    assert adjoint.rf_decay(pk, awin[:0]) == (0.0, 0.0)
+
+
 def test_saved_entry_points_check_their_arguments():
     """bp_forward_saving and bp_adjoint_saved refuse a missing slot map, and the saved sweep refuses any gradient
     but the RF waveform's (argument checks only: no GPU call)."""

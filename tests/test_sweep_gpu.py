@@ -124,3 +124,25 @@ def test_against_the_segment_sweep(n, names, monkeypatch):
         want = _gradients(ph, seq, c, names)
         assert seen and not any(seen)
     _close(got, want, names)
+
+
+@pytest.mark.parametrize("t2", [10e-6, 20e-6, 50e-6, 100e-6, 150e-6, 200e-6, 1e-3])
+@pytest.mark.parametrize("names", [("rf",), ("t2", "db0", "b1"), ("t1", "rf")])
+@pytest.mark.parametrize("every", [None, 64])
+def test_short_t2(t2, names, every):
+    """Relaxation as fast as the pulses: integrating a state backward over a duration t multiplies its rounding errors
+    by exp(t / T2), so past t / T2 = 2 the states come forward from saved ones."""
+    n = 37
+    g = torch.Generator().manual_seed(7)
+    ph = _phantom(n, 4)
+    ph = replace(ph, t2=(t2 * (0.9 + 0.2 * torch.rand(n, generator=g, dtype=F64))).float().double())
+    b = sequences.SequenceBuilder()
+    r = np.random.RandomState(3)
+    for i in range(2):
+        b.rf_waveform((r.rand(200, 2) - 0.3) * 4000, 10e-6, grad=(300.0, 0.0, 1000.0))
+        b.readout(20, min(10e-6, 0.2 * t2), grad=(-2500.0, 300.0, 400.0), phase=0.3 * i)
+        b.delay(0.2e-3, grad=(2000.0, 0.0, 0.0))
+    seq, c = b.build(), _coils(n, 4)
+    got = _gradients(ph, seq, c, names, every=every)
+    _, want = bloch.gradients(bloch.case_from(ph, seq, c), _loss, names)
+    _close(got, want, names)
