@@ -125,7 +125,7 @@ def test_divided_forward(n, room, monkeypatch):
 def test_states_saved_over_many_chunks(n):
     """A state saved at every window of a sequence of many chunks (one warp with helpers, one warp, four warps per
     CTA; no barrier between a chunk's steps in the last two), again and again: each the state a division passes on."""
-    ph, seq = _phantom(n, 5), _sequence((64, 95) * 6, 6)
+    ph, seq = _phantom(n, 5), _sequence((64, 95) * 8, 6)
     pk, _, _, state0 = _packed(ph, seq, bpb.birdcage_sensitivities(ph.pos, 1))
     win = engine.plan_windows(pk.flags, 32, seg_max=32)
     wdev, W = torch.from_numpy(win).to(pk.device), win.shape[0]
