@@ -233,6 +233,23 @@ class Plan:
         self.max_len = max(b - a for a, b in self.seg_ranges)
 
 
+def sweep_pieces(awin: np.ndarray, wa: int, wb: int, run_starts: np.ndarray, room: int):
+    """[(first window, end window, first segment, end segment)]: windows [wa, wb) of ``awin`` in pieces that one sweep
+    takes, of at most ``BP_SWEEP_MAX`` segments and with at most ``room`` runs of samples starting in them (or one
+    window)."""
+    start, end, out = awin[:, 0], awin[:, 1], []
+    while wa < wb:
+        s0 = int(start[wa])
+        b = int(np.searchsorted(end, s0 + _lib.BP_SWEEP_MAX, "right"))
+        r = int(np.searchsorted(run_starts, s0)) + room
+        if r < len(run_starts):
+            b = min(b, int(np.searchsorted(end, run_starts[r], "right")))
+        b = min(max(b, wa + 1), wb)
+        out.append((wa, b, s0, int(end[b - 1])))
+        wa = b
+    return out
+
+
 class Checkpointed:
     """The device side of a simulation with gradients on a packed case: the forward that stores the state at every
     interval start, and the backward (per interval in reverse: replay, reverse sweep, segment-gradient reduction);
@@ -289,6 +306,10 @@ class Checkpointed:
         self.ws = _lib.adjoint_workspace(pk.n, pk.flags.shape[0], pk.n_adc, pk.n_coils, plan.every, plan.max_aw,
                                          self.grid, self.outer)
         self.z = None  # kept: the first samples of the forward's runs
+        self.pieces = None  # uniform: every interval in pieces for the sweep, the runs' sums of one under Z_BYTES
+        if self.uniform:
+            room, starts = max(engine.Z_BYTES // (8 * max(pk.n, 1)), 1), pk.sample_runs().starts
+            self.pieces = [sweep_pieces(plan.awin, aa, ab, starts, room) for aa, ab in plan.aranges]
         if self.kept is not None:
             pass
         elif self.saved is None:
@@ -385,15 +406,16 @@ class Checkpointed:
     def sweeps(self, seg_mask: int, need_seg: bool) -> bool:
         """Whether the backward runs ``bp_cotangent`` and ``bp_sweep`` (else ``bp_adjoint``)."""
         offsets = need_seg and seg_mask & _lib.BP_SEG_ALL & ~(_lib.BP_SEG_WX | _lib.BP_SEG_WY)
-        return self.uniform and not offsets and (not need_seg or self.plan.max_len <= _lib.BP_SWEEP_MAX)
+        return self.uniform and not offsets
 
     def sweep_buffers(self, h, spin_gradients: bool, want_gc: bool, need_seg: bool):
-        """The sweep's workspace: the cotangents split for the tensor cores, the runs' sums of one interval, the first
+        """The sweep's workspace: the cotangents split for the tensor cores, the runs' sums of one piece, the first
         samples of its runs (with coil gradients) and the per-CTA RF gradient."""
-        pk, plan, b = self.pk, self.plan, {}
+        pk, b = self.pk, {}
         runs = pk.sample_runs()
+        ranges = [p[2:] for pieces in self.pieces for p in pieces]
         if h is not None and runs.n_runs:
-            at = np.searchsorted(runs.starts, np.asarray(plan.seg_ranges, dtype=np.int64))
+            at = np.searchsorted(runs.starts, np.asarray(ranges, dtype=np.int64))
             cap = max(int((at[:, 1] - at[:, 0]).max()), 1)
             pair = lambda: torch.empty(cap, pk.n, 2, dtype=F32, device=self.dev)
             b["hs"] = torch.empty(pk.n_adc, 8 * ((pk.n_coils + 7) // 8), dtype=torch.int64, device=self.dev)
@@ -407,17 +429,16 @@ class Checkpointed:
         b["gseg"] = None
         if need_seg:
             rows = max(_lib.lib().bp_sweep_grid(pk.n, b1 - b0, int(spin_gradients))
-                       for b0, b1 in {(0, e - s) for s, e in plan.seg_ranges})
+                       for b0, b1 in {(0, e - s) for s, e in ranges})
             if rows < 1:
                 raise RuntimeError("bp_sweep_grid failed")
-            b["gseg"] = torch.empty(rows, plan.max_len, 2, dtype=F32, device=self.dev)
+            b["gseg"] = torch.empty(rows, max(e - s for s, e in ranges), 2, dtype=F32, device=self.dev)
         return b
 
-    def _sweep(self, k, b, states, wslot, chain, chain_in, lam, gs, gc, seg, z=None):
-        """Interval k's samples (``z``: its runs' first samples, with coil gradients) and its sweep from ``states``."""
+    def _sweep(self, piece, b, states, wslot, chain, chain_in, lam, gs, gc, seg, z=None):
+        """A piece's samples (``z``: its runs' first samples, with coil gradients) and its sweep from ``states``."""
         pk, plan, lib, stream = self.pk, self.plan, _lib.lib(), _lib.stream_ptr()
-        aa, ab = plan.aranges[k]
-        s0, s1 = plan.seg_ranges[k]
+        aa, ab, s0, s1 = piece
         runs = pk.sample_runs()
         g0 = b.get("g0")
         if g0 is not None:
@@ -493,22 +514,32 @@ class Checkpointed:
         aa, ab = plan.aranges[k]
         s0, s1 = plan.seg_ranges[k]
         if self.kept is not None:  # every state is there
-            z = None if self.z is None else self.z[int(np.searchsorted(pk.sample_runs().starts, s0)):]
-            self._sweep(k, swept, self.kept[aa:], None, None, 0, lam, gs, gc, seg, z)
+            for p in reversed(self.pieces[k]):
+                z = None if self.z is None else self.z[int(np.searchsorted(pk.sample_runs().starts, p[2])):]
+                self._sweep(p, swept, self.kept[p[0]:], None, None, 0, lam, gs, gc, seg, z)
             return
         state.copy_(self.ckpts[ck])
         z = None if swept is None else swept.get("z")
-        if z is None:
-            self._fwd(state, plan.awin_dev, aa, ab, None, wstates=wstates)
-        else:  # with the first samples of the interval's runs
+
+        def first_samples(wa, wb, ws):  # windows [wa, wb) stepped from `state`, with the first samples of their runs
             runs = pk.sample_runs()
-            code = lib.bp_propagate(ptr(pk.spins), n, ptr(pk.segs), ptr(pk.seg64), ptr(plan.awin_dev), aa, ab, ptr(state),
-                                    ptr(wstates), 1, None, ptr(runs.runs), runs.n_runs, ptr(z), swept["cap"], 0, 0,
+            code = lib.bp_propagate(ptr(pk.spins), n, ptr(pk.segs), ptr(pk.seg64), ptr(plan.awin_dev), wa, wb, ptr(state),
+                                    ptr(ws), 1, None, ptr(runs.runs), runs.n_runs, ptr(z), swept["cap"], 0, 0,
                                     ptr(self.status), stream)
             _lib.check(code, "bp_propagate")
+
+        pieces = None if swept is None else self.pieces[k]
+        if z is not None and len(pieces) == 1:
+            first_samples(aa, ab, wstates)
+        else:
+            self._fwd(state, plan.awin_dev, aa, ab, None, wstates=wstates)
         wstates[ab - aa].copy_(state)  # the state after the interval's last window
         if swept is not None:
-            self._sweep(k, swept, wstates, None, None, 0, lam, gs, gc, seg, z)
+            for p in reversed(pieces):
+                if z is not None and len(pieces) > 1:  # (z holds one piece's)
+                    state.copy_(wstates[p[0] - aa])
+                    first_samples(p[0], p[1], None)
+                self._sweep(p, swept, wstates[p[0] - aa:], None, None, 0, lam, gs, gc, seg, z)
             return
         if self.phys is None:
             code = lib.bp_adjoint(ptr(pk.spins), ptr(pk.sens), n, C, ptr(pk.segs), ptr(pk.seg64), ptr(plan.awin_dev),
@@ -542,10 +573,12 @@ class Checkpointed:
             for k in reversed(range(ka, kb)):
                 aa, ab = plan.aranges[k]
                 s0, s1 = plan.seg_ranges[k]
-                chain_in = int(ab < W and bool(sv.rf[ab]))
                 if swept is not None:
-                    self._sweep(k, swept, self.slots, self.aslot_dev, chain, chain_in, lam, None, None, seg)
+                    for p in reversed(self.pieces[k]):
+                        self._sweep(p, swept, self.slots, self.aslot_dev, chain, int(p[1] < W and bool(sv.rf[p[1]])), lam,
+                                    None, None, seg)
                     continue
+                chain_in = int(ab < W and bool(sv.rf[ab]))
                 code = lib.bp_adjoint_saved(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs),
                                             ptr(pk.seg64), ptr(plan.awin_dev), aa, ab, s0, s1 - s0, ptr(self.slots),
                                             ptr(self.aslot_dev), ptr(chain), chain_in, ptr(h), pk.n_adc, ptr(lam),
@@ -560,7 +593,8 @@ class Checkpointed:
         k, plan = len(self.plan.starts), self.plan
         readout = int(self.pk.n_adc > 0)
         run = lambda windows: engine.forward_launches(self.pk, windows) if readout else 1
-        swept = 2 * readout + k * (1 + readout + int(need_seg))  # the split, then per interval samples, sweep, sums
+        n_pieces = sum(map(len, self.pieces)) if self.uniform else 0
+        swept = 2 * readout + n_pieces * (1 + readout + int(need_seg))  # the split, then per piece samples, sweep, sums
         if self.saved is not None:
             blocks = self.blocks()
             forward = sum(run(plan.franges[kb - 1][1] - plan.franges[ka][0]) for ka, kb in blocks)

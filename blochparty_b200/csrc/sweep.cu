@@ -703,7 +703,7 @@ extern "C" int bp_sweep(const float* spins, int n, const void* segs, const doubl
                         int wb, int seg0, int seg_len, const float* wstates, const int* wslot, float* chain,
                         int chain_in, const int* runs, int n_runs, const float* g0, const float* g1, float* lam,
                         float* gs, float* gseg, double* seg, int* status, void* stream) {
-    if (n < 1 || wa < 0 || wb < wa || seg0 < 0 || seg_len < 0 || seg_len > SW_MAX || n_runs < 0) return BP_E_ARG;
+    if (n < 1 || wa < 0 || wb < wa || seg0 < 0 || seg_len < 0 || (gseg && seg_len > SW_MAX) || n_runs < 0) return BP_E_ARG;
     if (!spins || !segs || !seg64 || !windows || !wstates || !lam || !status || (g0 && !runs) || (gseg && !seg))
         return BP_E_ARG;
     if ((gs != nullptr) == (wslot != nullptr) || (wslot && !chain) || (gs && g0 && !g1)) return BP_E_ARG;
@@ -717,7 +717,7 @@ extern "C" int bp_sweep(const float* spins, int n, const void* segs, const doubl
     a.runs = reinterpret_cast<const int4*>(runs), a.n_runs = n_runs;
     a.g0 = reinterpret_cast<const float2*>(g0), a.g1 = reinterpret_cast<const float2*>(g1);
     a.lam = lam, a.gs = gs, a.gseg = gseg, a.status = status;
-    const int grid = bp_sweep_grid(n, seg_len, gs != nullptr);
+    const int grid = bp_sweep_grid(n, gseg ? seg_len : 0, gs != nullptr);
     if (grid < 1) return BP_E_LAUNCH;
     const size_t smem = gseg ? (size_t)2 * seg_len * sizeof(float) : 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);

@@ -331,6 +331,37 @@ def test_saved_states_plan():
     assert sv2 is not None and sv2.final and sv2.n_slots == 2 and list(sv2.points) == [pulse_ends[0]]
 
 
+@pytest.mark.parametrize("room", [1, 3, 1000])
+def test_sweep_pieces(room):
+    """An interval's windows in pieces for the sweep: all of them once and in order, each piece of at most BP_SWEEP_MAX
+    segments and ``room`` runs, or of a single window, and none cut earlier than it has to be."""
+    from blochparty_b200 import adjoint
+
+    g = np.random.default_rng(room)
+    b = sequences.SequenceBuilder()
+    for i in range(60):
+        b.rf(20e-6, flip_deg=10.0).readout(int(g.integers(1, 150)), 10e-6, grad=(1e3 * i, 0.0, 0.0)).delay(1e-3)
+        if i % 20 == 7:  # many runs in one window
+            for _ in range(6):
+                b.readout(2, 10e-6).delay(1e-5, grad=(5.0 * i, 0.0, 0.0))
+    seq = b.build()
+    flags = engine.pack_segments(seq.dt, seq.rf, seq.grad, None, seq.adc_phase, list(seq.is_rf), list(seq.adc),
+                                 list(seq.spoil), "cpu")[3]
+    w = _lib.BP_ADJ_WIN
+    awin = engine.plan_windows(flags, w, seg_max=w, breaks=adjoint.run_breaks(flags))
+    starts = engine.sample_runs(flags)[0][:, 0]
+    count = lambda p: int(((starts >= p[2]) & (starts < p[3])).sum())
+    for wa, wb in ((0, awin.shape[0]), (5, awin.shape[0] - 3), (4, 4)):
+        pieces = adjoint.sweep_pieces(awin, wa, wb, starts, room)
+        assert [p[0] for p in pieces] + [wb] == [wa] + [p[1] for p in pieces]
+        for i, p in enumerate(pieces):
+            assert p[2] == awin[p[0], 0] and p[3] == awin[p[1] - 1, 1]
+            assert p[1] == p[0] + 1 or (p[3] - p[2] <= _lib.BP_SWEEP_MAX and count(p) <= room)
+            if i + 1 < len(pieces):
+                more = (p[0], p[1] + 1, p[2], awin[p[1], 1])
+                assert more[3] - more[2] > _lib.BP_SWEEP_MAX or count(more) > room
+
+
 def test_backward_integration_is_bounded_by_the_decay():
     """rf_decay: the longest RF window and the longest run of them, times the largest rate of any spin; what a sweep may
     integrate backward is decided on it, not on one step."""

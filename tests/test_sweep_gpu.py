@@ -9,7 +9,7 @@ import pytest
 import torch
 
 import blochparty_b200 as bpb
-from blochparty_b200 import adjoint, sequences
+from blochparty_b200 import adjoint, engine, sequences
 from oracle import bloch
 
 pytestmark = pytest.mark.gpu
@@ -146,3 +146,24 @@ def test_short_t2(t2, names, every):
     got = _gradients(ph, seq, c, names, every=every)
     _, want = bloch.gradients(bloch.case_from(ph, seq, c), _loss, names)
     _close(got, want, names)
+
+
+@pytest.mark.parametrize("names", [("t1", "t2", "coils"), ("pos", "rf"), ("rf",)])
+def test_long_intervals(names, monkeypatch):
+    """An interval of more segments than one sweep takes, and one with more runs of samples than the sums' workspace
+    holds: swept in pieces, the same bits as with short intervals and with every state kept."""
+    n = 50
+    ph, seq, c = _phantom(n, 6), _sequence((95, 64, 130, 33) * 5, rf_steps=20), _coils(n, 9)
+    assert len(seq) > 2048 + 64
+    seen = _spy(monkeypatch)
+    want = _gradients(ph, seq, c, names, every=64)
+    for every, room in ((3200, None), (3200, 3), (320, 1), (None, None), (None, 2)):
+        with monkeypatch.context() as m:
+            if room:
+                m.setattr(engine, "Z_BYTES", 8 * n * room)
+            got = _gradients(ph, seq, c, names, every=every)
+        for k in names:
+            assert torch.equal(got[k], want[k]), (every, room, k)
+    assert seen and all(seen)
+    _, exact = bloch.gradients(bloch.case_from(ph, seq, c), _loss, names)
+    _close(want, exact, names)
