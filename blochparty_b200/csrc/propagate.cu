@@ -465,27 +465,24 @@ __global__ void __launch_bounds__(RO_THREADS, 3) bp_readout_kernel(ReadArgs a) {
     fetch(g0);
     for (int grp = g0; grp < g_end; grp += RO_WARPS) {
         asm volatile("cp.async.wait_all;" ::: "memory");
-        float sens_inv;
+        float sens_inv[2];  // of this lane's two coils
         PropSpin p{};
         float2 zin[RO_SUBS];
         {
             float v[16];
-            uint32_t mag = 0u;
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                v[c] = in[c * 32 + lane];
-                const uint32_t u = __float_as_uint(fabsf(v[c]));
-                mag = max(mag, u < 0x7f800000u ? u : 0u);
-            }
+            for (int c = 0; c < 16; ++c) v[c] = in[c * 32 + lane];
             p.x = (double)in[16 * 32 + lane], p.y = (double)in[17 * 32 + lane], p.z = (double)in[18 * 32 + lane];
             p.r2 = in[19 * 32 + lane], p.db0 = (double)in[20 * 32 + lane];
 #pragma unroll
             for (int b = 0; b < RO_SUBS; ++b) zin[b] = in_z[b * 32 + lane];
             fetch(grp + RO_WARPS);
-            float scale;
-            warp_scale(mag, scale, sens_inv);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
+            for (int c = 0; c < 8; ++c) {  // every coil by its own scale
+                const uint32_t u = __float_as_uint(fabsf(v[2 * c])), w = __float_as_uint(fabsf(v[2 * c + 1]));
+                float scale, inverse;
+                warp_scale(max(u < 0x7f800000u ? u : 0u, w < 0x7f800000u ? w : 0u), scale, inverse);
+                if (t == (c >> 1)) sens_inv[c & 1] = inverse;
                 sens[sens_slot(lane, c)] = split_sens(v[2 * c] * scale, v[2 * c + 1] * scale);
             }
         }
@@ -499,11 +496,13 @@ __global__ void __launch_bounds__(RO_THREADS, 3) bp_readout_kernel(ReadArgs a) {
                 const FreeFactors f = prop_factors(a.segs[ratio[b]].dt, a.seg64[ratio[b]], p, 1);
                 float2 q8;
                 factor_powers(f, q8, q32);
-                float zr = 1.0f, zi = 0.0f;
+                double x, y, zr = 1.0, zi = 0.0;  // (float64: one rounding, and no slower than a float32 recurrence)
+                factor64(f, x, y);
 #pragma unroll
                 for (int i = 0; i < RO_ROWS; ++i) {
-                    tab[i * RO_TAB_ROW + pw] = zr, tab[i * RO_TAB_ROW + pw + 2] = zi;
-                    if (i + 1 < RO_ROWS) readout_advance(f, zr, zi);
+                    tab[i * RO_TAB_ROW + pw] = (float)zr, tab[i * RO_TAB_ROW + pw + 2] = (float)zi;
+                    const double nr = fma(x, zr, -y * zi);
+                    zi = fma(x, zi, y * zr), zr = nr;
                 }
                 step8[pw] = q8.x, step8[pw + 2] = q8.y;
                 reinterpret_cast<float*>(nstep)[(pw >> 2) * 2 + (pw & 1)] = -q8.y;
@@ -542,8 +541,8 @@ __global__ void __launch_bounds__(RO_THREADS, 3) bp_readout_kernel(ReadArgs a) {
             for (int h = 0; h < 2; ++h)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    acc[b][h][0][i] = fmaf(dr[h][i] * inverse, sens_inv, acc[b][h][0][i]);
-                    acc[b][h][1][i] = fmaf(di[h][i] * inverse, sens_inv, acc[b][h][1][i]);
+                    acc[b][h][0][i] = fmaf(dr[h][i] * inverse, sens_inv[i & 1], acc[b][h][0][i]);
+                    acc[b][h][1][i] = fmaf(di[h][i] * inverse, sens_inv[i & 1], acc[b][h][1][i]);
                 }
         }
         __syncwarp();  // (a group whose blocks were all skipped)
@@ -569,7 +568,7 @@ __global__ void __launch_bounds__(RO_THREADS, 3) bp_readout_kernel(ReadArgs a) {
         float s = 0.0f;  // the warps in fixed order: the CTA's sum does not depend on timing
 #pragma unroll
         for (int w = 0; w < RO_WARPS; ++w) s += reinterpret_cast<const float*>(sm[w])[k];
-        atomicAdd(a.raw + (size_t)(sub[b].w + (row & 31)) * nv + 2 * coil + im, (double)s);
+        atomicAdd(a.raw + (size_t)(sub[b].w + (row & 31)) * nv + 2 * coil + im, (double)s * RO_CUT);
     }
 }
 

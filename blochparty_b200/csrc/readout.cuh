@@ -3,9 +3,14 @@
 // A run is up to 128 samples of which sample p (from 0) of spin j is z_j q_j^p: z_j the spin's first sample (written by
 // the propagation), q_j the complex factor of the segment that separates the samples. Coil c's sum is sum_j z_j q_j^p
 // s_jc, a matrix product over the spins: [samples][2 x spins] x [2 x spins][16]. Both operands are scaled by a power
-// of two (32 spins' largest value to 2^12) and split into two half-precision values (11 + 11 bits: x = hi + lo to 2^-23
-// of x down to 2^-14 of the largest), and hi hi + hi lo + lo hi accumulate in float32 (mma.sync.m16n8k16; the dropped
-// lo lo is 2^-24) over 32 spins, then by rounded float32 adds over the warp's spins. Measured, mma.sync issues
+// of two (32 spins' largest value to 2^12; every coil by its own) and split into two half-precision values (11 + 11 bits:
+// x = hi + lo to 2^-23 of x down to 2^-14 of the largest), and hi hi + hi lo + lo hi accumulate in float32
+// (mma.sync.m16n8k16; the dropped lo lo is 2^-24) over 8 spins, then by rounded float32 adds over the warp's spins: the
+// tensor cores cut a sum's bits off towards zero (Fasi, Higham, Mikaitis and Pranesh, "Numerical behavior of NVIDIA tensor
+// cores", 2021), and with 32 spins in one accumulator all signals came out 1.8e-7 too small; now 5e-8, which RO_CUT makes
+// up for. Relative error of the signal against float64 (float32 products and sums; 32 spins; 8 spins and RO_CUT):
+// 256 spins 2.1e-7, 2.7e-7, 1.6e-7; 9,025 spins 2.5e-7, 3.0e-7, 2.0e-7; 524,288 spins x 2 TRs of four echoes 3.4e-8,
+// 2.2e-7, 3.6e-8. The readout of 1,048,576 spins x 512 samples x 8 coils went from 0.658 to 0.673 ms. Measured, mma.sync issues
 // every 8 cycles per SM quarter for half and tf32 alike, and half holds twice the spins: 1.5 instructions per sample
 // of 32 spins at 8 coils, 12 cycles, beside about 14 other issue slots; the float32 sum on the FMA pipe took 32
 // multiply-adds and 14 other slots.
@@ -18,6 +23,9 @@
 
 #include "bloch_common.cuh"
 
+// One cut costs half a unit in the last place of a float32 on average: 2^-24 / m of a sum with significand m in [1, 2),
+// 2^-24 / (2 ln 2) over the usual distribution of significands.
+#define RO_CUT (1.0 + 0.7213 / 16777216.0)
 #define RO_ROWS 8          // rows of the sample table (a fragment's rows)
 // Shared memory of a warp's 32 spins, laid out so that a lane's two spins of every eight (8 g + t and 8 g + 4 + t) come
 // as the operands of paired instructions, without moves: a pair is 16 bytes, (re, re', im, im'), and the rows of the
@@ -93,10 +101,16 @@ __device__ __forceinline__ CPair cmul2(const CPair& a, const CPair& b, const flo
     return CPair{__ffma2_rn(a.re, b.re, __fmul2_rn(a.im, nim)), __ffma2_rn(a.re, b.im, __fmul2_rn(a.im, b.re))};
 }
 
-// q^8 and q^32 of the factor q = (1 + e2)(c + i s), in float64 and rounded once.
-__device__ __forceinline__ void factor_powers(const FreeFactors& f, float2& q8, float2& q32) {
+// The factor q = (1 + e2)(c + i s) in float64.
+__device__ __forceinline__ void factor64(const FreeFactors& f, double& x, double& y) {
     const double a = 1.0 + (double)f.e2;
-    double x = a * ((double)f.ch + (double)f.cl), y = a * ((double)f.sh + (double)f.sl);
+    x = a * ((double)f.ch + (double)f.cl), y = a * ((double)f.sh + (double)f.sl);
+}
+
+// q^8 and q^32, in float64 and rounded once.
+__device__ __forceinline__ void factor_powers(const FreeFactors& f, float2& q8, float2& q32) {
+    double x, y;
+    factor64(f, x, y);
 #pragma unroll
     for (int i = 0; i < 5; ++i) {
         const double t = fma(x, x, -y * y);
@@ -107,6 +121,15 @@ __device__ __forceinline__ void factor_powers(const FreeFactors& f, float2& q8, 
     q32 = make_float2((float)x, (float)y);
 }
 
+// a += b on paired instructions, rounded to nearest.
+__device__ __forceinline__ void add4(float* a, const float* b) {
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+        const float2 s = __fadd2_rn(make_float2(a[i], a[i + 1]), make_float2(b[i], b[i + 1]));
+        a[i] = s.x, a[i + 1] = s.y;
+    }
+}
+
 // Two fragment rows' samples (z: this lane's row, zb: the row 8 below; two spins) times the spins' sensitivities s0 and
 // s1, added to dr (real parts) and di (imaginary parts).
 __device__ __forceinline__ void readout_mma(const CPair& z, const CPair& zb, const uint4& s0, const uint4& s1, float* dr,
@@ -114,10 +137,13 @@ __device__ __forceinline__ void readout_mma(const CPair& z, const CPair& zb, con
     uint32_t h[2], l[2], hb[2], lb[2];
     split_half2(z.re, z.im, h, l);
     split_half2(zb.re, zb.im, hb, lb);
-    mma_half(dr, l[0], lb[0], l[1], lb[1], s0.x, s1.x);  // the small terms first
-    mma_half(di, l[0], lb[0], l[1], lb[1], s0.z, s1.z);
-    mma_half(dr, h[0], hb[0], h[1], hb[1], s0.y, s1.y);
-    mma_half(di, h[0], hb[0], h[1], hb[1], s0.w, s1.w);
-    mma_half(dr, h[0], hb[0], h[1], hb[1], s0.x, s1.x);
-    mma_half(di, h[0], hb[0], h[1], hb[1], s0.z, s1.z);
+    float tr[4] = {0.0f, 0.0f, 0.0f, 0.0f}, ti[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    mma_half(tr, l[0], lb[0], l[1], lb[1], s0.x, s1.x);  // the small terms first
+    mma_half(ti, l[0], lb[0], l[1], lb[1], s0.z, s1.z);
+    mma_half(tr, h[0], hb[0], h[1], hb[1], s0.y, s1.y);
+    mma_half(ti, h[0], hb[0], h[1], hb[1], s0.w, s1.w);
+    mma_half(tr, h[0], hb[0], h[1], hb[1], s0.x, s1.x);
+    mma_half(ti, h[0], hb[0], h[1], hb[1], s0.z, s1.z);
+    add4(dr, tr);
+    add4(di, ti);
 }

@@ -71,6 +71,36 @@ def test_against_the_oracle(n, coils, lengths):
         assert err < 1e-5, (i, err)
 
 
+@pytest.mark.parametrize("n,coils", [(256, 4), (4096, 8), (40000, 13)])
+def test_signal_to_float32_rounding(n, coils):
+    """One pulse and one readout, so that the state's own error is small: the coil sums are as good as float32 ones with
+    rounded operations, without a bias (the bound: 2^-23, a rounding of each factor; sums with truncated operations are
+    2e-7 off whatever the size)."""
+    ph = _phantom(n, 8)
+    b = sequences.SequenceBuilder().rf(20e-6, flip_deg=35.0).delay(0.3e-3, grad=(2000.0, 500.0, 0.0))
+    seq = b.readout(95, 10e-6, grad=(-2500.0, 300.0, 400.0)).build()
+    c = bpb.birdcage_sensitivities(ph.pos, coils).to(torch.complex64).to(torch.complex128)
+    sig, _ = bloch.simulate(bloch.case_from(ph, seq, c))
+    r = bpb.simulate(ph, seq, c).signal.to(sig.dtype)
+    err, bias = float((r - sig).norm() / sig.norm()), complex(((r - sig) * sig.conj()).sum()) / float(sig.norm()) ** 2
+    assert err < 2.0 ** -23 and abs(bias) < 2.0 ** -24, (err, bias)
+
+
+def test_coils_of_far_apart_sensitivities():
+    """A coil 10^10 below the others of its group keeps its precision (the plain float32 bar, as above: random
+    sensitivities cancel, so that a signal is a small part of the sum of its terms' sizes)."""
+    n = 700
+    ph, seq, g = _phantom(n, 9), _sequence((33, 64), 9, rf_adc=False), torch.Generator().manual_seed(3)
+    rnd = lambda: torch.rand(n, 9, generator=g, dtype=F64).float().double() - 0.5
+    scale = torch.tensor([1.0, 1e-10, 1e3, 1e-7, 1.0, 1e7, 1e-12, 1.0, 1e-5], dtype=F64)
+    c = (torch.complex(rnd(), rnd()) * scale).to(torch.complex64).to(torch.complex128)
+    sig, _ = bloch.simulate(bloch.case_from(ph, seq, c))
+    r = bpb.simulate(ph, seq, c).signal.to(sig.dtype)
+    for i in range(9):
+        err = float((r[i] - sig[i]).norm() / sig[i].norm())
+        assert err < 1e-5, (i, err)
+
+
 def _packed(ph, seq, coils):
     dev = torch.device("cuda", 0)
     inp = Inputs(ph.pos, ph.pd, ph.t1, ph.t2, ph.db0, ph.b1, coils, seq.dt, seq.rf, seq.grad, seq.adc_phase, None,
