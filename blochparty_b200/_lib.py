@@ -122,7 +122,7 @@ SIGNATURES = {
     "bp_forward_saving": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, _P, _P, _P, _P, c_int, _P, _P]),
     "bp_adjoint_physics": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, c_int, _P,
                                    _P, _P, _P, c_int, c_int, _P, _P, _P, _P]),
-    "bp_cotangent_split": (c_int, [_P, c_int, c_int, _P, _P, _P]),
+    "bp_cotangent_split": (c_int, [_P, c_int, c_int, _P, c_int, _P, c_int, _P, _P, _P]),
     "bp_cotangent": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, _P, c_int, _P, _P, _P, _P, _P, _P, _P]),
     "bp_sweep_grid": (c_int, [c_int, c_int, c_int]),
     "bp_sweep": (c_int, [_P, c_int, _P, _P, _P, c_int, c_int, c_int, c_int, _P, _P, _P, c_int, _P, c_int, _P, _P, _P, _P,

@@ -418,13 +418,14 @@ class Checkpointed:
             at = np.searchsorted(runs.starts, np.asarray(ranges, dtype=np.int64))
             cap = max(int((at[:, 1] - at[:, 0]).max()), 1)
             pair = lambda: torch.empty(cap, pk.n, 2, dtype=F32, device=self.dev)
-            b["hs"] = torch.empty(pk.n_adc, 8 * ((pk.n_coils + 7) // 8), dtype=torch.int64, device=self.dev)
-            b["most"] = torch.empty(1, dtype=torch.int32, device=self.dev)
+            width = 8 * ((pk.n_coils + 7) // 8)
+            b["hs"] = torch.empty(pk.n_adc, width, dtype=torch.int64, device=self.dev)
+            b["inverse"] = torch.empty(pk.n_adc, width, dtype=F32, device=self.dev)
             b["g0"], b["cap"] = pair(), cap
             b["g1"] = pair() if spin_gradients else None
             b["z"] = pair() if want_gc and self.kept is None else None
-            code = _lib.lib().bp_cotangent_split(ptr(h), pk.n_adc, pk.n_coils, ptr(b["hs"]), ptr(b["most"]),
-                                                 _lib.stream_ptr())
+            code = _lib.lib().bp_cotangent_split(ptr(h), pk.n_adc, pk.n_coils, ptr(runs.runs), runs.n_runs, ptr(runs.subs),
+                                                 runs.n_subs, ptr(b["hs"]), ptr(b["inverse"]), _lib.stream_ptr())
             _lib.check(code, "bp_cotangent_split")
         b["gseg"] = None
         if need_seg:
@@ -444,7 +445,7 @@ class Checkpointed:
         if g0 is not None:
             code = lib.bp_cotangent(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64),
                                     ptr(plan.awin_dev), aa, ab, ptr(runs.runs), runs.n_runs, ptr(b["hs"]),
-                                    ptr(b["most"]), ptr(g0), ptr(b["g1"]), ptr(z), ptr(gc), stream)
+                                    ptr(b["inverse"]), ptr(g0), ptr(b["g1"]), ptr(z), ptr(gc), stream)
             _lib.check(code, "bp_cotangent")
         code = lib.bp_sweep(ptr(pk.spins), pk.n, ptr(pk.segs), ptr(pk.seg64), ptr(plan.awin_dev), aa, ab, s0, s1 - s0,
                             ptr(states), ptr(wslot), ptr(chain), chain_in, ptr(runs.runs), runs.n_runs, ptr(g0),
@@ -594,7 +595,7 @@ class Checkpointed:
         readout = int(self.pk.n_adc > 0)
         run = lambda windows: engine.forward_launches(self.pk, windows) if readout else 1
         n_pieces = sum(map(len, self.pieces)) if self.uniform else 0
-        swept = 2 * readout + n_pieces * (1 + readout + int(need_seg))  # the split, then per piece samples, sweep, sums
+        swept = readout + n_pieces * (1 + readout + int(need_seg))  # the split, then per piece samples, sweep, sums
         if self.saved is not None:
             blocks = self.blocks()
             forward = sum(run(plan.franges[kb - 1][1] - plan.franges[ka][0]) for ka, kb in blocks)

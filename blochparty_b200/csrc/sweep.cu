@@ -23,45 +23,36 @@
 
 // ---- the samples' part ----
 
-// 2^k that takes the largest finite magnitude of h (its bits in *most) to [2^12, 2^13), and its inverse.
-__device__ __forceinline__ void h_scale(const uint32_t* most, float& scale, float& inverse) {
-    const uint32_t m = *most, e = min(max(m >> 23, 13u), 253u);
-    scale = __uint_as_float((m == 0u ? 127u : 266u - e) << 23);
-    inverse = __uint_as_float((m == 0u ? 127u : e - 12u) << 23);
-}
-
-__global__ void bp_h_most_kernel(const float* __restrict__ h, int64_t n, uint32_t* most) {
-    uint32_t m = 0u;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t u = __float_as_uint(fabsf(h[i]));
-        m = max(m, u < 0x7f800000u ? u : 0u);
+// A block is up to 32 samples of one run (subs: run, block). hs [rows][8 ncg]: the halves of (h0, -h1) of every row and
+// coil, scaled by a power of two that takes the largest finite magnitude of the block and coil to 2^12; zero coils to pad;
+// inverse [rows][8 ncg]: the scales' inverses, in the row of a block's first sample. (One scale for the whole sequence lost
+// the gradients of late pulses where a loss weighs early samples 10^9 above late ones. With the turned halves too, as the
+// readout's, bp_cotangent read twice the bytes: 0.83 -> 0.89 ms at 1,048,576 spins x 512 samples.)
+#define HS_THREADS 256
+__global__ void __launch_bounds__(HS_THREADS) bp_h_split_kernel(const float* __restrict__ h, int n_coils, int width,
+                                                                const int4* __restrict__ runs,
+                                                                const int2* __restrict__ subs, uint2* __restrict__ hs,
+                                                                float* __restrict__ inverse) {
+    const int lane = threadIdx.x & 31;
+    const int2 sub = subs[blockIdx.x];
+    const int4 run = runs[sub.x];
+    const int64_t row0 = run.w + 32 * sub.y, row = row0 + lane;
+    const bool there = lane < run.z - 32 * sub.y;
+    for (int c = threadIdx.x >> 5; c < width; c += HS_THREADS / 32) {  // a warp per coil, a lane per sample
+        float re = 0.0f, im = 0.0f, scale, inv;
+        if (there && c < n_coils) re = h[row * 2 * n_coils + 2 * c], im = h[row * 2 * n_coils + 2 * c + 1];
+        const uint32_t u = __float_as_uint(fabsf(re)), v = __float_as_uint(fabsf(im));
+        warp_scale(max(u < 0x7f800000u ? u : 0u, v < 0x7f800000u ? v : 0u), scale, inv);
+        const uint4 s = split_sens(re * scale, im * scale);
+        if (there) hs[row * width + c] = make_uint2(s.x, s.y);
+        if (lane == 0) inverse[row0 * width + c] = inv;
     }
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(most, m);
-}
-
-// hs [rows][8 ncg]: the halves of (h0, -h1) of every row and coil, scaled; zero coils to pad. (With the turned halves
-// too, as the readout's, bp_cotangent read twice the bytes: 0.83 -> 0.89 ms at 1,048,576 spins x 512 samples.)
-__global__ void bp_h_split_kernel(const float* __restrict__ h, int rows, int n_coils, int width, const uint32_t* most,
-                                  uint2* __restrict__ hs) {
-    float scale, inverse;
-    h_scale(most, scale, inverse);
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (int64_t)rows * width) return;
-    const int64_t r = i / width;
-    const int c = (int)(i - r * width);
-    uint2 v = make_uint2(0u, 0u);
-    if (c < n_coils) {
-        const uint4 u = split_sens(h[r * 2 * n_coils + 2 * c] * scale, h[r * 2 * n_coils + 2 * c + 1] * scale);
-        v = make_uint2(u.x, u.y);
-    }
-    hs[i] = v;
 }
 
 #define CO_THREADS 128
 #define CO_WARPS (CO_THREADS / 32)
 #define CO_TAB_STRIDE 36  // float2 per row of the powers (32 spins + 4)
-#define CO_ONE 128.0f  // the powers' scale: a power of two that keeps their low halves normal, and 255 times them a half
+#define CO_ONE 1024.0f  // the powers' scale: a power of two that keeps their low halves normal, and 31 times them a half
 
 struct CotArgs {
     const float* spins;
@@ -73,7 +64,7 @@ struct CotArgs {
     const int4* runs;
     int n_runs;
     const uint2* hs;       // [rows][8 ncg]
-    const uint32_t* most;
+    const float* inverse;  // the same: of the scales, by block
     float2* g0;            // [runs that start in the windows][n]
     float2* g1;            // null, or the same of G1
     const float2* z;       // with gc: the runs' first samples, [runs that start in the windows][n]
@@ -107,9 +98,6 @@ __global__ void __launch_bounds__(CO_THREADS, WANT1 ? 3 : 4) bp_cotangent_kernel
     float2* tab = tabs[warp];
     const int lo = run_from(a.runs, a.n_runs, a.windows[a.wa].x), hi = run_from(a.runs, a.n_runs, a.windows[a.wb - 1].y);
     const int ncg = (a.n_coils + 7) / 8, width = 8 * ncg;
-    float hs_scale, hs_inv;
-    h_scale(a.most, hs_scale, hs_inv);
-    const float inv = hs_inv * (1.0f / CO_ONE);
     const int jl = min(j0 + lane, n - 1);
     const Spin sp = load_spin(a.spins, n, jl, true);
     const PropSpin p{(double)sp.px, (double)sp.py, (double)sp.pz, (double)sp.db0, sp.pd, sp.r1, sp.r2};
@@ -162,6 +150,7 @@ __global__ void __launch_bounds__(CO_THREADS, WANT1 ? 3 : 4) bp_cotangent_kernel
                 for (int blk = 0; blk < rr.z; blk += 32) {
                     float dr[4] = {0.f, 0.f, 0.f, 0.f}, di[4] = {0.f, 0.f, 0.f, 0.f};
                     float er[4] = {0.f, 0.f, 0.f, 0.f}, ei[4] = {0.f, 0.f, 0.f, 0.f};
+                    const float2 iv = *reinterpret_cast<const float2*>(a.inverse + (size_t)(rr.w + blk) * width + 8 * cg + 2 * t);
                     CPair xa = wa, xb = wb;
                     const int cnt = min(32, rr.z - blk);
                     for (int kb = 0; kb < cnt; kb += 8) {
@@ -180,8 +169,8 @@ __global__ void __launch_bounds__(CO_THREADS, WANT1 ? 3 : 4) bp_cotangent_kernel
                         mma_half(di, ha[0], hb[0], ha[1], hb[1], c0.y, c1.y);
                         mma_half(dr, ha[0], hb[0], ha[1], hb[1], b0.x, b1.x);
                         mma_half(di, ha[0], hb[0], ha[1], hb[1], c0.x, c1.x);
-                        if (WANT1) {  // the same weighed by the samples' numbers
-                            const float2 num = make_float2((float)(blk + p0), (float)(blk + p1));
+                        if (WANT1) {  // the same weighed by the samples' numbers in the block
+                            const float2 num = make_float2((float)p0, (float)p1);
                             split_half2(__fmul2_rn(xa.re, num), __fmul2_rn(xa.im, num), ha, la);
                             split_half2(__fmul2_rn(xb.re, num), __fmul2_rn(xb.im, num), hb, lb);
                             mma_half(er, la[0], lb[0], la[1], lb[1], b0.x, b1.x);
@@ -194,10 +183,24 @@ __global__ void __launch_bounds__(CO_THREADS, WANT1 ? 3 : 4) bp_cotangent_kernel
                         xa = cmul2(xa, qa, na);
                         xb = cmul2(xb, qb, nb);
                     }
+                    const float2 inv = __fmul2_rn(iv, make_float2(1.0f / CO_ONE, 1.0f / CO_ONE));
+                    const float2 from = make_float2((float)blk, (float)blk);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        tr[i] += dr[i], ti[i] += di[i];
-                        if (WANT1) ur[i] += er[i], ui[i] += ei[i];
+                    for (int i = 0; i < 4; i += 2) {  // (two coils on paired instructions)
+                        const float2 x = __fmul2_rn(make_float2(dr[i], dr[i + 1]), inv);
+                        const float2 y = __fmul2_rn(make_float2(di[i], di[i + 1]), inv);
+                        float2 v = __fadd2_rn(make_float2(tr[i], tr[i + 1]), x);
+                        tr[i] = v.x, tr[i + 1] = v.y;
+                        v = __fadd2_rn(make_float2(ti[i], ti[i + 1]), y);
+                        ti[i] = v.x, ti[i + 1] = v.y;
+                        if (WANT1) {
+                            v = __ffma2_rn(make_float2(er[i], er[i + 1]), inv, make_float2(ur[i], ur[i + 1]));
+                            v = __ffma2_rn(from, x, v);
+                            ur[i] = v.x, ur[i + 1] = v.y;
+                            v = __ffma2_rn(make_float2(ei[i], ei[i + 1]), inv, make_float2(ui[i], ui[i + 1]));
+                            v = __ffma2_rn(from, y, v);
+                            ui[i] = v.x, ui[i + 1] = v.y;
+                        }
                     }
                     if (blk + 32 < rr.z) {
                         const float2 fa = steps[warp][1][sa], fb = steps[warp][1][sb];
@@ -214,12 +217,12 @@ __global__ void __launch_bounds__(CO_THREADS, WANT1 ? 3 : 4) bp_cotangent_kernel
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         const int c = 8 * cg + 2 * t + i;
-                        const float xr = tr[2 * h + i] * inv, xi = ti[2 * h + i] * inv;
+                        const float xr = tr[2 * h + i], xi = ti[2 * h + i];
                         const float sr = a.sens[(size_t)(2 * c) * n + jj], si = a.sens[(size_t)(2 * c + 1) * n + jj];
                         g0[mt][h].x = fmaf(sr, xr, fmaf(si, xi, g0[mt][h].x));
                         g0[mt][h].y = fmaf(sr, xi, fmaf(-si, xr, g0[mt][h].y));
                         if (WANT1) {
-                            const float yr = ur[2 * h + i] * inv, yi = ui[2 * h + i] * inv;
+                            const float yr = ur[2 * h + i], yi = ui[2 * h + i];
                             g1[mt][h].x = fmaf(sr, yr, fmaf(si, yi, g1[mt][h].x));
                             g1[mt][h].y = fmaf(sr, yi, fmaf(-si, yr, g1[mt][h].y));
                         }
@@ -628,30 +631,26 @@ __global__ void bp_sweep_reduce_kernel(const float* __restrict__ gseg, int n_cta
 }
 
 // ---- launchers ----
-extern "C" int bp_cotangent_split(const float* h, int n_adc, int n_coils, void* hs, void* most, void* stream) {
-    if (n_adc < 1 || n_coils < 1 || n_coils > BP_MAX_COILS || !h || !hs || !most) return BP_E_ARG;
-    if ((reinterpret_cast<uintptr_t>(hs) & 7) != 0 || (reinterpret_cast<uintptr_t>(most) & 3) != 0) return BP_E_ALIGN;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int64_t total = (int64_t)n_adc * 2 * n_coils;
-    const int width = 8 * ((n_coils + 7) / 8);
-    if (cudaMemsetAsync(most, 0, sizeof(uint32_t), st) != cudaSuccess) return BP_E_LAUNCH;
-    const int64_t want = (total + 255) / 256;
-    bp_h_most_kernel<<<(unsigned)(want < 1024 ? want : 1024), 256, 0, st>>>(h, total, static_cast<uint32_t*>(most));
-    const int64_t cells = (int64_t)n_adc * width;
-    bp_h_split_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, st>>>(h, n_adc, n_coils, width,
-                                                                       static_cast<const uint32_t*>(most),
-                                                                       static_cast<uint2*>(hs));
+extern "C" int bp_cotangent_split(const float* h, int n_adc, int n_coils, const int* runs, int n_runs, const int* subs,
+                                  int n_subs, void* hs, float* inverse, void* stream) {
+    if (n_adc < 1 || n_coils < 1 || n_coils > BP_MAX_COILS || n_runs < 0 || n_subs < 0) return BP_E_ARG;
+    if (n_runs == 0 || n_subs == 0) return BP_OK;
+    if (!h || !runs || !subs || !hs || !inverse) return BP_E_ARG;
+    if (((reinterpret_cast<uintptr_t>(hs) | reinterpret_cast<uintptr_t>(inverse)) & 7) != 0) return BP_E_ALIGN;
+    bp_h_split_kernel<<<(unsigned)n_subs, HS_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+        h, n_coils, 8 * ((n_coils + 7) / 8), reinterpret_cast<const int4*>(runs), reinterpret_cast<const int2*>(subs),
+        static_cast<uint2*>(hs), inverse);
     return cudaGetLastError() == cudaSuccess ? BP_OK : BP_E_LAUNCH;
 }
 
 extern "C" int bp_cotangent(const float* spins, const float* sens, int n, int n_coils, const void* segs,
                             const double* seg64, const int* windows, int wa, int wb, const int* runs, int n_runs,
-                            const void* hs, const void* most, float* g0, float* g1, const float* z, float* gc,
+                            const void* hs, const float* inverse, float* g0, float* g1, const float* z, float* gc,
                             void* stream) {
     if (n < 1 || n_coils < 1 || n_coils > BP_MAX_COILS || wa < 0 || wb < wa || n_runs < 0) return BP_E_ARG;
     if (wb == wa || n_runs == 0) return BP_OK;
-    if (!spins || !sens || !segs || !seg64 || !windows || !runs || !hs || !most || !g0 || (gc && !z)) return BP_E_ARG;
-    if (((reinterpret_cast<uintptr_t>(hs) | reinterpret_cast<uintptr_t>(g0) | reinterpret_cast<uintptr_t>(g1) |
+    if (!spins || !sens || !segs || !seg64 || !windows || !runs || !hs || !inverse || !g0 || (gc && !z)) return BP_E_ARG;
+    if (((reinterpret_cast<uintptr_t>(hs) | reinterpret_cast<uintptr_t>(inverse) | reinterpret_cast<uintptr_t>(g0) | reinterpret_cast<uintptr_t>(g1) |
           reinterpret_cast<uintptr_t>(z)) & 7) != 0)
         return BP_E_ALIGN;
     CotArgs a{};
@@ -660,7 +659,7 @@ extern "C" int bp_cotangent(const float* spins, const float* sens, int n, int n_
     a.windows = reinterpret_cast<const int4*>(windows);
     a.n = n, a.n_coils = n_coils, a.wa = wa, a.wb = wb;
     a.runs = reinterpret_cast<const int4*>(runs), a.n_runs = n_runs;
-    a.hs = static_cast<const uint2*>(hs), a.most = static_cast<const uint32_t*>(most);
+    a.hs = static_cast<const uint2*>(hs), a.inverse = inverse;
     a.g0 = reinterpret_cast<float2*>(g0), a.g1 = reinterpret_cast<float2*>(g1);
     a.z = reinterpret_cast<const float2*>(z), a.gc = gc;
     const int x = (n + CO_THREADS - 1) / CO_THREADS;

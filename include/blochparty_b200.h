@@ -319,10 +319,12 @@ int bp_adjoint_saved(const float* spins, const float* sens, int n, int n_coils, 
 /* The reverse sweep in two kernels, for the gradients that need no per-segment sums but the RF waveform's, over windows
  * that are each RF segments with one dt and offset, without samples or spoils, or free segments with one set of factors,
  * spoiling at most in the last, and spins whose relaxation over an RF segment is invertible (dt / T1, dt / T2 <= 1.35).
+ * RF segments are integrated backward over a duration t (a window with gs, else a run of windows), which multiplies
+ * rounding errors by exp(t / T1) and exp(t / T2): the caller sees to it that they stay small (t / T <= 2).
  * A run of samples (runs, as bp_propagate's) belongs to the windows it starts in.
  *
- * bp_cotangent_split: hs [n_adc][8 ceil(C/8)] (8 bytes each, 8-byte aligned) and most (4 bytes) from h = dL/d(raw coil
- * sums) [n_adc][2C].
+ * bp_cotangent_split: hs [n_adc][8 ceil(C/8)] (8 bytes each, 8-byte aligned) and inverse (the same shape of float32,
+ * 8-byte aligned) from h = dL/d(raw coil sums) [n_adc][2C]; subs: the runs' 32-sample blocks (bp_sample_runs).
  * bp_cotangent: for every run that starts in windows [wa, wb) what its samples add to lambda at its first sample, g0
  * [those runs][n] (float32, float32), and weighed by the samples' numbers g1 (or NULL); with gc [2C][n] += the coil
  * gradients, from z, the runs' first samples in the same layout (bp_propagate's z).
@@ -331,10 +333,11 @@ int bp_adjoint_saved(const float* spins, const float* sens, int n, int n_coils, 
  * start, then after the last. Without: states by slot, wslot, chain and chain_in as bp_adjoint_saved's. gseg
  * [bp_sweep_grid][seg_len][2] (or NULL; seg_len <= 2048 then) is scratch for the RF waveform's gradient, added to
  * columns 1 and 2 of seg [S][8] (float64) as bp_seg_reduce does. status as bp_adjoint_saved's. */
-int bp_cotangent_split(const float* h, int n_adc, int n_coils, void* hs, void* most, void* stream);
+int bp_cotangent_split(const float* h, int n_adc, int n_coils, const int32_t* runs, int n_runs, const int32_t* subs,
+                       int n_subs, void* hs, float* inverse, void* stream);
 int bp_cotangent(const float* spins, const float* sens, int n, int n_coils, const void* segs, const double* seg64,
                  const int32_t* windows, int wa, int wb, const int32_t* runs, int n_runs, const void* hs,
-                 const void* most, float* g0, float* g1, const float* z, float* gc, void* stream);
+                 const float* inverse, float* g0, float* g1, const float* z, float* gc, void* stream);
 int bp_sweep_grid(int n, int seg_len, int spin_gradients);
 int bp_sweep(const float* spins, int n, const void* segs, const double* seg64, const int32_t* windows, int wa, int wb,
              int seg0, int seg_len, const float* wstates, const int32_t* wslot, float* chain, int chain_in,

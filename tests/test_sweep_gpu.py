@@ -167,3 +167,46 @@ def test_long_intervals(names, monkeypatch):
     assert seen and all(seen)
     _, exact = bloch.gradients(bloch.case_from(ph, seq, c), _loss, names)
     _close(want, exact, names)
+
+
+def test_weights_far_apart():
+    """A loss that weighs early samples 10^9 above late ones, and one coil 10^9 below another: the late pulses' RF
+    gradient, which only late samples reach, and the faint coil's keep their precision."""
+    n = 45
+    ph, c = _phantom(n, 10), _coils(n, 3)
+    b = sequences.SequenceBuilder()
+    for i in range(3):
+        b.rf_waveform((np.random.RandomState(i).rand(40, 2) - 0.4) * 2500, 10e-6, grad=(300.0, 0.0, 1000.0))
+        b.readout(50, 10e-6, grad=(-2500.0, 300.0, 400.0)).delay(1e-3, grad=(3e3, 1e3, 0.0)).spoil()
+    seq = b.build()
+    weight = torch.tensor([1e9, 1.0, 1e-3], dtype=F64).repeat_interleave(50)[None, :] * torch.tensor(
+        [[1.0], [1e-9], [1.0]], dtype=F64)
+
+    def loss(sig, m):
+        w = weight * torch.randn(sig.shape, generator=torch.Generator().manual_seed(5), dtype=F64)
+        return (sig.real.double() * w).sum() + 0.5 * (sig.imag.double() * w).sum()
+
+    rf, co = seq.rf.clone().requires_grad_(), c.clone().requires_grad_()
+    r = bpb.simulate(ph, replace(seq, rf=rf), co, checkpoint_every=64)
+    g_rf, g_c = torch.autograd.grad(loss(r.signal, r.m), (rf, co))
+    _, want = bloch.gradients(bloch.case_from(ph, seq, c), loss, ("rf", "coils"))
+    starts = np.flatnonzero(np.diff(np.asarray(seq.is_rf).astype(int), prepend=0) == 1)
+    for s in starts:
+        _close({"rf": g_rf[s:s + 40]}, {"rf": want["rf"][s:s + 40]}, ("rf",))
+    for i in range(3):
+        _close({"c": g_c[:, i]}, {"c": want["coils"][:, i]}, ("c",))
+
+
+def test_runs_of_any_length(monkeypatch):
+    """Runs longer than the forward's longest, the samples' numbers in hundreds: their part of the maps' gradients."""
+    ph, c, names = _phantom(40, 11), _coils(40, 4), ("t2", "db0", "coils")
+    b = sequences.SequenceBuilder()
+    for i in range(2):
+        b.rf(20e-6, flip_deg=30.0).readout(900, 5e-6, grad=(-900.0, 300.0, 400.0)).delay(1e-3)
+    seq = b.build()
+    run = adjoint.engine.sample_runs
+    assert run(np.full(900, 8 | 2, dtype=np.int32))[0][:, 2].max() <= engine.RUN_MAX
+    monkeypatch.setattr(engine, "RUN_MAX", 1 << 20)
+    got = _gradients(ph, seq, c, names, every=3200)
+    _, want = bloch.gradients(bloch.case_from(ph, seq, c), _loss, names)
+    _close(got, want, names)
