@@ -20,7 +20,7 @@
 #include <cstdint>
 #include <cstring>
 
-#include "bloch_common.cuh"
+#include "packed.cuh"
 #include "../../include/blochparty_b200.h"
 
 #define MLP_H 64
@@ -500,17 +500,18 @@ struct PulseArgs {
     const float* params;  // the pulse's network
     const SegRec* segs;   // the occurrence's segments for the fallback: segs[seg0 .. seg0 + k_steps)
     int seg0, k_steps, n;
-    double T, gz, thickness, z0, phi0;  // duration [s], slice gradient [Hz/m], thickness [m], centre [m], RF phase
+    double T, gz, per_thickness, z0, phi0;  // duration [s], slice gradient [Hz/m], 1 / thickness [1/m], centre [m], RF phase
     float b0off;          // the occurrence's uniform off-resonance [Hz]
     int* counts;          // null or [2]: spins through the network, spins through the fallback
     float dom_df, dom_b1, dom_z;  // the network's training domain
-    double fmax;                  // dom_df + |gz| dom_z thickness: the scale of the input f^
+    double per_fmax;              // 1 / (dom_df + |gz| dom_z thickness): the scale of the input f^ (a float64 division a
+                                  // spin was 3 % of the kernel)
 };
 
 // The network's inputs (f^, b^) of a spin (f^ clamped to [-1, 1]: rows outside the domain, whose outputs are not
 // used, stay finite).
 __device__ __forceinline__ void pulse_inputs(const PulseArgs& a, const Spin& p, float df, float x[MLP_X]) {
-    const float fh = (float)(((double)df + a.gz * ((double)p.pz - a.z0)) / a.fmax);
+    const float fh = (float)(((double)df + a.gz * ((double)p.pz - a.z0)) * a.per_fmax);
     x[0] = fminf(fmaxf(fh, -1.f), 1.f);
     x[1] = fminf(fmaxf((p.b1 - 1.0f) / a.dom_b1, -1.f), 1.f);
 }
@@ -583,7 +584,7 @@ __device__ __forceinline__ void apply_pulse_map(const float* y, const PulseArgs&
         R[6 + c] = fmaf(k, X[6 + c], R[6 + c]);
     }
     const float th = 0.5f * T;
-    const float e1 = expm1f(-th * p.r1), e2 = expm1f(-th * p.r2);
+    const float e1 = relax_expm1(-th * p.r1), e2 = relax_expm1(-th * p.r2);
     const float ax = (mx + lx) * (1.0f + e2), ay = (my + ly) * (1.0f + e2);
     const float az = fmaf((mz + lz) - p.pd, e1, mz + lz);
     const float nx = fmaf(R[0], ax, fmaf(R[1], ay, R[2] * az));
@@ -605,7 +606,7 @@ __global__ void __launch_bounds__(128) bp_surrogate_pulse_kernel(PulseArgs a) {
     const int jj = active ? j : 0;
     const Spin p = load_spin(a.spins, a.n, jj, active);
     const float df = p.db0 + a.b0off;
-    const float zr = (float)(((double)p.pz - a.z0) / a.thickness);
+    const float zr = (float)(((double)p.pz - a.z0) * a.per_thickness);
     const bool inside = fabsf(df) <= a.dom_df && fabsf(p.b1 - 1.0f) <= a.dom_b1 && fabsf(zr) <= a.dom_z;
     if (a.counts) {
         const unsigned in_mask = __ballot_sync(0xffffffffu, active && inside);
@@ -643,8 +644,8 @@ extern "C" int bp_surrogate_pulse(const float* spins, float* state, int n, const
     if (!spins || !state || !params || !segs || n < 1 || seg0 < 0 || k_steps < 1 || T <= 0 || thickness <= 0 ||
         !(dom_df > 0) || !(dom_b1 > 0) || !(dom_z > 0))
         return BP_E_ARG;
-    PulseArgs a{spins, state, params, static_cast<const SegRec*>(segs), seg0, k_steps, n, T, gz, thickness, z0, phi0,
-                b0off, counts, dom_df, dom_b1, dom_z, dom_df + fabs(gz) * dom_z * thickness};
+    PulseArgs a{spins, state, params, static_cast<const SegRec*>(segs), seg0, k_steps, n, T, gz, 1.0 / thickness, z0, phi0,
+                b0off, counts, dom_df, dom_b1, dom_z, 1.0 / (dom_df + fabs(gz) * dom_z * thickness)};
     bp_surrogate_pulse_kernel<<<(n + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(a);
     return cudaGetLastError() == cudaSuccess ? BP_OK : BP_E_LAUNCH;
 }
@@ -655,7 +656,10 @@ extern "C" int bp_surrogate_pulse(const float* spins, float* state, int n, const
 // the shared memory held three tiles per SM, now four. The GELU's arithmetic runs on paired instructions with one
 // reciprocal for two values (the special-function unit was its bound). One 300-step pulse over 393,216 spins: 0.0924 ms
 // before; 0.0782 with the pairs and one group in each of three CTAs, 0.0761 with two blocks of columns in flight, 0.0739
-// with two groups in each of two CTAs; five groups in one CTA 0.0787, four 0.086.
+// with two groups in each of two CTAs (five groups in one CTA 0.0787, four 0.086); 0.0715 with one multiplication fewer in
+// the GELU, 0.0690 with the wait for a layer's product at the loop's head and all four blocks of columns in flight, 0.0670
+// without float64 divisions. (Half a layer's product issued while the other half's operand is formed: 0.0715, the barriers
+// cost more; spins and states read ahead: the same.)
 // Per tile of 128 spins (a group's thread t = spin row t = tensor-memory lane t), four rounds, one per layer: every
 // thread stores its row of the layer's input, split into bfloat16 high and low parts, as the A operand (K-major),
 // one thread issues D = A_hi W_hi^T + A_hi W_lo^T + A_lo W_hi^T (M = 128, float32 accumulation in tensor memory),
@@ -710,20 +714,21 @@ __device__ __forceinline__ bool group_sync_or(int group, bool pred) {
     return any != 0;
 }
 
-// gelu_f of two values: its arithmetic on paired instructions, exp2 and the reciprocal without the handling of
-// denormals (1 + exp(-2u) is never one, and an exp(-2u) that is one does not change the sum).
+// gelu_f of two values: x / (1 + 2^u), u = -2 c log2(e) (x + 0.044715 x^3), its arithmetic on paired instructions, exp2
+// and the reciprocal without the handling of denormals (1 + 2^u is never one, and a 2^u that is one does not change the
+// sum). One reciprocal for the two, 1 / d = d' / (d d'): with one each the special-function unit held the kernel up (a
+// 300-step pulse over 393,216 spins 0.0797 against 0.0740 ms); the two roundings more (1e-7) are a hundredth of what the
+// layers' split operands keep.
 __device__ __forceinline__ float2 gelu_pair(const float2& x) {
-    const float k = -2.0f * 0.7978845608028654f * 1.4426950408889634f;  // -2 c log2(e)
-    const float2 t = __ffma2_rn(__fmul2_rn(x, make_float2(0.044715f, 0.044715f)), __fmul2_rn(x, x), x);
-    float2 u = __fmul2_rn(t, make_float2(k, k)), e, s;
+    const float k = -2.0f * 0.7978845608028654f * 1.4426950408889634f, k3 = 0.044715f * k;
+    float2 u = __fmul2_rn(x, __ffma2_rn(__fmul2_rn(x, x), make_float2(k3, k3), make_float2(k, k))), e;
     u.x = fminf(u.x, 60.0f), u.y = fminf(u.y, 60.0f);  // (the product of the denominators stays finite)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(u.x));
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(u.y));
     const float2 d = __fadd2_rn(e, make_float2(1.0f, 1.0f));
-    float both;  // one reciprocal for the two: 1 / x = y / (x y)
+    float both;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(both) : "f"(d.x * d.y));
-    s = __fmul2_rn(make_float2(d.y, d.x), make_float2(both, both));
-    return __fmul2_rn(x, s);
+    return __fmul2_rn(x, __fmul2_rn(make_float2(d.y, d.x), make_float2(both, both)));
 }
 
 // NCH x 8 values of this thread's row -> A hi and A lo rows, chunks [chunk0, chunk0 + NCH) (16-byte stores)
@@ -802,7 +807,7 @@ __global__ void __launch_bounds__(SI_THREADS, 2) bp_surrogate_pulse_mma_kernel(c
         const int j = active ? j0 : 0;
         const Spin p = load_spin(a.spins, a.n, j, active);
         const float df = p.db0 + a.b0off;
-        const float zr = (float)(((double)p.pz - a.z0) / a.thickness);
+        const float zr = (float)(((double)p.pz - a.z0) * a.per_thickness);
         const bool inside = active && fabsf(df) <= a.dom_df && fabsf(p.b1 - 1.0f) <= a.dom_b1 && fabsf(zr) <= a.dom_z;
         // spins outside the domain join the group's queue; whenever it holds 128, its threads step them (full warps
         // whatever the spins' order)
@@ -828,37 +833,39 @@ __global__ void __launch_bounds__(SI_THREADS, 2) bp_surrogate_pulse_mma_kernel(c
             store_row_bf16x2<SI_K1 / 8>(ahi, alo, tid, g, 0);
         }
 #pragma unroll 1
-        for (int layer = 0; layer < 4; ++layer) {  // a real loop: one copy of the code serves the four layers
-            fence_proxy_async_smem();
-            tc_fence_before();
-            if (group_sync_or(group, err)) {
-                fail = true;
-                break;
+        // a layer's product, issued by one thread
+        auto issue = [&](int layer) {
+            if (!w_ready && !mbar_wait_bounded(wbar, 0)) err = true;
+            w_ready = true;
+            if (err) return;
+            tc_fence_after();
+            const uint32_t wh = layer == 0 ? sW + SI_OFF_W1
+                              : layer == 3 ? sW + SI_OFF_W4
+                                           : sW + (uint32_t)(2 * (layer - 1)) * SI_W_BYTES;
+            const uint32_t wl = wh + (layer == 0 ? SI_W1_BYTES : layer == 3 ? SI_W4_BYTES : SI_W_BYTES);
+            const uint32_t sbo_w = layer == 0 ? SI_SBO_W1 : SI_SBO;
+            const uint32_t idesc = umma_idesc_bf16_f32(128, layer == 3 ? MLP_OUT : MLP_H);
+            uint64_t ah_d = umma_desc(sA, SI_LBO, SI_SBO), al_d = umma_desc(sA + SI_A_BYTES, SI_LBO, SI_SBO);
+            uint64_t bh_d = umma_desc(wh, SI_LBO, sbo_w), bl_d = umma_desc(wl, SI_LBO, sbo_w);
+            const int k_steps = layer == 0 ? SI_K1 / 16 : MLP_H / 16;
+            for (int kk = 0; kk < k_steps; ++kk) {
+                umma_bf16(tmem, ah_d, bh_d, idesc, kk > 0 ? 1u : 0u);
+                umma_bf16(tmem, ah_d, bl_d, idesc, 1u);
+                umma_bf16(tmem, al_d, bh_d, idesc, 1u);
+                ah_d += 2 * SI_LBO / 16, al_d += 2 * SI_LBO / 16, bh_d += 2 * SI_LBO / 16, bl_d += 2 * SI_LBO / 16;
             }
-            if (tid == 0) {
-                if (!w_ready && !mbar_wait_bounded(wbar, 0)) err = true;
-                w_ready = true;
-                if (!err) {
-                    tc_fence_after();
-                    const uint32_t wh = layer == 0 ? sW + SI_OFF_W1
-                                      : layer == 3 ? sW + SI_OFF_W4
-                                                   : sW + (uint32_t)(2 * (layer - 1)) * SI_W_BYTES;
-                    const uint32_t wl = wh + (layer == 0 ? SI_W1_BYTES : layer == 3 ? SI_W4_BYTES : SI_W_BYTES);
-                    const uint32_t sbo_w = layer == 0 ? SI_SBO_W1 : SI_SBO;
-                    const uint32_t idesc = umma_idesc_bf16_f32(128, layer == 3 ? MLP_OUT : MLP_H);
-                    uint64_t ah_d = umma_desc(sA, SI_LBO, SI_SBO), al_d = umma_desc(sA + SI_A_BYTES, SI_LBO, SI_SBO);
-                    uint64_t bh_d = umma_desc(wh, SI_LBO, sbo_w), bl_d = umma_desc(wl, SI_LBO, sbo_w);
-                    const int k_steps = layer == 0 ? SI_K1 / 16 : MLP_H / 16;
-                    for (int kk = 0; kk < k_steps; ++kk) {
-                        umma_bf16(tmem, ah_d, bh_d, idesc, kk > 0 ? 1u : 0u);
-                        umma_bf16(tmem, ah_d, bl_d, idesc, 1u);
-                        umma_bf16(tmem, al_d, bh_d, idesc, 1u);
-                        ah_d += 2 * SI_LBO / 16, al_d += 2 * SI_LBO / 16, bh_d += 2 * SI_LBO / 16, bl_d += 2 * SI_LBO / 16;
-                    }
-                    umma_commit(bar);
-                }
-            }
-            mma_out = true;
+            umma_commit(bar);
+        };
+        fence_proxy_async_smem();
+        tc_fence_before();
+        if (group_sync_or(group, err)) {
+            fail = true;
+            break;
+        }
+        if (tid == 0) issue(0);
+        mma_out = true;
+#pragma unroll 1
+        for (int layer = 0; layer < 4; ++layer) {  // a real loop: one copy of the code serves the layers
             if (mbar_wait_bounded(bar, mma_phase)) {
                 mma_phase ^= 1u;
                 mma_out = false;
@@ -866,31 +873,39 @@ __global__ void __launch_bounds__(SI_THREADS, 2) bp_surrogate_pulse_mma_kernel(c
                 err = true;  // (seen by all at the next barrier; what is stored until then is not used)
             }
             tc_fence_after();
-            if (layer < 3) {
-                // the layer's output 16 columns at a time: bias and GELU, split straight into the next A operand
-                // (the MMA that read the A operand has completed)
-                const float* b = bias + layer * MLP_H;
-#pragma unroll 2
-                for (int c0 = 0; c0 < MLP_H; c0 += 16) {
-                    float d[16];
-                    tmem_ld16(lane_addr + (uint32_t)c0, d);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
-                        const float2 g = gelu_pair(__fadd2_rn(make_float2(d[i], d[i + 1]),
-                                                              make_float2(b[c0 + i], b[c0 + i + 1])));
-                        d[i] = g.x, d[i + 1] = g.y;
-                    }
-                    store_row_bf16x2<2>(ahi, alo, tid, d, c0 / 8);
-                }
-            } else {
+            if (layer == 3) {
                 float d[16];
                 tmem_ld16(lane_addr, d);
                 tmem_ld_wait();
 #pragma unroll
                 for (int o = 0; o < MLP_OUT; ++o) y[o] = d[o] + bias[3 * MLP_H + o];
+                tc_fence_before();
+                break;
             }
+            // the layer's output 16 columns at a time: bias and GELU, split straight into the next A operand (the MMA that
+            // read the A operand has completed)
+            const float* b = bias + layer * MLP_H;
+#pragma unroll
+            for (int c0 = 0; c0 < MLP_H; c0 += 16) {
+                float d[16];
+                tmem_ld16(lane_addr + (uint32_t)c0, d);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; i += 2) {
+                    const float2 g = gelu_pair(__fadd2_rn(make_float2(d[i], d[i + 1]),
+                                                          make_float2(b[c0 + i], b[c0 + i + 1])));
+                    d[i] = g.x, d[i + 1] = g.y;
+                }
+                store_row_bf16x2<2>(ahi, alo, tid, d, c0 / 8);
+            }
+            fence_proxy_async_smem();
             tc_fence_before();
+            if (group_sync_or(group, err)) {
+                fail = true;
+                break;
+            }
+            if (tid == 0) issue(layer + 1);
+            mma_out = true;
         }
         if (fail) break;
         const int nq = *queued;  // (no thread adds to it between the first layer's barrier and the next)
@@ -1024,8 +1039,8 @@ extern "C" int bp_surrogate_pulse_mma(const float* spins, float* state, int n, c
     int grid = 0;
     const int code = pulse_mma_grid(n, max_ctas, &grid);
     if (code != BP_OK) return code;
-    PulseMmaArgs a{{spins, state, nullptr, static_cast<const SegRec*>(segs), seg0, k_steps, n, T, gz, thickness, z0,
-                    phi0, b0off, counts, dom_df, dom_b1, dom_z, dom_df + fabs(gz) * dom_z * thickness},
+    PulseMmaArgs a{{spins, state, nullptr, static_cast<const SegRec*>(segs), seg0, k_steps, n, T, gz, 1.0 / thickness, z0,
+                    phi0, b0off, counts, dom_df, dom_b1, dom_z, 1.0 / (dom_df + fabs(gz) * dom_z * thickness)},
                    static_cast<const uint8_t*>(wtiles), status, {}};
     std::memcpy(a.net.bias, params_host + P_B1, MLP_H * sizeof(float));
     std::memcpy(a.net.bias + MLP_H, params_host + P_B2, MLP_H * sizeof(float));

@@ -275,14 +275,27 @@ def find_occurrences(surrogates, inp, tol: float = 1e-6):
     d = lambda t: t.detach().to(F64).cpu().numpy()
     dt, rf, grad = d(inp.dt), d(inp.rf), d(inp.grad)
     S = len(dt)
-    b0 = np.zeros(S) if inp.b0_offset is None else d(inp.b0_offset)
-    is_rf, adc, spoil = (np.fromiter(f, dtype=bool, count=S) for f in (inp.is_rf, inp.adc, inp.spoil))
-    w = rf[:, 0] + 1j * rf[:, 1]
-    gxy = np.abs(grad[:, :2]).max(1)
+    b0 = None if inp.b0_offset is None else d(inp.b0_offset)
+    is_rf, adc, spoil = (engine._bools(f, S) for f in (inp.is_rf, inp.adc, inp.spoil))
+    w = np.ascontiguousarray(rf[:, :2]).view(np.complex128)[:, 0]
+    gxy = np.maximum(np.abs(grad[:, 0]), np.abs(grad[:, 1]))
     base = ~is_rf | adc | spoil
-    clean = [sg.clean_windows(dt, grad[:, 2], base | (gxy > 1e-9 * max(abs(sg.gz), 1.0))) for sg in surrogates]
+    prefix = {}  # the prefix counts of every (dt, gz) among the surrogates
+
+    def clean_of(sg):
+        key = (sg.dt, sg.gz)
+        if key not in prefix:
+            prefix[key] = sg.clean_windows(dt, grad[:, 2], base | (gxy > 1e-9 * max(abs(sg.gz), 1.0)))
+        return prefix[key]
+
     # b0_offset steps: a window [s, e) is uniform when no step lies in (s, e)
-    steps = np.concatenate([[0], np.cumsum(np.concatenate([[False], np.abs(np.diff(b0)) > 1e-9]))])
+    steps = None if b0 is None else np.concatenate([[0], np.cumsum(np.concatenate([[False], np.abs(np.diff(b0)) > 1e-9]))])
+    waves = []  # the waveforms, and two samples that a match has to have (the strongest, and one a tenth of a pulse on)
+    for sg in surrogates:
+        z = sg.rf[:, 0].numpy() + 1j * sg.rf[:, 1].numpy()
+        p = int(np.abs(z).argmax())
+        q = p + max(1, sg.K // 10)
+        waves.append((z, p, q if q < sg.K else max(0, p - max(1, sg.K // 10))))
     occ = []
     cands = np.flatnonzero(is_rf & ~np.concatenate([[False], is_rf[:-1]]))
     while cands.size:
@@ -291,19 +304,26 @@ def find_occurrences(surrogates, inp, tol: float = 1e-6):
         for i, sg in enumerate(surrogates):
             e = cands + sg.K
             ok = ~taken & (e <= S)
-            ec = np.minimum(e, S)
-            ok &= (clean[i][ec] == clean[i][cands]) & (steps[ec] == steps[np.minimum(cands + 1, S)])
+            ec, clean = np.minimum(e, S), clean_of(sg)
+            ok &= clean[ec] == clean[cands]
+            if steps is not None:
+                ok &= steps[ec] == steps[np.minimum(cands + 1, S)]
             idx = np.flatnonzero(ok)
+            z, p, q = waves[i]
+            most = np.abs(z).max()
+            # a match has every |w_k - z_k e^(i phi)| <= tol most, so |w_p conj(w_q) - z_p conj(z_q)| <= tol most (2 + tol)
+            # most: the rest need not be compared as a whole
+            wp, wq = w[cands[idx] + p], w[cands[idx] + q]
+            idx = idx[np.abs(wp * np.conj(wq) - z[p] * np.conj(z[q])) <= tol * (2.1 + tol) * most ** 2]
             if idx.size == 0:
                 continue
-            z = sg.rf[:, 0].numpy() + 1j * sg.rf[:, 1].numpy()
             W = w[cands[idx, None] + np.arange(sg.K)]
             c = W @ np.conj(z)
             phi = np.where(c != 0, np.angle(c), 0.0)
-            good = np.abs(W - z[None, :] * np.exp(1j * phi)[:, None]).max(1) <= tol * np.abs(z).max()
+            good = np.abs(W - z[None, :] * np.exp(1j * phi)[:, None]).max(1) <= tol * most
             for j, ph in zip(idx[good].tolist(), phi[good].tolist()):
                 s0 = int(cands[j])
-                occ.append((s0, sg.K, i, ph, float(b0[s0])))
+                occ.append((s0, sg.K, i, ph, 0.0 if b0 is None else float(b0[s0])))
             taken[idx[good]] = True
             ends.append(e[idx[good]])
         cands = np.concatenate(ends) if ends else np.zeros(0, dtype=np.int64)
