@@ -233,6 +233,13 @@ class Plan:
         self.max_len = max(b - a for a, b in self.seg_ranges)
 
 
+def room_to_keep(free: int, cached: int, total: int) -> int:
+    """Bytes that one simulation's graph may hold in states of every window: a sixteenth of the device's memory, and only
+    from what lies above half of it free (``cached``: what the allocator holds unused), so that the graphs of many
+    simulations in one loss leave that half alone, and later ones fall back to checkpoints."""
+    return max(min(total // 16, free + cached - total // 2), 0)
+
+
 def sweep_pieces(awin: np.ndarray, wa: int, wb: int, run_starts: np.ndarray, room: int):
     """[(first window, end window, first segment, end segment)]: windows [wa, wb) of ``awin`` in pieces that one sweep
     takes, of at most ``BP_SWEEP_MAX`` segments and with at most ``room`` runs of samples starting in them (or one
@@ -281,14 +288,19 @@ class Checkpointed:
                 budget_bytes = torch.cuda.mem_get_info(device)[0] // 2 if torch.cuda.is_available() else 1 << 62
             self.layout = saved_layout(plan, 24 * pk.n, budget_bytes)
         # keep: the caller leaves the stored states to this class; then, where the sweep takes a window in one step and
-        # the states fit a quarter of the free memory, the forward saves the state at every adjoint window's start and
-        # the backward replays nothing (its intervals are as long as the sweep takes)
+        # the states fit ``room_to_keep``, the forward saves the state at every adjoint window's start and the backward
+        # replays nothing (its intervals are as long as the sweep takes)
         self.kept = None
         if self.layout is None and keep and invertible:
             plan = Plan(pk, _lib.BP_SWEEP_MAX, device)
-            room = torch.cuda.mem_get_info(device)[0] // 4 if torch.cuda.is_available() else 0
-            if (self.sweepable(plan) and 24 * pk.n * (plan.awin.shape[0] + 1) <= room
-                    and 8 * pk.n * pk.sample_runs().n_runs <= min(engine.Z_BYTES, room)):
+            room = 0
+            if torch.cuda.is_available():
+                free, total = torch.cuda.mem_get_info(device)
+                cached = torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
+                room = room_to_keep(free, cached, total)
+            z_bytes = 8 * pk.n * pk.sample_runs().n_runs
+            if (z_bytes <= engine.Z_BYTES and 24 * pk.n * (plan.awin.shape[0] + 1) + z_bytes <= room
+                    and self.sweepable(plan)):
                 self.kept = torch.empty(plan.awin.shape[0] + 1, 6, pk.n, dtype=F32, device=device)
         if self.layout is None and self.kept is None:
             plan = Plan(pk, every, device)

@@ -362,6 +362,19 @@ def test_sweep_pieces(room):
                 assert more[3] - more[2] > _lib.BP_SWEEP_MAX or count(more) > room
 
 
+def test_room_to_keep_leaves_half_the_device():
+    """However many graphs are alive, each taking all that it may: half of the device stays free, and the last ones keep
+    nothing; what the allocator holds unused counts as free."""
+    from blochparty_b200 import adjoint
+
+    total, held = 180 << 30, 0
+    for _ in range(100):
+        held += adjoint.room_to_keep(total - held, 0, total)
+    assert held == total // 2 and adjoint.room_to_keep(total - held, 0, total) == 0
+    assert adjoint.room_to_keep(total // 4, total // 2, total) == total // 16
+    assert adjoint.room_to_keep(total // 4, 0, total) == 0
+
+
 def test_backward_integration_is_bounded_by_the_decay():
     """rf_decay: the longest RF window and the longest run of them, times the largest rate of any spin; what a sweep may
     integrate backward is decided on it, not on one step."""

@@ -210,3 +210,26 @@ def test_runs_of_any_length(monkeypatch):
     got = _gradients(ph, seq, c, names, every=3200)
     _, want = bloch.gradients(bloch.case_from(ph, seq, c), _loss, names)
     _close(got, want, names)
+
+
+def test_many_graphs_alive():
+    """Every window's states are kept while more than half of the device is free, else the checkpoints' replay: the same
+    gradients, bit for bit."""
+    n, names = 60, ("t1", "coils")
+    ph, seq, c = _phantom(n, 12), _sequence((40, 17)), _coils(n, 2)
+    kept, init = [], adjoint.Checkpointed.__init__
+
+    def spy(self, *a, **kw):
+        init(self, *a, **kw)
+        kept.append(self.kept is not None)
+
+    out = []
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(adjoint.Checkpointed, "__init__", spy)
+        for share in (0.9, 0.4):
+            m.setattr(torch.cuda, "mem_get_info", lambda *a: (int(share * (180 << 30)), 180 << 30))
+            m.setattr(torch.cuda, "memory_reserved", lambda *a: 0)
+            m.setattr(torch.cuda, "memory_allocated", lambda *a: 0)
+            out.append(_gradients(ph, seq, c, names))
+    assert kept == [True, False]
+    assert all(torch.equal(out[0][k], out[1][k]) for k in names)
