@@ -104,10 +104,11 @@ SIGNATURES = {
     "bp_final_m": (c_int, [_P, c_int, _P, _P]),
     "bp_propagate": (c_int, [_P, c_int, _P, _P, _P, c_int, c_int, _P, _P, c_int, _P, _P, c_int, _P, c_int, c_int, c_int,
                              _P, _P]),
-    "bp_readout": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, _P, c_int, _P, c_int, _P, c_int, c_int, _P,
-                           _P]),
-    "bp_forward_spans": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, _P, c_int, _P, _P, _P, c_int, _P, c_int, _P, c_int,
-                                 _P, _P, c_int, _P, _P]),
+    "bp_readout": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, c_int, c_int, _P, c_int, _P, c_int, c_int, _P, c_int,
+                           c_int, _P, _P]),
+    "bp_forward_spans": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, _P, c_int, _P, _P, _P, c_int, _P, _P]),
+    "bp_forward_spans_readout": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, _P, c_int, _P, _P, _P, c_int, _P, c_int, _P,
+                                         c_int, c_int, _P, _P, c_int, _P, _P]),
     "bp_signal_finish": (c_int, [_P, _P, c_int, c_int, _P, _P]),
     "bp_ffma_peak": (c_int, [_P, c_int, _P, _P]),
     "bp_ffma2_peak": (c_int, [_P, c_int, _P, _P]),

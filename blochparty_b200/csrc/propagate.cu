@@ -59,17 +59,28 @@ struct PropArgs {
     int* status;
 };
 
-// The first run that starts at segment s or later (inside: that ends after s).
-__device__ __forceinline__ int first_run(const int4* __restrict__ runs, int n_runs, int s, bool inside) {
-    int lo = 0, hi = n_runs;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (runs[mid].x + (inside ? runs[mid].z - 1 : 0) < s)
-            lo = mid + 1;
-        else
-            hi = mid;
+// The first of [0, n) for which `before` does not hold (it holds up to there), by a warp: 32 probes a step.
+template <class F>
+__device__ __forceinline__ int warp_bound(int n, int lane, F before) {
+    int lo = 0, len = n;
+    while (len > 0) {
+        const int step = (len + 31) / 32, i = lo + lane * step;
+        const int k = __popc(__ballot_sync(0xffffffffu, i < lo + len && before(i)));
+        if (k == 0) break;
+        const int end = min(lo + k * step, lo + len);
+        lo += (k - 1) * step + 1;
+        len = end - lo;
     }
     return lo;
+}
+
+// The first run of windows that start at segment s: the first that starts there or later, or with BP_CLIP_BEGIN that
+// ends after s. (warp)
+__device__ __forceinline__ int windows_run(const int4* __restrict__ runs, int n_runs, int s, int clip, int lane) {
+    return warp_bound(n_runs, lane, [&](int i) {
+        const int4 r = runs[i];
+        return r.x + ((clip & BP_CLIP_BEGIN) ? r.z - 1 : 0) < s;
+    });
 }
 
 // The kernel's list of a chunk's steps: a first segment, its length, and what it is.
@@ -134,7 +145,7 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 8 : HELP ? 5 : 4) bp_propagate_
         tma_load_1d(k64buf + buf * CH, a.seg64 + c, bytes, &bars[buf]);
     };
     if (tid == 0 && (int)blockIdx.x < n_tiles) issue(s_begin, 0);
-    const int run_lo = a.z ? first_run(a.runs, a.n_runs, s_begin, (a.clip & BP_CLIP_BEGIN) != 0) : 0;
+    const int run_lo = a.z ? windows_run(a.runs, a.n_runs, s_begin, a.clip, lane) : 0;
 
     int it = 0;  // chunks staged so far (buffer it & 1, its phase (it >> 1) & 1)
     for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
@@ -376,6 +387,7 @@ struct ReadArgs {
     int n_runs;
     const int2* subs;      // [n_subs]: run, 32-sample block of it
     int n_subs;
+    int first_y;           // the block of the grid's first row: the grid takes RO_SUBS blocks a row, from the windows' first
     const float2* z;
     int z_cap;
     int per_part;          // groups of 32 spins per blockIdx.x
@@ -388,36 +400,45 @@ __global__ void __launch_bounds__(RO_THREADS, 3) bp_readout_kernel(ReadArgs a) {
     __shared__ __align__(16) float fetched[RO_WARPS][RO_FETCH * 32];
     __shared__ __align__(16) float2 fetched_z[RO_WARPS][RO_SUBS * 32];
     __shared__ int4 sub[RO_SUBS];   // samples (0: none), slot of z, 32-sample block, first ADC row
-    __shared__ int ratio[RO_SUBS];  // the segment of the factor; -1 - (segment) where it is the block before's
+    __shared__ int ratio[RO_SUBS];  // the segment of the factor; -1 where it is the block before's
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = a.n, cg = blockIdx.z;
-    if (tid == 0) {
+    if (warp == 0) {
         const int s_begin = a.windows[a.w_begin].x, s_end = a.windows[a.w_end - 1].y;
-        const int lo = first_run(a.runs, a.n_runs, s_begin, (a.clip & BP_CLIP_BEGIN) != 0);
-        const int hi = min(first_run(a.runs, a.n_runs, s_end, false), lo + a.z_cap);
-        int before = -1;  // the block before's factor segment
-        for (int b = 0; b < RO_SUBS; ++b) {
-            const int i = blockIdx.y * RO_SUBS + b;
-            sub[b] = make_int4(0, 0, 0, 0);
-            ratio[b] = -1;
-            if (i >= a.n_subs) continue;
-            const int2 rb = a.subs[i];
-            if (rb.x < lo || rb.x >= hi) continue;
-            const int4 r = a.runs[rb.x];
-            const int begin = max(r.x, s_begin);  // (a run's samples lie on consecutive segments)
-            const int end = (a.clip & BP_CLIP_END) ? min(r.x + r.z, s_end) : r.x + r.z;
-            const int samples = min(32, end - begin - 32 * rb.y);
-            if (samples <= 0) continue;
-            sub[b] = make_int4(samples, rb.x - lo, rb.y, r.w + begin - r.x + 32 * rb.y);
-            const int seg = r.y >= 0 ? r.y : r.x;
-            bool same = before >= 0;
-            if (same) {
-                const SegRec u = a.segs[before], v = a.segs[seg];
-                const double4 x = a.seg64[before], y = a.seg64[seg];
-                same = u.dt == v.dt && x.x == y.x && x.y == y.y && x.z == y.z && x.w == y.w;
+        const int lo = windows_run(a.runs, a.n_runs, s_begin, a.clip, lane);
+        const int hi = min(warp_bound(a.n_runs, lane, [&](int i) { return a.runs[i].x < s_end; }), lo + a.z_cap);
+        const int from = warp_bound(a.n_subs, lane, [&](int i) { return a.subs[i].x < lo; }) +
+                         (a.first_y + (int)blockIdx.y) * RO_SUBS;
+        // a lane per block; then what each shares with the block before it
+        int4 sb = make_int4(0, 0, 0, 0);
+        int seg = -1;
+        if (lane < RO_SUBS && from + lane < a.n_subs) {
+            const int2 rb = a.subs[from + lane];
+            if (rb.x >= lo && rb.x < hi) {
+                const int4 r = a.runs[rb.x];
+                const int begin = max(r.x, s_begin);  // (a run's samples lie on consecutive segments)
+                const int end = (a.clip & BP_CLIP_END) ? min(r.x + r.z, s_end) : r.x + r.z;
+                const int samples = min(32, end - begin - 32 * rb.y);
+                if (samples > 0) {
+                    sb = make_int4(samples, rb.x - lo, rb.y, r.w + begin - r.x + 32 * rb.y);
+                    seg = r.y >= 0 ? r.y : r.x;
+                }
             }
-            ratio[b] = same ? -1 : seg;
-            before = seg;
+        }
+        int before = -1;  // the factor's segment of the last block before this one that has samples
+#pragma unroll
+        for (int b = 0; b < RO_SUBS; ++b) {
+            const int other = __shfl_sync(0xffffffffu, seg, b);
+            if (b < lane && other >= 0) before = other;
+        }
+        if (lane < RO_SUBS) {
+            bool same = before >= 0 && seg >= 0;
+            if (same && seg != before) {
+                const double4 x = a.seg64[before], y = a.seg64[seg];
+                same = a.segs[before].dt == a.segs[seg].dt && x.x == y.x && x.y == y.y && x.z == y.z && x.w == y.w;
+            }
+            sub[lane] = sb;
+            ratio[lane] = same ? -1 : seg;
         }
     }
     __syncthreads();
@@ -636,10 +657,10 @@ extern "C" int bp_propagate(const float* spins, int n, const void* segs, const d
 
 extern "C" int bp_readout(const float* spins, const float* sens, int n, int n_coils, const void* segs,
                           const double* seg64, const int* windows, int w_begin, int w_end, const int* runs, int n_runs,
-                          const int* subs, int n_subs, const float* z, int z_cap, int clip, double* raw,
+                          const int* subs, int n_subs, int most_subs, const float* z, int z_cap, int clip, double* raw,
                           void* stream) {
     if (n < 1 || n_coils < 1 || n_coils > BP_MAX_COILS || w_begin < 0 || w_end < w_begin || n_runs < 0 || n_subs < 0 ||
-        z_cap < 0)
+        most_subs < 0 || z_cap < 0)
         return BP_E_ARG;
     if (w_end == w_begin || n_subs == 0 || n_runs == 0) return BP_OK;
     if (!spins || !sens || !segs || !seg64 || !windows || !runs || !subs || !z || !raw) return BP_E_ARG;
@@ -668,17 +689,12 @@ extern "C" int bp_readout(const float* spins, const float* sens, int n, int n_co
     int parts = (groups + 31) / 32;
     if (parts > 444) parts = 444;
     a.per_part = (groups + parts - 1) / parts;
-    const int blocks = (n_subs + RO_SUBS - 1) / RO_SUBS;
-    const dim3 grid((unsigned)((groups + a.per_part - 1) / a.per_part), (unsigned)blocks, (unsigned)((n_coils + 7) / 8));
-    if (blocks > 65535) {  // (the grid's second dimension)
-        for (int b = 0; b < blocks; b += 65535) {
-            const int cnt = blocks - b < 65535 ? blocks - b : 65535;
-            a.subs = reinterpret_cast<const int2*>(subs) + (size_t)b * RO_SUBS;
-            a.n_subs = n_subs - b * RO_SUBS;
-            bp_readout_kernel<<<dim3(grid.x, (unsigned)cnt, grid.z), RO_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(a);
-        }
-    } else {
-        bp_readout_kernel<<<grid, RO_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(a);
+    const int at_most = most_subs < n_subs ? most_subs : n_subs, rows = (at_most + RO_SUBS - 1) / RO_SUBS;
+    const dim3 grid((unsigned)((groups + a.per_part - 1) / a.per_part), 1u, (unsigned)((n_coils + 7) / 8));
+    for (int y = 0; y < rows; y += 65535) {  // (the most of a grid's second dimension)
+        a.first_y = y;
+        bp_readout_kernel<<<dim3(grid.x, (unsigned)(rows - y < 65535 ? rows - y : 65535), grid.z), RO_THREADS, 0,
+                            static_cast<cudaStream_t>(stream)>>>(a);
     }
     return cudaGetLastError() == cudaSuccess ? BP_OK : BP_E_LAUNCH;
 }

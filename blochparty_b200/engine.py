@@ -63,6 +63,12 @@ class SampleRuns:
         self.n_runs, self.n_subs = runs.shape[0], subs.shape[0]
         self.runs, self.subs = both[: runs.size], both[runs.size:]
         self.starts = runs[:, 0]
+        self.blocks = np.concatenate([[0], np.cumsum((runs[:, 2] + 31) // 32)])  # blocks before every run
+
+    def most_blocks(self, runs: int) -> int:
+        """The most 32-sample blocks that ``runs`` runs in a row have."""
+        ends = np.minimum(np.arange(self.n_runs) + runs, self.n_runs)
+        return int((self.blocks[ends] - self.blocks[:-1]).max()) if self.n_runs else 0
 
     def most_in(self, segments: int) -> int:
         """The most runs that start within any stretch of ``segments`` segments."""
@@ -298,6 +304,8 @@ def _window_step(pk: Packed, windows: int) -> tuple[int, int]:
     where the runs' first samples fit ``Z_BYTES``, else as many as keep any launch's runs under it."""
     runs, step = pk.sample_runs(), max(windows, 1)
     cap, room = runs.n_runs, max(Z_BYTES // (8 * max(pk.n, 1)), 1)
+    if step * _lib.BP_SEG_MAX < pk.flags.shape[0]:  # (some of the sequence's windows: not all of its runs)
+        cap = min(cap, runs.most_in(step * _lib.BP_SEG_MAX) + 1)
     if cap > room:
         step = max(1, step * room // cap)
         while step > 1 and runs.most_in(step * _lib.BP_SEG_MAX) + 1 > room:
@@ -326,6 +334,7 @@ def run_forward(pk: Packed, state: torch.Tensor, windows_dev: torch.Tensor, w_be
     runs = pk.sample_runs() if raw is not None else None
     step, cap = _window_step(pk, w_end - w_begin) if runs is not None else (max(w_end - w_begin, 1), 0)
     z = torch.empty(cap, pk.n, 2, dtype=F32, device=pk.device) if cap else None
+    most_subs = 0 if z is None else runs.n_subs if cap == runs.n_runs else runs.most_blocks(cap)
     for wa in range(w_begin, w_end, step):
         wb = min(wa + step, w_end)
         clip = 0 if whole_runs else ((_lib.BP_CLIP_BEGIN if wa == w_begin else 0)
@@ -343,7 +352,7 @@ def run_forward(pk: Packed, state: torch.Tensor, windows_dev: torch.Tensor, w_be
         if z is not None:
             code = lib.bp_readout(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64),
                                   ptr(windows_dev), wa, wb, ptr(runs.runs), runs.n_runs, ptr(runs.subs), runs.n_subs,
-                                  ptr(z), cap, clip, ptr(raw), stream)
+                                  most_subs, ptr(z), cap, clip, ptr(raw), stream)
             _lib.check(code, "bp_readout")
     return z if step >= w_end - w_begin else None
 
@@ -423,13 +432,14 @@ def forward_spans(pk: Packed, state: torch.Tensor, plan, spans, raw: torch.Tenso
         cap = min(runs.n_runs, max(Z_BYTES // (8 * max(pk.n, 1)), 1))
         if 0 < int(np.diff(run_at).max()) <= cap:
             z = torch.empty(cap, pk.n, 2, dtype=F32, device=pk.device)
-    code = _lib.lib().bp_forward_spans(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64),
-                                       ptr(wdev), rng.ctypes.data, n_spans, ctypes.addressof(spans) if n_spans else None,
-                                       ptr(state), ptr(raw), max_ctas, ptr(runs.runs) if z is not None else None,
-                                       runs.n_runs if z is not None else 0, ptr(runs.subs) if z is not None else None,
-                                       runs.n_subs if z is not None else 0,
-                                       run_at.ctypes.data if z is not None else None, ptr(z), cap, ptr(status),
-                                       _lib.stream_ptr())
+    args = (ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64), ptr(wdev), rng.ctypes.data, n_spans,
+            ctypes.addressof(spans) if n_spans else None, ptr(state), ptr(raw), max_ctas)
+    if z is None:
+        code = _lib.lib().bp_forward_spans(*args, ptr(status), _lib.stream_ptr())
+    else:
+        code = _lib.lib().bp_forward_spans_readout(*args, ptr(runs.runs), runs.n_runs, ptr(runs.subs), runs.n_subs,
+                                                   runs.most_blocks(cap), run_at.ctypes.data, ptr(z), cap, ptr(status),
+                                                   _lib.stream_ptr())
     _lib.check(code, "bp_forward_spans")
 
 

@@ -137,6 +137,8 @@ int bp_final_m(const float* state, int n, float* m, void* stream);
  *           and b0_offset; no sample but the last spoils; a run starts where those factors, a sample or its absence,
  *           a spoil or a multiple of 32 segments starts
  *   subs    [n_subs] int32 x 2: run, block of 32 samples of it, for every run and block in order
+ *   most_subs  at least the blocks of the runs that start in the windows (and of the one they start inside of): what a
+ *           launch is sized for (n_subs will do)
  *   z       [z_cap][n] (float32, float32) workspace (8-byte aligned), run by run from the first run of the windows;
  *           z_cap at least the runs that start in the windows (and the one they start inside of)
  *   clip    which of a run that reaches beyond the windows' samples are theirs: 0, the whole run where it starts
@@ -149,7 +151,7 @@ int bp_propagate(const float* spins, int n, const void* segs, const double* seg6
                  int n_runs, float* z, int z_cap, int clip, int max_ctas, int32_t* status, void* stream);
 int bp_readout(const float* spins, const float* sens, int n, int n_coils, const void* segs, const double* seg64,
                const int32_t* windows, int w_begin, int w_end, const int32_t* runs, int n_runs, const int32_t* subs,
-               int n_subs, const float* z, int z_cap, int clip, double* raw, void* stream);
+               int n_subs, int most_subs, const float* z, int z_cap, int clip, double* raw, void* stream);
 
 /* Readout runs through a nonuniform FFT (simulate(..., readout="nufft"); replaces the NUFFT readouts of
  * engines/gpu/cuda/kernels.cu.in:91-140 with engines/gpu/driver.py:236-266). A run is L consecutive samples with
@@ -457,11 +459,12 @@ int bp_surrogate_pulse_mma(const float* spins, float* state, int n, const float*
  *   BP_SPAN_MAP      bp_pulse_apply(map, n, state, phase)                 (map: device [12][n] float64)
  *   BP_SPAN_NET_MMA  bp_surrogate_pulse_mma(..., params (host), wtiles, ...)
  *   BP_SPAN_NET_F32  bp_surrogate_pulse(..., params (device), ...)
- * with phase = the RF phase (phi0 of a network), and the network fields as in those calls. With a workspace z
- * [z_cap][n] pairs the windows are stepped by bp_propagate, with one bp_readout (runs, subs as there) over as many
- * ranges as z holds the runs of, and once at the end; run_at (host int32 [n_spans + 2]): the runs that start before
- * each range, then all; no range may have more than z_cap of them. With z = NULL and raw they are stepped by
- * bp_forward. Returns the first failing call's status (launches before it stay queued). */
+ * with phase = the RF phase (phi0 of a network), and the network fields as in those calls. bp_forward_spans steps the
+ * windows by bp_forward (without raw by bp_propagate). bp_forward_spans_readout has a workspace z [z_cap][n] pairs and
+ * steps them by bp_propagate, with one bp_readout (runs, subs as there, most_subs the most blocks of any z_cap runs in a
+ * row) over as many ranges as z holds the runs of, and once at the end; run_at (host int32 [n_spans + 2]): the runs that
+ * start before each range, then all; no range may have more than z_cap of them. Both return the first failing call's
+ * status (launches before it stay queued). */
 #define BP_SPAN_MAP 0
 #define BP_SPAN_NET_MMA 1
 #define BP_SPAN_NET_F32 2
@@ -478,9 +481,12 @@ typedef struct {
 } BpSpan;
 int bp_forward_spans(const float* spins, const float* sens, int n, int n_coils, const void* segs,
                      const double* seg64, const int32_t* windows, const int32_t* ranges, int n_spans,
-                     const BpSpan* spans, float* state, double* raw, int max_ctas, const int32_t* runs, int n_runs,
-                     const int32_t* subs, int n_subs, const int32_t* run_at, float* z, int z_cap, int32_t* status,
-                     void* stream);
+                     const BpSpan* spans, float* state, double* raw, int max_ctas, int32_t* status, void* stream);
+int bp_forward_spans_readout(const float* spins, const float* sens, int n, int n_coils, const void* segs,
+                             const double* seg64, const int32_t* windows, const int32_t* ranges, int n_spans,
+                             const BpSpan* spans, float* state, double* raw, int max_ctas, const int32_t* runs,
+                             int n_runs, const int32_t* subs, int n_subs, int most_subs, const int32_t* run_at, float* z,
+                             int z_cap, int32_t* status, void* stream);
 
 /* Measurement kernel (the roofline denominator): 4 CTAs x 256 threads per SM, each thread `iters` x 128
  * independent FFMAs; `*flops` receives the flop count of the launch, which the caller divides by the launch's

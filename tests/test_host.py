@@ -559,6 +559,9 @@ def test_sample_runs(seed):
     assert np.array_equal(np.bincount(subs[:, 0], minlength=len(want)), -(-want[:, 2] // 32))
     most = max(int(((want[:, 0] >= s) & (want[:, 0] < s + 500)).sum()) for s in want[:, 0])
     assert got.most_in(500) == most
+    for k in (1, 3, len(want) + 5):
+        blocks = np.bincount(subs[:, 0], minlength=len(want))
+        assert got.most_blocks(k) == max(int(blocks[i:i + k].sum()) for i in range(len(want)))
 
 
 @pytest.mark.parametrize("rows", [1, 4, 6])
