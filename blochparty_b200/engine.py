@@ -335,18 +335,16 @@ def run_forward(pk: Packed, state: torch.Tensor, windows_dev: torch.Tensor, w_be
     step, cap = _window_step(pk, w_end - w_begin) if runs is not None else (max(w_end - w_begin, 1), 0)
     z = torch.empty(cap, pk.n, 2, dtype=F32, device=pk.device) if cap else None
     most_subs = 0 if z is None else runs.n_subs if cap == runs.n_runs else runs.most_blocks(cap)
+    if wstates is not None and wslot is None and step < w_end - w_begin:  # every few windows' states over several launches
+        wslot = torch.full((w_end,), -1, dtype=torch.int32, device=pk.device)
+        at = wslot[w_begin::wstate_stride]
+        at.copy_(torch.arange(at.shape[0], dtype=torch.int32, device=pk.device))
     for wa in range(w_begin, w_end, step):
         wb = min(wa + step, w_end)
         clip = 0 if whole_runs else ((_lib.BP_CLIP_BEGIN if wa == w_begin else 0)
                                      | (_lib.BP_CLIP_END if wb == w_end else 0))
-        slot0 = None if wstates is None or wslot is not None else (wa - w_begin)
-        ws = wstates
-        if slot0:  # (a strided save over several launches: the slots continue)
-            if slot0 % wstate_stride:
-                raise ValueError("window states every few windows need one launch")
-            ws = wstates[slot0 // wstate_stride:]
         code = lib.bp_propagate(ptr(pk.spins), pk.n, ptr(pk.segs), ptr(pk.seg64), ptr(windows_dev), wa, wb, ptr(state),
-                                ptr(ws), wstate_stride, ptr(wslot), ptr(runs.runs) if z is not None else None,
+                                ptr(wstates), wstate_stride, ptr(wslot), ptr(runs.runs) if z is not None else None,
                                 runs.n_runs if z is not None else 0, ptr(z), cap, clip, max_ctas, ptr(status), stream)
         _lib.check(code, "bp_propagate")
         if z is not None:

@@ -170,3 +170,25 @@ def test_states_saved_over_many_chunks(n):
         engine.run_forward(pk, state0.clone(), wdev, 0, W, None, status, wstates=saved)
         assert torch.equal(saved, torch.stack(want))
     _lib.check_status(status, "bp_propagate")
+
+
+@pytest.mark.parametrize("stride", [1, 3, 7])
+@pytest.mark.parametrize("begin", [0, 2])
+def test_strided_states_over_several_launches(stride, begin, monkeypatch):
+    """The state at every few windows' start, from a forward in one launch and from one whose workspace divides it."""
+    n = 300
+    ph, seq = _phantom(n, 3), _sequence((95, 64, 33, 200, 31, 95) * 3, 4)
+    pk, win, wdev, state0 = _packed(ph, seq, bpb.birdcage_sensitivities(ph.pos, 2))
+    W = win.shape[0]
+    status = torch.zeros(1, dtype=torch.int32, device=pk.device)
+    out = []
+    for room in (None, 1):
+        if room:
+            monkeypatch.setattr(engine, "Z_BYTES", 8 * n * room)
+            assert engine._window_step(pk, W - begin)[0] < W - begin
+        saved = torch.full((-(-(W - begin) // stride), 6, n), -1.0, device=pk.device)
+        raw = torch.zeros(pk.n_adc, 4, dtype=F64, device=pk.device)
+        engine.run_forward(pk, state0.clone(), wdev, begin, W, raw, status, wstates=saved, wstate_stride=stride)
+        out.append(saved)
+    assert torch.equal(out[0], out[1]) and not (out[0] == -1.0).all(2).any()
+    _lib.check_status(status, "bp_propagate")
