@@ -91,7 +91,7 @@ class Packed:
     psi: torch.Tensor  # (A,) float64 receiver phase of every sample
     flags: np.ndarray  # (S,) int32 on the host
     device: torch.device
-    runs: SampleRuns | None = None  # the runs of samples (sample_runs), laid out on the first forward with a readout
+    runs: SampleRuns | None = None  # the runs of samples (sample_runs)
 
     def sample_runs(self) -> SampleRuns:
         if self.runs is None:
@@ -292,7 +292,10 @@ def pack_with_state(case, device):
                                                    case.is_rf, case.adc, case.spoil, device, extent)
     if extent is None:
         mark_small_rf(spins, segs, flags)
-    return Packed(n, n_coils, n_adc, spins, sens, segs, seg64, psi, flags, device), state
+    pk = Packed(n, n_coils, n_adc, spins, sens, segs, seg64, psi, flags, device)
+    if segs.is_cuda and n_adc:
+        pk.sample_runs()  # (a forward is then launches alone: it can be the first thing in a captured graph)
+    return pk, state
 
 
 def pack(case, device) -> Packed:

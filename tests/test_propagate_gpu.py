@@ -192,3 +192,22 @@ def test_strided_states_over_several_launches(stride, begin, monkeypatch):
         out.append(saved)
     assert torch.equal(out[0], out[1]) and not (out[0] == -1.0).all(2).any()
     _lib.check_status(status, "bp_propagate")
+
+
+def test_first_forward_in_a_graph():
+    """A packed case's first forward can be captured: no copy from the host is left for it."""
+    ph, seq = _phantom(500, 3), _sequence((95, 64), 4)
+    pk, win, wdev, state0 = _packed(ph, seq, bpb.birdcage_sensitivities(ph.pos, 4))
+    status = torch.zeros(1, dtype=torch.int32, device=pk.device)
+    state, raw = state0.clone(), torch.zeros(pk.n_adc, 8, dtype=F64, device=pk.device)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        engine.run_forward(pk, state, wdev, 0, win.shape[0], raw, status)
+    assert torch.equal(state, state0) and not raw.any()
+    graph.replay()
+    want_state, want = state0.clone(), torch.zeros_like(raw)
+    engine.run_forward(pk, want_state, wdev, 0, win.shape[0], want, status)
+    torch.cuda.synchronize()
+    assert torch.equal(state, want_state) and float((raw - want).abs().max()) <= 1e-13 * float(want.abs().max())
+    _lib.check_status(status, "bp_propagate")
