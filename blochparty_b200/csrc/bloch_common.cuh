@@ -40,6 +40,13 @@ struct __align__(16) SegRec {
     int flags;
 };
 
+// The SMs of the current device (148 on a B200): what grids and the lines between kernel variants are sized by.
+static inline int num_sms() {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 struct Spin {
     float px, py, pz, pd, r1, r2, db0, b1;
 };

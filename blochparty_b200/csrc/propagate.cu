@@ -594,12 +594,6 @@ __global__ void __launch_bounds__(RO_THREADS, 3) bp_readout_kernel(ReadArgs a) {
 }
 
 // ---- launch helpers ----
-static int num_sms() {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
 template <int K, int NT, int CH, bool HELP>
 static int launch_propagate(const PropArgs& a, int max_ctas, cudaStream_t stream) {
     constexpr size_t smem = prop_smem<CH, HELP>();
@@ -683,11 +677,11 @@ extern "C" int bp_readout(const float* spins, const float* sens, int n, int n_co
     a.z_cap = z_cap;
     a.clip = clip;
     a.raw = raw;
-    // the spins' split depends on their number alone (so the sums' order does): parts of at least 1,024 spins, at most
-    // 444 of them (three CTAs on each of 148 SMs, so that 128 samples alone fill the GPU)
-    const int groups = (n + 31) / 32;
+    // the spins' split depends on their number and the device alone (so the sums' order does): parts of at least 1,024
+    // spins, at most three per SM (the CTAs one holds, so that 128 samples alone fill the GPU)
+    const int groups = (n + 31) / 32, most_parts = 3 * num_sms();
     int parts = (groups + 31) / 32;
-    if (parts > 444) parts = 444;
+    if (parts > most_parts) parts = most_parts;
     a.per_part = (groups + parts - 1) / parts;
     const int at_most = most_subs < n_subs ? most_subs : n_subs, rows = (at_most + RO_SUBS - 1) / RO_SUBS;
     const dim3 grid((unsigned)((groups + a.per_part - 1) / a.per_part), 1u, (unsigned)((n_coils + 7) / 8));

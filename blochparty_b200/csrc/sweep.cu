@@ -664,7 +664,7 @@ extern "C" int bp_cotangent(const float* spins, const float* sens, int n, int n_
     a.z = reinterpret_cast<const float2*>(z), a.gc = gc;
     const int x = (n + CO_THREADS - 1) / CO_THREADS;
     // the runs divided among CTAs until the spins' CTAs fill the GPU about twice (not with coil gradients)
-    int y = gc ? 1 : (2 * 592 + x - 1) / x;
+    int y = gc ? 1 : (2 * 4 * num_sms() + x - 1) / x;
     if (y > n_runs) y = n_runs;
     if (y > 1024) y = 1024;
     const dim3 grid((unsigned)x, (unsigned)(y < 1 ? 1 : y));
@@ -679,9 +679,8 @@ extern "C" int bp_cotangent(const float* spins, const float* sens, int n, int n_
 template <int K, int NT, bool SG>
 static int sweep_grid(int n, int seg_len) {
     const size_t smem = (size_t)2 * seg_len * sizeof(float);
-    int dev = 0, sms = 148, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = num_sms();
+    int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bp_sweep_kernel<K, NT, SG>, NT, smem) != cudaSuccess)
         return -1;
     const int tiles = (n + NT * K - 1) / (NT * K), room = sms * (per_sm > 0 ? per_sm : 1);
@@ -689,7 +688,7 @@ static int sweep_grid(int n, int seg_len) {
 }
 
 // one warp per CTA while the spins leave SM quarters with few warps (as bp_propagate)
-static bool few(int n) { return n <= 148 * 4 * 32 * 2; }
+static bool few(int n) { return n <= num_sms() * 4 * 32 * 2; }
 
 extern "C" int bp_sweep_grid(int n, int seg_len, int spin_gradients) {
     if (n < 1 || seg_len < 0 || seg_len > SW_MAX) return -BP_E_ARG;
