@@ -378,6 +378,7 @@ class Checkpointed:
                 if self.n_block_states:
                     self.ckpts[bi].copy_(state)
                 self._fwd_saving(state, ka, kb, self.raw if pk.n_adc else None)
+                self.slots_of = bi
             if self.saved.final:
                 self.slots[self.final_slot].copy_(state)
             return
@@ -571,18 +572,20 @@ class Checkpointed:
 
     def _saved_backward(self, h, lam, gseg, seg, seg_mask, want_gc, chain, state, swept=None):
         """The backward without a replay: per block in reverse, its saved states (rebuilt by one forward of the
-        block from its start, except the last block's, which the forward left), then per interval in reverse the
-        sweep from the saved states, carrying the chain of RF windows integrated backward across the intervals,
-        and the segment reduction."""
+        block from its start, unless the slots hold them: the forward left the last block's), then per interval in
+        reverse the sweep from the saved states, carrying the chain of RF windows integrated backward across the
+        intervals, and the segment reduction."""
         pk, plan, sv = self.pk, self.plan, self.saved
         lib, stream, W = _lib.lib(), _lib.stream_ptr(), plan.awin.shape[0]
         if want_gc or not rf_only(seg_mask):
             raise ValueError("the backward from saved states forms the RF waveform's gradient alone")
-        blocks = self.blocks()
-        for bi, (ka, kb) in reversed(list(enumerate(blocks))):
-            if bi + 1 < len(blocks):
+        for bi, (ka, kb) in reversed(list(enumerate(self.blocks()))):
+            if bi != self.slots_of:
                 state.copy_(self.ckpts[bi])
                 self._fwd_saving(state, ka, kb, None)
+                if sv.final and kb == len(plan.starts):
+                    self.slots[self.final_slot].copy_(state)
+                self.slots_of = bi
             for k in reversed(range(ka, kb)):
                 aa, ab = plan.aranges[k]
                 s0, s1 = plan.seg_ranges[k]

@@ -9,7 +9,7 @@ import pytest
 import torch
 
 import blochparty_b200 as bpb
-from blochparty_b200 import adjoint, engine, sequences
+from blochparty_b200 import _lib, adjoint, engine, sequences
 from oracle import bloch
 
 pytestmark = pytest.mark.gpu
@@ -233,3 +233,36 @@ def test_many_graphs_alive():
             out.append(_gradients(ph, seq, c, names))
     assert kept == [True, False]
     assert all(torch.equal(out[0][k], out[1][k]) for k in names)
+
+
+@pytest.mark.parametrize("states", [8, 10, 1000])
+@pytest.mark.parametrize("ends_with_rf", [False, True])
+def test_backward_twice_from_saved_states(states, ends_with_rf):
+    """The RF waveform's gradient from one forward, backward twice (a graph kept for a second gradient): the same bits
+    with the saved states in blocks, whose last one the first backward has written over, as with all of them kept."""
+    n = 70
+    ph, seq, c = _phantom(n, 13), _sequence((40, 17, 64, 9) * 3), _coils(n, 3)
+    if ends_with_rf:
+        cut = int(np.flatnonzero(np.asarray(seq.is_rf))[-1]) + 1
+        seq = bpb.Sequence(seq.dt[:cut], seq.rf[:cut], seq.grad[:cut], seq.adc_phase[:cut], seq.is_rf[:cut], seq.adc[:cut],
+                           seq.spoil[:cut])
+    dev = torch.device("cuda", 0)
+    inp = bpb.api.Inputs(ph.pos, ph.pd, ph.t1, ph.t2, ph.db0, ph.b1, c, seq.dt, seq.rf, seq.grad, seq.adc_phase, None,
+                         list(seq.is_rf), list(seq.adc), list(seq.spoil), None)
+    pk = engine.pack(inp, dev)
+    g = torch.Generator().manual_seed(1)
+    h, lam0 = torch.randn(pk.n_adc, 6, generator=g).to(dev), torch.randn(3, n, generator=g).to(dev)
+    mask = _lib.BP_SEG_WX | _lib.BP_SEG_WY | _lib.BP_SPIN_NO_OFFSETS | _lib.BP_SPIN_NONE
+    out = []
+    for budget in (24 * n * states, 1 << 40):
+        run = adjoint.Checkpointed(pk, 64, dev, saved=True, budget_bytes=budget)
+        assert run.saved is not None and run.saved.final == ends_with_rf
+        assert len(run.blocks()) > 1 or budget >= 24 * n * 1000
+        run.forward(engine.initial_state(ph.pd, None, dev))
+        for _ in range(2):
+            lam = lam0.clone()
+            seg = run.backward(h, lam, mask, False, True)[2]
+            out.append((seg.clone(), lam))
+        run.check()
+    for seg, lam in out[1:]:
+        assert torch.equal(seg, out[0][0]) and torch.equal(lam, out[0][1])
