@@ -193,6 +193,8 @@ def pack_segments(dt, rf, grad, b0_offset, adc_phase, is_rf, adc, spoil, device,
         return np.ascontiguousarray(t)
 
     phase = _np64(adc_phase)
+    if phase.shape == (S, 1):
+        phase = phase[:, 0]
     if dt.shape != (S,) or phase.shape != (S,):
         raise ValueError(f"a sequence of {S} segments takes a duration and a phase for each, got {dt.shape}, {phase.shape}")
     dt, rf, grad, phase = rows(dt, S), rows(rf[:, :2], S, 2), rows(_np64(grad), S, 3), rows(phase, S)

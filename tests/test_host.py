@@ -589,6 +589,8 @@ def test_segment_packing_broadcasts():
     for b0 in (torch.tensor(7.0, dtype=F64), torch.tensor([7.0], dtype=F64)):
         got = pack(rf, grad, b0)
         assert all(torch.equal(a, b) for a, b in zip(got[:3], want[:3])) and (got[3] == want[3]).all()
+    column = engine.pack_segments(dt, rf, grad, None, phase[:, None], *marks, "cpu")
+    assert torch.equal(column[2], want[2])
     for bad in ((rnd(S, 1), grad, None), (rnd(S - 1, 2), grad, None), (rf, rnd(S, 2), None), (rf, grad, rnd(S - 1))):
         with pytest.raises((ValueError, IndexError)):
             pack(*bad)
