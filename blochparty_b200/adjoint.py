@@ -1,18 +1,24 @@
 """Gradients: the forward with checkpoints and the hand-written adjoint behind a ``torch.autograd.Function``.
 
 Replaces blochparty ``engines/gpu/adjoint.py`` (``_GPUSimulate`` :45-261, ``_simulate_grad`` :264-323) for static
-spins. The forward stores the state at the start of every checkpoint interval (``checkpoint_every`` segments, a
-multiple of ``BP_ADJ_WIN`` = 32). The backward walks the intervals in reverse: it replays an interval with the
-forward kernel, storing the state at every 32-segment window start, then runs ``bp_adjoint`` over it (each window
-recomputed into shared memory and swept backward) and ``bp_seg_reduce`` (segment gradients summed over CTAs in
-fixed order, float64). Windows fall on multiples of 32 segments whatever the interval, so the gradients are the
-same bits for every ``checkpoint_every`` and every run.
+spins. Where the sequence's adjoint windows (``run_breaks``) are all runs of RF segments or of free ones and no
+per-segment gradient but the RF waveform's is wanted (every GRE here), the backward takes a run of samples and a window in
+one step each (``bp_cotangent``, ``bp_sweep``). Its states come from one of three places:
 
-For the RF waveform's gradient alone, on sequences whose adjoint windows are all runs of RF segments or of free
-segments (every GRE here), the forward saves instead the state after each RF run (``bp_forward_saving``) and the
-backward sweeps every interval from those states with no replay (``bp_adjoint_saved``): its RF windows integrate
-their states backward from the state after the pulse, its free windows carry lambda alone (``SavedStates``,
-``saved_layout``; in blocks, each block's states rebuilt by one forward of the block, when they do not all fit).
+* the RF waveform's gradient alone: the forward saves the state after each RF run and the backward integrates the runs
+  backward from them, with no replay (``SavedStates``, ``saved_layout``; in blocks, each block's states rebuilt by one
+  forward of the block, when they do not all fit);
+* per-spin gradients, no interval of the caller's: the forward saves every window's state, where they fit
+  (``room_to_keep``);
+* else the state at the start of every checkpoint interval (``checkpoint_every`` segments, a multiple of ``BP_ADJ_WIN`` =
+  32): the backward walks the intervals in reverse and replays each with the states at its windows' starts.
+
+RF segments are integrated backward only over stretches that are short next to the relaxation (``rf_decay``).
+
+Other gradients (of dt, the gradients, b0_offset; of the field model) and other sequences take the segment-by-segment
+sweep after the replay: ``bp_adjoint`` (each window recomputed into shared memory and swept backward) and
+``bp_seg_reduce`` (segment gradients summed over CTAs in fixed order, float64). Windows fall on multiples of 32 segments
+whatever the interval, so the gradients are the same bits for every ``checkpoint_every`` and every run.
 
 Chain rules on the host (float64), from the kernels' raw gradients: r1 = 1/T1 -> dL/dT1 = -dL/dr1 / T1^2; the
 segment record (dt, w_x = -2 pi dt rf_x, w_y, k = g dt, beta = b0_offset dt) -> dL/d(dt, rf, grad, b0_offset);
@@ -95,7 +101,7 @@ def run_breaks(flags: np.ndarray) -> np.ndarray:
 
 
 class SavedStates:
-    """Where the backward without a replay (``bp_adjoint_saved``) needs states: for adjoint windows ``awin`` whose
+    """Where the backward without a replay needs states: for adjoint windows ``awin`` whose
     every window is either RF segments with one dt and offset, no sample and no spoil (``rf[w]``: integrated backward
     from the state after it), or free segments with one set of factors spoiling at most in its last segment (lambda
     alone), the state after each run of RF windows. ``slot`` [W + 1] int32: the slot of the state at window w's start
@@ -272,7 +278,7 @@ class Checkpointed:
         self.phys = phys  # the field model (``PhysGrad``): the forward, replay and sweep take its variants
         # saved: the caller wants the RF waveform's gradient alone; then, where the sequence's windows allow it, the
         # forward saves the states after every run of RF windows and the backward needs no replay
-        # (bp_forward_saving, bp_adjoint_saved). When those states do not fit half the free memory (or
+        # (the sweep integrates the runs backward from them). When those states do not fit half the free memory (or
         # ``budget_bytes``), the forward stores the state at every start of a block of intervals instead, and the
         # backward rebuilds each block's saved states by one forward of the block (no readout) before its sweep.
         # Its intervals are at most 2048 segments (the sweep sums an interval's RF gradient in shared memory).
@@ -505,7 +511,9 @@ class Checkpointed:
             self.phys.gconc.zero_()
         swept = self.sweep_buffers(h, self.saved is None, want_gc, need_seg) if sweeps else None
         if self.saved is not None:
-            self._saved_backward(h, lam, gseg, seg, seg_mask, want_gc, b["chain"], state, swept)
+            if swept is None or want_gc or not rf_only(seg_mask):
+                raise ValueError("the backward from saved states forms the RF waveform's gradient alone")
+            self._saved_backward(lam, seg, b["chain"], state, swept)
             return gs, gc, seg
         n_blocks = len(self.blocks())
         for bi, (ka, kb) in reversed(list(enumerate(self.blocks()))):
@@ -570,15 +578,13 @@ class Checkpointed:
         if need_seg:
             _lib.check(lib.bp_seg_reduce(ptr(gseg), self.grid, s1 - s0, s0, ptr(seg), stream), "bp_seg_reduce")
 
-    def _saved_backward(self, h, lam, gseg, seg, seg_mask, want_gc, chain, state, swept=None):
+    def _saved_backward(self, lam, seg, chain, state, swept):
         """The backward without a replay: per block in reverse, its saved states (rebuilt by one forward of the
         block from its start, unless the slots hold them: the forward left the last block's), then per interval in
         reverse the sweep from the saved states, carrying the chain of RF windows integrated backward across the
         intervals, and the segment reduction."""
-        pk, plan, sv = self.pk, self.plan, self.saved
-        lib, stream, W = _lib.lib(), _lib.stream_ptr(), plan.awin.shape[0]
-        if want_gc or not rf_only(seg_mask):
-            raise ValueError("the backward from saved states forms the RF waveform's gradient alone")
+        plan, sv = self.plan, self.saved
+        W = plan.awin.shape[0]
         for bi, (ka, kb) in reversed(list(enumerate(self.blocks()))):
             if bi != self.slots_of:
                 state.copy_(self.ckpts[bi])
@@ -587,22 +593,9 @@ class Checkpointed:
                     self.slots[self.final_slot].copy_(state)
                 self.slots_of = bi
             for k in reversed(range(ka, kb)):
-                aa, ab = plan.aranges[k]
-                s0, s1 = plan.seg_ranges[k]
-                if swept is not None:
-                    for p in reversed(self.pieces[k]):
-                        self._sweep(p, swept, self.slots, self.aslot_dev, chain, int(p[1] < W and bool(sv.rf[p[1]])), lam,
-                                    None, None, seg)
-                    continue
-                chain_in = int(ab < W and bool(sv.rf[ab]))
-                code = lib.bp_adjoint_saved(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs),
-                                            ptr(pk.seg64), ptr(plan.awin_dev), aa, ab, s0, s1 - s0, ptr(self.slots),
-                                            ptr(self.aslot_dev), ptr(chain), chain_in, ptr(h), pk.n_adc, ptr(lam),
-                                            ptr(gseg), seg_mask, self.grid, ptr(self.status), stream)
-                _lib.check(code, "bp_adjoint_saved")
-                if gseg is not None:
-                    _lib.check(lib.bp_seg_reduce(ptr(gseg), self.grid, s1 - s0, s0, ptr(seg), stream),
-                               "bp_seg_reduce")
+                for p in reversed(self.pieces[k]):
+                    chain_in = int(p[1] < W and bool(sv.rf[p[1]]))
+                    self._sweep(p, swept, self.slots, self.aslot_dev, chain, chain_in, lam, None, None, seg)
 
     def launches(self, need_seg: bool) -> tuple[int, int]:
         """(forward, backward) kernel launches of one call each."""
@@ -614,7 +607,7 @@ class Checkpointed:
         if self.saved is not None:
             blocks = self.blocks()
             forward = sum(run(plan.franges[kb - 1][1] - plan.franges[ka][0]) for ka, kb in blocks)
-            return forward, len(blocks) - 1 + (swept if self.uniform else k * (2 if need_seg else 1))
+            return forward, len(blocks) - 1 + swept
         if self.kept is not None:
             return run(plan.awin.shape[0]), swept
         rebuild = sum(kb - ka - 1 for ka, kb in self.blocks()) if self.outer else 0
@@ -658,7 +651,7 @@ class PhysGrad:
 
 def rf_only(seg_mask: int) -> bool:
     """Whether ``seg_mask`` asks for the RF waveform's gradient alone (no per-spin, coil or offset gradient): the
-    sweep that ``bp_adjoint_saved`` runs."""
+    sweep from saved states."""
     return bool(seg_mask & _lib.BP_SPIN_NONE) and not seg_mask & _lib.BP_SEG_ALL & ~(_lib.BP_SEG_WX | _lib.BP_SEG_WY)
 
 

@@ -84,10 +84,10 @@ def simulate(phantom, seq, coils: Tensor | None = None, *, m_init: Tensor | None
     coils: (N, C) complex receive sensitivities (default: one uniform coil), C <= 32.
     m_init: (N, 3) starting magnetization (default: equilibrium, Mz = PD).
     checkpoint_every: with gradients, the adjoint stores the state every this many segments (a multiple of 32);
-        default about sqrt(segments).
-    options: ``readout`` "fp32" (default: float32 coil products reduced by warp shuffles), "bf16x3" (the coil
-        contraction on the tensor cores in split bfloat16 with float32 accumulation) or "nufft" (readout runs
-        through a nonuniform FFT: at least a few thousand spins; with gradients the float32 readout is taken, as
+        default the state of every window of up to 32 segments where memory allows, else about sqrt(segments).
+    options: ``readout`` "fp32" (default: coil sums to float32 precision, on the tensor cores in pairs of halves),
+        "bf16x3" (the coil contraction on the tensor cores in split bfloat16 with float32 accumulation) or "nufft"
+        (readout runs through a nonuniform FFT: at least a few thousand spins; with gradients the float32 readout is taken, as
         blochparty's GPU engines do); ``pulses`` "step" (default), "reuse" (every recurring pulse through its exact
         per-spin map; stepped with gradients) or "surrogate"
         (shaped pulses through a trained ``surrogate``), whose ``surrogate_inference`` is "mma" (default: the
