@@ -15,8 +15,9 @@ one step each (``bp_cotangent``, ``bp_sweep``). Its states come from one of thre
 
 RF segments are integrated backward only over stretches that are short next to the relaxation (``rf_decay``).
 
-Other gradients (of dt, the gradients, b0_offset; of the field model) and other sequences take the segment-by-segment
-sweep after the replay: ``bp_adjoint`` (each window recomputed into shared memory and swept backward) and
+Other gradients (of dt, the gradients, b0_offset; of the field model) and other sequences (among them those whose runs of
+samples are short, ``engine.short_runs``) take the segment-by-segment sweep after the replay, or from the saved states
+(``bp_adjoint_saved``): ``bp_adjoint`` (each window recomputed into shared memory and swept backward) and
 ``bp_seg_reduce`` (segment gradients summed over CTAs in fixed order, float64). Windows fall on multiples of 32 segments
 whatever the interval, so the gradients are the same bits for every ``checkpoint_every`` and every run.
 
@@ -275,6 +276,10 @@ class Checkpointed:
     def __init__(self, pk: engine.Packed, every: int, device, outer: int = 0, phys=None, saved: bool = False,
                  budget_bytes: int | None = None, keep: bool = False):
         self.pk, self.dev = pk, device
+        # short runs of samples: bp_forward and the segment-by-segment sweeps, in the replays too (which bp_forward takes
+        # where a window of the sweep may hold as many samples as it has segments)
+        self.windowed = (phys is None and pk.windowed(grad=True)
+                         and _lib.lib().bp_forward_samp_max(pk.n_coils) >= _lib.BP_ADJ_WIN)
         self.phys = phys  # the field model (``PhysGrad``): the forward, replay and sweep take its variants
         # saved: the caller wants the RF waveform's gradient alone; then, where the sequence's windows allow it, the
         # forward saves the states after every run of RF windows and the backward needs no replay
@@ -297,7 +302,7 @@ class Checkpointed:
         # the states fit ``room_to_keep``, the forward saves the state at every adjoint window's start and the backward
         # replays nothing (its intervals are as long as the sweep takes)
         self.kept = None
-        if self.layout is None and keep and invertible:
+        if self.layout is None and keep and invertible and not self.windowed:
             plan = Plan(pk, _lib.BP_SWEEP_MAX, device)
             room = 0
             if torch.cuda.is_available():
@@ -314,7 +319,8 @@ class Checkpointed:
         self.saved = plan.saved
         # whether every adjoint window is one run of RF or of free segments and can be integrated backward: then the
         # gradients that need no per-segment sums but the RF waveform's take a window in one step (bp_cotangent, bp_sweep)
-        self.uniform = invertible and (plan.saved is not None or self.kept is not None or self.sweepable(plan))
+        self.uniform = invertible and not self.windowed and (plan.saved is not None or self.kept is not None
+                                                             or self.sweepable(plan))
         k = len(plan.starts)
         self.outer = outer if outer > 1 and k > outer and self.saved is None and self.kept is None else 0
         fws = _lib.forward_workspace(pk.n, pk.n_adc, pk.n_coils)
@@ -371,7 +377,7 @@ class Checkpointed:
         pk, plan = self.pk, self.plan
         fa, fb = plan.franges[ka][0], plan.franges[kb - 1][1]
         engine.run_forward(pk, state, plan.fwin_dev, fa, fb, raw, self.status, wstates=self.slots,
-                           wslot=self.fslot_dev, whole_runs=True)
+                           wslot=self.fslot_dev, whole_runs=True, windowed=self.windowed)
 
     def forward(self, state: torch.Tensor) -> None:
         """All intervals from ``state`` ([6][n], advanced in place), the raw coil sums into ``raw`` (zeroed first),
@@ -391,12 +397,13 @@ class Checkpointed:
         if self.kept is not None:
             W = plan.awin.shape[0]
             self.z = engine.run_forward(pk, state, plan.awin_dev, 0, W, self.raw if pk.n_adc else None, self.status,
-                                        wstates=self.kept, whole_runs=True)
+                                        wstates=self.kept, whole_runs=True, windowed=False)
             self.kept[W].copy_(state)
             return
         if self.phys is None:  # one call, the checkpoints saved on the way
             engine.run_forward(pk, state, plan.fwin_dev, 0, plan.fwin.shape[0], self.raw if pk.n_adc else None,
-                               self.status, wstates=self.ckpts, wslot=self.ckslot_dev, whole_runs=True)
+                               self.status, wstates=self.ckpts, wslot=self.ckslot_dev, whole_runs=True,
+                               windowed=self.windowed)
             return
         for k, (fa, fb) in enumerate(plan.franges):
             if not self.outer:
@@ -410,7 +417,7 @@ class Checkpointed:
         pk = self.pk
         if self.phys is None:
             engine.run_forward(pk, state, wdev, wa, wb, raw, self.status, wstates=wstates, wstate_stride=1,
-                               whole_runs=True)
+                               whole_runs=True, windowed=self.windowed)
             return
         import ctypes
 
@@ -511,9 +518,9 @@ class Checkpointed:
             self.phys.gconc.zero_()
         swept = self.sweep_buffers(h, self.saved is None, want_gc, need_seg) if sweeps else None
         if self.saved is not None:
-            if swept is None or want_gc or not rf_only(seg_mask):
+            if want_gc or not rf_only(seg_mask):
                 raise ValueError("the backward from saved states forms the RF waveform's gradient alone")
-            self._saved_backward(lam, seg, b["chain"], state, swept)
+            self._saved_backward(h, lam, gseg, seg, seg_mask, b["chain"], state, swept)
             return gs, gc, seg
         n_blocks = len(self.blocks())
         for bi, (ka, kb) in reversed(list(enumerate(self.blocks()))):
@@ -578,13 +585,13 @@ class Checkpointed:
         if need_seg:
             _lib.check(lib.bp_seg_reduce(ptr(gseg), self.grid, s1 - s0, s0, ptr(seg), stream), "bp_seg_reduce")
 
-    def _saved_backward(self, lam, seg, chain, state, swept):
+    def _saved_backward(self, h, lam, gseg, seg, seg_mask, chain, state, swept):
         """The backward without a replay: per block in reverse, its saved states (rebuilt by one forward of the
         block from its start, unless the slots hold them: the forward left the last block's), then per interval in
-        reverse the sweep from the saved states, carrying the chain of RF windows integrated backward across the
-        intervals, and the segment reduction."""
-        plan, sv = self.plan, self.saved
-        W = plan.awin.shape[0]
+        reverse the sweep from the saved states (``swept`` None: segment by segment), carrying the chain of RF windows
+        integrated backward across the intervals, and the segment reduction."""
+        pk, plan, sv = self.pk, self.plan, self.saved
+        lib, stream, W = _lib.lib(), _lib.stream_ptr(), plan.awin.shape[0]
         for bi, (ka, kb) in reversed(list(enumerate(self.blocks()))):
             if bi != self.slots_of:
                 state.copy_(self.ckpts[bi])
@@ -593,21 +600,31 @@ class Checkpointed:
                     self.slots[self.final_slot].copy_(state)
                 self.slots_of = bi
             for k in reversed(range(ka, kb)):
-                for p in reversed(self.pieces[k]):
-                    chain_in = int(p[1] < W and bool(sv.rf[p[1]]))
-                    self._sweep(p, swept, self.slots, self.aslot_dev, chain, chain_in, lam, None, None, seg)
+                for p in reversed([(*plan.aranges[k], *plan.seg_ranges[k])] if swept is None else self.pieces[k]):
+                    aa, ab, s0, s1 = p
+                    chain_in = int(ab < W and bool(sv.rf[ab]))
+                    if swept is not None:
+                        self._sweep(p, swept, self.slots, self.aslot_dev, chain, chain_in, lam, None, None, seg)
+                        continue
+                    code = lib.bp_adjoint_saved(ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64),
+                                                ptr(plan.awin_dev), aa, ab, s0, s1 - s0, ptr(self.slots),
+                                                ptr(self.aslot_dev), ptr(chain), chain_in, ptr(h), pk.n_adc, ptr(lam),
+                                                ptr(gseg), seg_mask, self.grid, ptr(self.status), stream)
+                    _lib.check(code, "bp_adjoint_saved")
+                    if gseg is not None:
+                        _lib.check(lib.bp_seg_reduce(ptr(gseg), self.grid, s1 - s0, s0, ptr(seg), stream), "bp_seg_reduce")
 
     def launches(self, need_seg: bool) -> tuple[int, int]:
         """(forward, backward) kernel launches of one call each."""
         k, plan = len(self.plan.starts), self.plan
         readout = int(self.pk.n_adc > 0)
-        run = lambda windows: engine.forward_launches(self.pk, windows) if readout else 1
+        run = lambda windows: engine.forward_launches(self.pk, windows) if readout and not self.windowed else 1
         n_pieces = sum(map(len, self.pieces)) if self.uniform else 0
         swept = readout + n_pieces * (1 + readout + int(need_seg))  # the split, then per piece samples, sweep, sums
         if self.saved is not None:
             blocks = self.blocks()
             forward = sum(run(plan.franges[kb - 1][1] - plan.franges[ka][0]) for ka, kb in blocks)
-            return forward, len(blocks) - 1 + swept
+            return forward, len(blocks) - 1 + (swept if self.uniform else k * (2 if need_seg else 1))
         if self.kept is not None:
             return run(plan.awin.shape[0]), swept
         rebuild = sum(kb - ka - 1 for ka, kb in self.blocks()) if self.outer else 0

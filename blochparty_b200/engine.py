@@ -35,6 +35,22 @@ RF, ADC, SPOIL, SAME_FREE, SAME_RFDT, SAME_OFF, SMALL = 1, 2, 4, 8, 16, 32, 64
 
 Z_BYTES = 1 << 30  # the forward's workspace at most: the first samples of the runs of one launch
 RUN_MAX = 256  # samples per run
+# A run of samples costs bp_readout its factor and a table of powers, up to about 40 ps a spin and group of eight coils
+# whatever its samples; bp_forward pays per sample. The lines between them: samples per 32-sample block (of the sequence),
+# and spins, more of them the more samples. 1,600 samples, 8 coils, bp_propagate + bp_readout against bp_forward [ms]:
+#   samples per run  4,096 spins   20,000        40,000        262,144
+#   1 (on RF)        0.90 / 0.43   1.69 / 0.51   2.68 / 0.61   15.1 / 2.5
+#   2                0.57 / 0.85   1.14 / 1.00   2.01 / 1.20   10.4 / 5.2
+#   4                0.30 / 0.53   0.61 / 0.64   1.04 / 0.76   5.1 / 3.3
+#   8                0.19 / 0.37   0.35 / 0.45   0.56 / 0.54   2.63 / 2.28
+#   16               0.13 / 0.29   0.24 / 0.36   0.33 / 0.43   1.40 / 1.82
+# and with gradients of the T1 map (8 coils), the sweep over runs against bp_adjoint:
+#   2                2.2 / 4.3     3.7 / 4.8     (100,000 spins) 12.7 / 10.6
+#   4                1.0 / 2.7     1.9 / 2.9     6.5 / 6.6, of the RF waveform 4.3 / 3.7
+#   8                0.55 / 1.9    1.1 / 2.1     3.3 / 4.5
+#   4 at 40,000 spins, of the T1 map 2.9 / 3.3, of the RF waveform 2.4 / 1.9
+ONE_SAMPLE, FEW_SAMPLES, FEW_SAMPLES_GRAD = 1.5, 10.0, 6.0
+SPINS_PER_SAMPLE, SPINS_GRAD = 5000, 15000
 
 
 def sample_runs(flags: np.ndarray):
@@ -97,6 +113,20 @@ class Packed:
         if self.runs is None:
             self.runs = SampleRuns(self.flags, self.device)
         return self.runs
+
+    def windowed(self, grad: bool = False) -> bool:
+        """``short_runs`` of this case."""
+        return self.n_adc > 0 and short_runs(self.n_adc, self.sample_runs().n_subs, self.n, grad)
+
+
+def short_runs(n_adc: int, n_blocks: int, n: int, grad: bool = False) -> bool:
+    """Whether a forward of ``n`` spins (with gradients: and its backward) takes ``bp_forward``'s windows instead of
+    ``bp_propagate`` and ``bp_readout``: where the runs of samples are short (the lines above)."""
+    if n_blocks == 0:
+        return False
+    mean = n_adc / n_blocks
+    few, spins = (FEW_SAMPLES_GRAD, SPINS_GRAD) if grad else (FEW_SAMPLES, 0)
+    return mean < ONE_SAMPLE or (mean < few and n > spins + SPINS_PER_SAMPLE * mean)
 
 
 def _bools(flags, n: int) -> np.ndarray:
@@ -321,6 +351,8 @@ def _window_step(pk: Packed, windows: int) -> tuple[int, int]:
 
 def forward_launches(pk: Packed, windows: int) -> int:
     """Kernel launches of ``run_forward`` with a readout over ``windows`` windows."""
+    if pk.windowed():
+        return 1
     step, cap = _window_step(pk, windows)
     return -(-windows // step) * (2 if cap else 1)
 
@@ -328,14 +360,24 @@ def forward_launches(pk: Packed, windows: int) -> int:
 def run_forward(pk: Packed, state: torch.Tensor, windows_dev: torch.Tensor, w_begin: int, w_end: int,
                 raw: torch.Tensor | None, status: torch.Tensor, wstates: torch.Tensor | None = None,
                 wstate_stride: int = 1, max_ctas: int = 0, wslot: torch.Tensor | None = None,
-                whole_runs: bool = False) -> torch.Tensor | None:
-    """The forward over windows [w_begin, w_end) from ``state``, advanced in place: ``bp_propagate``, then with
+                whole_runs: bool = False, windowed: bool | None = None) -> torch.Tensor | None:
+    """The forward over windows [w_begin, w_end) from ``state``, advanced in place. With ``windowed`` (``pk.windowed()``
+    unless given): one launch of ``bp_forward``, the samples formed window by window. Else: ``bp_propagate``, then with
     ``raw`` (the coil sums, added to) ``bp_readout``, over as many windows at a time as keep the workspace between
     them under ``Z_BYTES``. ``wstates``: states at window starts, every ``wstate_stride``-th or by slot (``wslot``).
     ``whole_runs``: a run of samples is formed whole by the call whose windows it starts in (calls over consecutive
     windows then give the same bits wherever they are divided); else the windows' samples alone. Returns the workspace
     (the runs' first samples, [run][N] pairs) when one launch took all windows."""
     lib, stream = _lib.lib(), _lib.stream_ptr()
+    if pk.windowed() if windowed is None else windowed:
+        case = (ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64), ptr(windows_dev), w_begin, w_end,
+                ptr(state), ptr(raw))
+        if wslot is None:
+            code = lib.bp_forward(*case, ptr(wstates), wstate_stride, max_ctas, ptr(status), stream)
+        else:
+            code = lib.bp_forward_saving(*case, ptr(wslot), ptr(wstates), max_ctas, ptr(status), stream)
+        _lib.check(code, "bp_forward")
+        return None
     runs = pk.sample_runs() if raw is not None else None
     step, cap = _window_step(pk, w_end - w_begin) if runs is not None else (max(w_end - w_begin, 1), 0)
     z = torch.empty(cap, pk.n, 2, dtype=F32, device=pk.device) if cap else None
@@ -433,7 +475,7 @@ def forward_spans(pk: Packed, state: torch.Tensor, plan, spans, raw: torch.Tenso
         first = [int(starts[wa]) if wa < len(starts) else pk.flags.shape[0] for wa, _ in ranges] + [pk.flags.shape[0]]
         run_at = np.ascontiguousarray(np.searchsorted(runs.starts, first), dtype=np.int32)
         cap = min(runs.n_runs, max(Z_BYTES // (8 * max(pk.n, 1)), 1))
-        if 0 < int(np.diff(run_at).max()) <= cap:
+        if not pk.windowed() and 0 < int(np.diff(run_at).max()) <= cap:
             z = torch.empty(cap, pk.n, 2, dtype=F32, device=pk.device)
     args = (ptr(pk.spins), ptr(pk.sens), pk.n, pk.n_coils, ptr(pk.segs), ptr(pk.seg64), ptr(wdev), rng.ctypes.data, n_spans,
             ctypes.addressof(spans) if n_spans else None, ptr(state), ptr(raw), max_ctas)

@@ -90,8 +90,7 @@ int bp_forward(const float* spins, const float* sens, int n, int n_coils, const 
 /* bp_forward that saves the state at chosen window starts (the checkpointed forward of a simulation whose backward
  * needs no replay, see bp_adjoint_saved): wslot [n_windows] int32, wslot[w] >= 0 the slot of `wstates` ([slots][6][n]
  * float32) that takes window w's start state, -1 none. Otherwise as bp_forward (no counterpart in the reference,
- * whose checkpointed forward stores every interval start: engines/gpu/driver.py:658-662). For callers of this interface
- * without a workspace; blochparty_b200 itself saves by bp_propagate's wslot. */
+ * whose checkpointed forward stores every interval start: engines/gpu/driver.py:658-662). */
 int bp_forward_saving(const float* spins, const float* sens, int n, int n_coils, const void* segs, const double* seg64,
                       const int32_t* windows, int w_begin, int w_end, float* state, double* raw, const int32_t* wslot,
                       float* wstates, int max_ctas, int32_t* status, void* stream);
@@ -314,8 +313,7 @@ int bp_adjoint(const float* spins, const float* sens, int n, int n_coils, const 
  *   chain_in  1 when window wb was integrated backward by the previous call (chain holds its start state)
  * The other arguments are bp_adjoint's (gs and gc are not used). status |= 4 when a window needed a state that was
  * not saved (its results are then invalid). A run is integrated backward over its whole duration t, which multiplies
- * rounding errors by exp(t / T1) and exp(t / T2): the caller sees to it that they stay small (t / T <= 2).
- * For callers of this interface; blochparty_b200 itself runs bp_cotangent and bp_sweep. */
+ * rounding errors by exp(t / T1) and exp(t / T2): the caller sees to it that they stay small (t / T <= 2). */
 int bp_adjoint_saved(const float* spins, const float* sens, int n, int n_coils, const void* segs, const double* seg64,
                      const int32_t* windows, int wa, int wb, int seg0, int seg_len, const float* wstates,
                      const int32_t* wslot, float* chain, int chain_in, const float* h, int n_adc, float* lam,

@@ -331,6 +331,20 @@ def test_saved_states_plan():
     assert sv2 is not None and sv2.final and sv2.n_slots == 2 and list(sv2.points) == [pulse_ends[0]]
 
 
+def test_short_runs_rule():
+    """Which forward a case takes, from its samples per 32-sample block and its spins: samples one by one always the
+    windows' kernel, few to a run from a number of spins on, long runs never; no samples at all never."""
+    from blochparty_b200.engine import short_runs
+
+    assert not short_runs(0, 0, 1 << 20) and not short_runs(0, 0, 1 << 20, grad=True)
+    assert short_runs(1000, 1000, 1) and short_runs(1000, 1000, 1, grad=True)
+    assert not short_runs(2000, 1000, 10_000) and short_runs(2000, 1000, 10_001)
+    assert not short_runs(2000, 1000, 25_000, grad=True) and short_runs(2000, 1000, 25_001, grad=True)
+    assert not short_runs(8000, 1000, 40_000) and short_runs(8000, 1000, 40_001)
+    assert not short_runs(8000, 1000, 1 << 24, grad=True)
+    assert not short_runs(10_000, 1000, 1 << 24)
+
+
 @pytest.mark.parametrize("room", [1, 3, 1000])
 def test_sweep_pieces(room):
     """An interval's windows in pieces for the sweep: all of them once and in order, each piece of at most BP_SWEEP_MAX
