@@ -78,13 +78,14 @@ class SampleRuns:
         both = torch.from_numpy(np.concatenate([runs.reshape(-1), subs.reshape(-1)])).to(device)
         self.n_runs, self.n_subs = runs.shape[0], subs.shape[0]
         self.runs, self.subs = both[: runs.size], both[runs.size:]
-        self.starts = runs[:, 0]
-        self.blocks = np.concatenate([[0], np.cumsum((runs[:, 2] + 31) // 32)])  # blocks before every run
+        self.starts, self.lengths = runs[:, 0], runs[:, 2]
 
     def most_blocks(self, runs: int) -> int:
         """The most 32-sample blocks that ``runs`` runs in a row have."""
-        ends = np.minimum(np.arange(self.n_runs) + runs, self.n_runs)
-        return int((self.blocks[ends] - self.blocks[:-1]).max()) if self.n_runs else 0
+        if runs >= self.n_runs:
+            return self.n_subs
+        before = np.concatenate([[0], np.cumsum((self.lengths + 31) // 32)])
+        return int((before[runs:] - before[:-runs]).max()) if runs else 0
 
     def most_in(self, segments: int) -> int:
         """The most runs that start within any stretch of ``segments`` segments."""
@@ -162,7 +163,8 @@ def _upload_spins(pos, pd, t1, t2, db0, b1, coils, m_init, device, want_state: b
     rows = [_host(t.expand(n)) for t in (pd, t1, t2, db0)]
     pos = _host(pos.expand(n, 3))
     b1 = None if b1 is None else _host(b1.expand(n))
-    coils = coils.reshape(n, n_coils)  # (raises where it has other than n rows: the packer reads n of them)
+    if coils.shape != (n, n_coils):
+        coils = coils.reshape(n, n_coils)  # (raises where it has other than n rows: the packer reads n of them)
     coils = _host(coils if coils.dtype in (torch.complex64, torch.complex128) else coils.to(torch.complex128))
     m0 = None if m_init is None else _host(m_init.expand(n, 3))
     spins = torch.empty(8, n, dtype=F32, device=device)
@@ -381,7 +383,7 @@ def run_forward(pk: Packed, state: torch.Tensor, windows_dev: torch.Tensor, w_be
     runs = pk.sample_runs() if raw is not None else None
     step, cap = _window_step(pk, w_end - w_begin) if runs is not None else (max(w_end - w_begin, 1), 0)
     z = torch.empty(cap, pk.n, 2, dtype=F32, device=pk.device) if cap else None
-    most_subs = 0 if z is None else runs.n_subs if cap == runs.n_runs else runs.most_blocks(cap)
+    most_subs = 0 if z is None else runs.most_blocks(cap)
     if wstates is not None and wslot is None and step < w_end - w_begin:  # every few windows' states over several launches
         wslot = torch.full((w_end,), -1, dtype=torch.int32, device=pk.device)
         at = wslot[w_begin::wstate_stride]
