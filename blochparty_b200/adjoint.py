@@ -141,15 +141,23 @@ class SavedStates:
         return cls(rf, slot, points, final)
 
 
+def durations_and_rate(pk: engine.Packed) -> tuple[np.ndarray, float]:
+    """The segments' durations as the kernels have them (float64), and the largest relaxation rate of any spin (NaN if one
+    is): from the packing, or read back."""
+    if getattr(pk, "dt", None) is not None:
+        return pk.dt.astype(np.float64), pk.rate
+    return (pk.segs[:, 0].cpu().numpy().astype(np.float64),
+            float(torch.maximum(pk.spins[4], pk.spins[5]).max()) if pk.n else 0.0)
+
+
 def rf_relaxation_invertible(pk: engine.Packed) -> bool:
     """Whether every spin's half-step relaxation over every RF segment keeps 1 + expm1(-dt r / 2) >= 1/2 (the
     backward integration divides by it) with a margin: dt r <= 1.35 (2 ln 2 = 1.386) for the longest RF segment."""
     rf = (pk.flags & engine.RF) != 0
     if not rf.any():
         return True
-    dt = float(pk.segs[torch.from_numpy(np.flatnonzero(rf)).to(pk.segs.device), 0].max())
-    r = float(torch.maximum(pk.spins[4], pk.spins[5]).max())
-    return dt * r <= 1.35
+    dt, r = durations_and_rate(pk)
+    return float(dt[rf].max()) * r <= 1.35
 
 
 # A stretch of RF segments is integrated backward over a duration t only while t r <= 2 for the largest rate r: the
@@ -165,10 +173,10 @@ def rf_decay(pk: engine.Packed, awin: np.ndarray) -> tuple[float, float]:
     if awin.shape[0] == 0 or pk.n == 0:
         return 0.0, 0.0
     rf = (pk.flags[awin[:, 0]] & engine.RF) != 0
-    t = np.add.reduceat(pk.segs[:, 0].cpu().numpy().astype(np.float64), awin[:, 0]) * rf
+    dt, r = durations_and_rate(pk)
+    t = np.add.reduceat(dt, awin[:, 0]) * rf
     total = np.cumsum(t)
     run = total - np.maximum.accumulate(np.where(rf, 0.0, total))  # since the last free window
-    r = float(torch.maximum(pk.spins[4], pk.spins[5]).max())
     return float(t.max()) * r, float(run.max()) * r
 
 
@@ -304,14 +312,9 @@ class Checkpointed:
         self.kept = None
         if self.layout is None and keep and invertible and not self.windowed:
             plan = Plan(pk, _lib.BP_SWEEP_MAX, device)
-            room = 0
-            if torch.cuda.is_available():
-                free, total = torch.cuda.mem_get_info(device)
-                cached = torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
-                room = room_to_keep(free, cached, total)
             z_bytes = 8 * pk.n * pk.sample_runs().n_runs
-            if (z_bytes <= engine.Z_BYTES and 24 * pk.n * (plan.awin.shape[0] + 1) + z_bytes <= room
-                    and self.sweepable(plan)):
+            if z_bytes <= engine.Z_BYTES and self._may_keep(24 * pk.n * (plan.awin.shape[0] + 1) + z_bytes) and (
+                    self.sweepable(plan)):
                 self.kept = torch.empty(plan.awin.shape[0] + 1, 6, pk.n, dtype=F32, device=device)
         if self.layout is None and self.kept is None:
             plan = Plan(pk, every, device)
@@ -359,6 +362,16 @@ class Checkpointed:
         self.raw = sized(fws.raw, (max(pk.n_adc, 1), 2 * pk.n_coils), F64, device, zero=True)
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
         self._bufs = None
+
+    def _may_keep(self, nbytes: int) -> bool:
+        """Whether ``nbytes`` fit ``room_to_keep`` (the allocator asked what it holds unused only where that decides)."""
+        if not torch.cuda.is_available():
+            return False
+        free, total = torch.cuda.mem_get_info(self.dev)
+        if nbytes <= room_to_keep(free, 0, total) or nbytes > total // 16:
+            return nbytes <= total // 16
+        cached = torch.cuda.memory_reserved(self.dev) - torch.cuda.memory_allocated(self.dev)
+        return nbytes <= room_to_keep(free, cached, total)
 
     def sweepable(self, plan: "Plan") -> bool:
         """Whether the sweep over runs can take ``plan``'s windows with per-spin gradients: each of RF or of free segments,

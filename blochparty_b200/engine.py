@@ -109,6 +109,8 @@ class Packed:
     flags: np.ndarray  # (S,) int32 on the host
     device: torch.device
     runs: SampleRuns | None = None  # the runs of samples (sample_runs)
+    dt: np.ndarray | None = None  # the segments' durations (float32) and the spins' largest relaxation rate, on the host
+    rate: float | None = None
 
     def sample_runs(self) -> SampleRuns:
         if self.runs is None:
@@ -327,6 +329,8 @@ def pack_with_state(case, device):
     if extent is None:
         mark_small_rf(spins, segs, flags)
     pk = Packed(n, n_coils, n_adc, spins, sens, segs, seg64, psi, flags, device)
+    if extent is not None:
+        pk.dt, pk.rate = _np64(case.dt).astype(np.float32), float(np.maximum(extent[4], extent[5]))
     if segs.is_cuda and n_adc:
         pk.sample_runs()  # (a forward is then launches alone: it can be the first thing in a captured graph)
     return pk, state
