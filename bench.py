@@ -463,8 +463,9 @@ def measure_fwd_adjoint(args, dev, pk, state0, flush, n, S):
         "states": saved_states_text(run),
         "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                      "traffic": None, "peak_source": "live FFMA probe (bp_ffma_peak) on this GPU",
-                     "kernel": ("bp_propagate_kernel + bp_readout_kernel (forward" + (")" if run.saved is not None
-                                                                                     else ", replay)")
+                     "kernel": (("bp_forward_kernel" if run.windowed else "bp_propagate_kernel + bp_readout_kernel")
+                                + " (forward" + (")" if run.saved is not None
+                                                 else ", replay)")
                                 + (" + bp_cotangent_kernel + bp_sweep_kernel + bp_sweep_reduce_kernel" if run.uniform
                                    else " + bp_adjoint_kernel + bp_seg_reduce_kernel")),
                      "flops_per_spin": {"forward": fwd, "backward": bwd}},
@@ -722,8 +723,8 @@ def main():
                      "peak_source": "live FFMA probe (bp_ffma_peak) on this GPU; MEASURED_PEAKS.json has no FP32",
                      "kernel": ("bp_forward_mma_kernel" if mma is not None else
                                 "bp_forward_kernel (NUFFT runs) + bp_nufft_finish_kernel" if nr is not None
-                                else "bp_propagate_kernel + bp_readout_kernel" if replaced is None
-                                else "bp_forward_kernel"),
+                                else "bp_forward_kernel" if pk.windowed()
+                                else "bp_propagate_kernel + bp_readout_kernel"),
                      "kernel_ms": kernel_ms,
                      "flops_per_launch": flops},
         "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,

@@ -18,10 +18,11 @@
 // per window and tile it loaded spins, state and sensitivities and stored the state, which took a third of the time at
 // 12 to 16 warps per SM, and with few spins every sample's work lay on the chain of segments.
 //
-// Measured against that kernel (bp_forward, which callers without a workspace still have; one B200): 8,388,608 spins x 8
-// TRs of the 4-echo head scan 143.0 -> 81.8 ms, 1,048,576 spins x 24 TRs of the slab 3D GRE 18.1 -> 11.7 ms, the
-// 393,216-spin TSE 185 -> 116 ms, 4,096 spins x 264 TRs of the 64 x 64 GRE 3.23 -> 0.97 ms. RF steps now take 61 cycles
-// per 32 spins and SM quarter (the FMA pipe alone 54); with few spins the chain of steps bounds it (about 3 us per TR).
+// Measured against that kernel (bp_forward, which is still the faster one for short runs of samples: the rule and both
+// sides' times are in blochparty_b200/engine.py; one B200): 8,388,608 spins x 8 TRs of the 4-echo head scan 143.0 -> 79.9
+// ms, 1,048,576 spins x 24 TRs of the slab 3D GRE 18.1 -> 11.7 ms, the 393,216-spin TSE 185 -> 114 ms, 4,096 spins x 264 TRs
+// of the 64 x 64 GRE 3.23 -> 0.79 ms. RF steps now take 61 cycles per 32 spins and SM quarter (the FMA pipe alone 54); with
+// few spins the chain of steps bounds it (about 3 us per TR).
 //
 // Free segments with one set of factors, all samples or none, are one step within a block of BP_ADJ_WIN segments (the
 // cuts depend on the sequence alone), the state from the merged factors, whose phase is taken in float64.
