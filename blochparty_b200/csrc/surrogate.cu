@@ -536,11 +536,10 @@ __device__ __forceinline__ void sincos_reduced(double x, float* s, float* c) {
     sincosf((float)(x - 2.0 * M_PI * rint(x * (0.5 / M_PI))), s, c);
 }
 
-__device__ __forceinline__ void quat_mul_f(const float a[4], const float b[4], float o[4]) {
-    o[0] = a[0] * b[0] - a[1] * b[1] - a[2] * b[2] - a[3] * b[3];
-    o[1] = a[0] * b[1] + a[1] * b[0] + a[2] * b[3] - a[3] * b[2];
-    o[2] = a[0] * b[2] - a[1] * b[3] + a[2] * b[0] + a[3] * b[1];
-    o[3] = a[0] * b[3] + a[1] * b[2] - a[2] * b[1] + a[3] * b[0];
+// The quaternion q turned about z on both sides, (c1, 0, 0, s1) q (c2, 0, 0, s2).
+__device__ __forceinline__ void turn_quat(float c1, float s1, const float q[4], float c2, float s2, float o[4]) {
+    const float a = c1 * q[0] - s1 * q[3], b = c1 * q[1] - s1 * q[2], c = c1 * q[2] + s1 * q[1], d = c1 * q[3] + s1 * q[0];
+    o[0] = a * c2 - d * s2, o[1] = b * c2 + c * s2, o[2] = c * c2 - b * s2, o[3] = d * c2 + a * s2;
 }
 
 // The network's outputs y (the reduced quaternion, dA~ / T, dC~ / T) applied to one spin's state (m + l):
@@ -556,10 +555,8 @@ __device__ __forceinline__ void apply_pulse_map(const float* y, const PulseArgs&
     float s1, c1, s2, c2;
     sincos_reduced(0.5 * (half + a.phi0), &s1, &c1);
     sincos_reduced(0.5 * (half - a.phi0), &s2, &c2);
-    const float qa[4] = {c1, 0.f, 0.f, s1}, qb[4] = {c2, 0.f, 0.f, s2};
-    float t4[4], q[4];
-    quat_mul_f(qa, qr, t4);
-    quat_mul_f(t4, qb, q);
+    float q[4];
+    turn_quat(c1, s1, qr, c2, s2, q);
     const float s = q[0], x = q[1], yq = q[2], z = q[3];
     float R[9] = {1 - 2 * (yq * yq + z * z), 2 * (x * yq - s * z), 2 * (x * z + s * yq),
                   2 * (x * yq + s * z), 1 - 2 * (x * x + z * z), 2 * (yq * z - s * x),
@@ -657,8 +654,8 @@ extern "C" int bp_surrogate_pulse(const float* spins, float* state, int n, const
 // reciprocal for two values (the special-function unit was its bound). One 300-step pulse over 393,216 spins: 0.0924 ms
 // before; 0.0782 with the pairs and one group in each of three CTAs, 0.0761 with two blocks of columns in flight, 0.0739
 // with two groups in each of two CTAs (five groups in one CTA 0.0787, four 0.086); 0.0715 with one multiplication fewer in
-// the GELU, 0.0690 with the wait for a layer's product at the loop's head and all four blocks of columns in flight, 0.0670
-// without float64 divisions. (Half a layer's product issued while the other half's operand is formed: 0.0715, the barriers
+// the GELU, 0.0690 with the wait for a layer's product at the loop's head and all four blocks of columns in flight, 0.0667
+// without float64 divisions and products with zero. (Half a layer's product issued while the other half's operand is formed: 0.0715, the barriers
 // cost more; spins and states read ahead: the same.)
 // Per tile of 128 spins (a group's thread t = spin row t = tensor-memory lane t), four rounds, one per layer: every
 // thread stores its row of the layer's input, split into bfloat16 high and low parts, as the A operand (K-major),
@@ -832,7 +829,6 @@ __global__ void __launch_bounds__(SI_THREADS, 2) bp_surrogate_pulse_mma_kernel(c
             for (int i = MLP_IN; i < SI_K1; ++i) g[i] = 0.0f;
             store_row_bf16x2<SI_K1 / 8>(ahi, alo, tid, g, 0);
         }
-#pragma unroll 1
         // a layer's product, issued by one thread
         auto issue = [&](int layer) {
             if (!w_ready && !mbar_wait_bounded(wbar, 0)) err = true;
