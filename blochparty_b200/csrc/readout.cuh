@@ -30,7 +30,7 @@
 // Shared memory of a warp's 32 spins, laid out so that a lane's two spins of every eight (8 g + t and 8 g + 4 + t) come
 // as the operands of paired instructions, without moves: a pair is 16 bytes, (re, re', im, im'), and the rows of the
 // table of powers are 80 words apart (the rows a load phase takes lie on different banks). With a complex number per
-// spin, and the imaginary sums' operand turned in registers, the ALU pipe was 58 % busy, now 48 %: 0.727 -> 0.665 ms for
+// spin, and the imaginary sums' operand turned in registers, the ALU pipe was 58 % busy, then 48 %: 0.727 -> 0.665 ms for
 // 1,048,576 spins x 512 samples x 8 coils, 3.11 -> 2.89 ms for 393,216 x 6,144.
 #define RO_TAB_ROW 80  // floats per table row (16 pairs + 16 words)
 __device__ __forceinline__ int pair_word(int spin) { return ((spin >> 3) * 4 + (spin & 3)) * 4 + ((spin >> 2) & 1); }
