@@ -284,10 +284,8 @@ class Checkpointed:
     def __init__(self, pk: engine.Packed, every: int, device, outer: int = 0, phys=None, saved: bool = False,
                  budget_bytes: int | None = None, keep: bool = False):
         self.pk, self.dev = pk, device
-        # short runs of samples: bp_forward and the segment-by-segment sweeps, in the replays too (which bp_forward takes
-        # where a window of the sweep may hold as many samples as it has segments)
-        self.windowed = (phys is None and pk.windowed(grad=True)
-                         and _lib.lib().bp_forward_samp_max(pk.n_coils) >= _lib.BP_ADJ_WIN)
+        # short runs of samples: bp_forward and the segment-by-segment sweeps, in the replays too
+        self.windowed = phys is None and pk.windowed(grad=True)
         self.phys = phys  # the field model (``PhysGrad``): the forward, replay and sweep take its variants
         # saved: the caller wants the RF waveform's gradient alone; then, where the sequence's windows allow it, the
         # forward saves the states after every run of RF windows and the backward needs no replay

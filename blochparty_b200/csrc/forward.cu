@@ -173,9 +173,11 @@ __global__ void __launch_bounds__(BP_THREADS, NCG == 1 ? 5 : 4) bp_forward_kerne
     for (int i = tid; i < BP_WARPS * samp_max<NCG>() * VG; i += BP_THREADS) acc[i] = 0.0f;
     __syncthreads();
 
+    // (without a readout nothing accumulates: a window may hold as many samples as segments)
+    const int samp_room = a.raw != nullptr ? samp_max<NCG>() : BP_SEG_MAX;
     auto issue = [&](int w, int buf) {
         const int4 win = a.windows[w];
-        if (!window_ok(win, samp_max<NCG>())) {  // never copy what does not fit: complete the phase without data
+        if (!window_ok(win, samp_room)) {  // never copy what does not fit: complete the phase without data
             atomicOr(a.status, BP_ERR_BAD_WINDOW);
             mbar_arrive(&bars[buf]);
             return;
@@ -195,7 +197,7 @@ __global__ void __launch_bounds__(BP_THREADS, NCG == 1 ? 5 : 4) bp_forward_kerne
             return;
         }
         const int4 win = a.windows[w];
-        if (!window_ok(win, samp_max<NCG>())) return;  // uniform; the status bit was set where it was staged
+        if (!window_ok(win, samp_room)) return;  // uniform; the status bit was set where it was staged
         if (tid == 0 && w + 1 < a.w_end) issue(w + 1, buf ^ 1);  // after the check: nothing left in flight
         const SegRec* q0 = segbuf + buf * BP_SEG_MAX;
         const int nseg = win.y - win.x;
